@@ -25,6 +25,7 @@ struct CgScalars {
   int guard;        // body passes, counted by the direction kernel
   int stop_rule;    // B200LA_STOP_ITERATE_CONTROL or B200LA_STOP_LMP_CG
   unsigned ticket[4];
+  unsigned err;     // a wait of the resident form ran out
 };
 
 }  // namespace b200la
@@ -45,6 +46,14 @@ struct b200la_cg_s {
   int g_format, g_param;       // schedule baked into the graph
   int g_gen;                   // the matrix's schedule generation at capture
   int grid_spmv, grid_ew;
+  // cluster form (cg_cluster_kernel): 0 blocks = not used
+  int cl_blocks, cl_regs;      // blocks of the cluster, rows a thread
+  size_t cl_smem;
+  // resident form (cg_resident_kernel): 0 blocks = the graph of three kernels
+  int res_blocks, res_rows;    // blocks, rows per block
+  void *zg, *pg[2];            // z = invD r and the last two directions, for the gathers
+  void *tag_slots;             // TagSync slots (kTagSlotBytes)
+  unsigned long long epoch;    // tag epochs used so far
 };
 
 namespace b200la {

@@ -708,6 +708,7 @@ int b200la_mat_zero_rows(b200la_mat m, const int *rows, int size, double alpha) 
     zero_rows_kernel<float><<<grid, kBlock, 0, s>>>(size, d_rows, m->rowptr, m->col, (float *)m->val, (float)alpha);
   B_CUDA(cudaGetLastError());
   B_CUDA(cudaFreeAsync(d_rows, s));
+  m->cl_state = 0;
   if (is_sliced(m->format)) {
     // the values changed: rebuild the sliced copy with the same geometry
     const int C = m->sell.c, sigma = m->sell.sigma;

@@ -113,6 +113,10 @@ struct b200la_mat_s {
   int format;         // B200LA_FMT_CSR / B200LA_FMT_SELL
   int param;          // CSR lanes per row / SELL width
   SellData sell;
+  // symmetric offset structure for the cluster-resident solver
+  // (cluster_cg.cuh): cl_state 0 not looked for yet, 1 found, -1 none
+  int cl_state;
+  int cl_H, cl_off[13];
   int sched_gen;      // bumped whenever the schedule or its device data change (graphs re-capture)
 };
 
@@ -229,17 +233,17 @@ template <typename T> __device__ __forceinline__ T ld_keep(const T *p) { return 
 // returned in every lane of the group.
 // X is the type of x and of the sum (the stored values T are widened to it:
 // FP32 values times FP64 vectors in the mixed-storage inner solve).
-template <typename T, int G, typename X = T>
+// ld(c) reads x[c].
+template <typename T, int G, typename X, typename Ld>
 __device__ __forceinline__ X csr_row_group(const int *__restrict__ rowptr, const int *__restrict__ col,
-                                           const T *__restrict__ val, const X *__restrict__ x, int row,
-                                           bool valid) {
+                                           const T *__restrict__ val, const Ld &ld, int row, bool valid) {
   const int lane = threadIdx.x & (G - 1);
   X sum = X(0);
   if (valid) {
     const int start = __ldg(rowptr + row), end = __ldg(rowptr + row + 1);
 #pragma unroll 4
     for (int j = start + lane; j < end; j += G)
-      sum = fma((X)ld_stream(val + j), ld_keep(x + ld_stream(col + j)), sum);
+      sum = fma((X)ld_stream(val + j), ld(ld_stream(col + j)), sum);
   }
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

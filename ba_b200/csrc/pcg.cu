@@ -10,17 +10,24 @@
 //   K2  alpha = rz/pAp; x += alpha p; r -= alpha Ap; z = invD r;
 //       fused sums r.r and r.z; its last block applies IterateControl
 //   K3  beta = rz_new/rz_old; p = beta p + z  (z recomputed from r, invD)
+// Where the system fits, the same loop runs in one launch instead, on one
+// cluster (cg_cluster_kernel) or on resident blocks (cg_resident_kernel): an
+// iteration of small systems is launches and reductions, not bytes.
 // All scalars live in device memory.  The three kernels form the body of a
 // CUDA-graph WHILE node, so one graph launch runs the whole solve; K3 clears
 // the loop condition once the state leaves "iterate".  K3 also counts body
 // passes and stops the loop after maxits + 2 passes whatever K2 reported, so
 // the device loop ends even if a reduction misbehaves.
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <type_traits>
 #include <vector>
 
 #include "cg_internal.cuh"
+#include "cluster_cg.cuh"
+#include "persist.cuh"
 #include "spmv.cuh"
 
 namespace b200la {
@@ -227,6 +234,212 @@ __global__ void __launch_bounds__(kBlock) cg_direction_kernel(CgVecs<T> v, CgSca
     v.p[i] = fma(beta, v.p[i], PRE ? v.r[i] * v.invd[i] : v.r[i]);
 }
 
+// ---- the whole loop in one launch, vectors resident ------------------------------
+// For systems whose iteration is bound by launches and not by bytes.  Every
+// block owns the rows that the schedule gives it (grid-stride, as in K1) and
+// keeps their x, r, p, Ap and invD in shared memory for the whole solve; one
+// iteration is a gather phase and an update phase with one grid-wide sum
+// (tag_sum) after each:
+//   gather  p = z + beta p_old on the fly for every column read (the same
+//           expression, so the same bits, as the owner's update of its own
+//           p), Ap, p.Ap; the owner writes its p for the next iteration's
+//           gathers
+//   update  alpha; x += alpha p; r -= alpha Ap; z = invD r (written for the
+//           gathers); r.r, r.z; every block then takes the same decision
+// Two buffers of p by iteration parity: p_old of this iteration is read while
+// p is written to the other.  z has one: a block rewrites its rows after the
+// p.Ap sum, which every block has added to once its gathers are done.
+// The first gather reads z = the given p and p_old = 0 with beta = 0.
+template <typename T> struct CgGather {
+  const T *z, *po;  // not read-only: rewritten between phases
+  T beta;
+  __device__ __forceinline__ T operator()(int c) const { return fma(beta, po[c], z[c]); }
+  __device__ __forceinline__ CgGather at(int row) const { return CgGather{z + row, po + row, beta}; }
+};
+
+template <typename T> struct CgResidentBufs {
+  T *z, *p0, *p1;
+  int rows;  // shared-memory rows per block
+};
+
+template <typename T, bool PRE> struct CgGatherEmit {
+  T *ps, *aps, *pn;
+  const T *rs, *ds;
+  T beta;
+  bool first;
+  int at, step;  // shared-memory index of this thread's next row
+  Acc<T> acc;
+  __device__ __forceinline__ void operator()(int row, T y) {
+    T p = ps[at];
+    if (!first) p = fma(beta, p, PRE ? rs[at] * ds[at] : rs[at]);
+    ps[at] = p;
+    aps[at] = y;
+    pn[row] = p;
+    acc.add(y * p);
+    at += step;
+  }
+};
+
+template <typename Op, typename T, bool PRE, int NT>
+__global__ void __launch_bounds__(NT, 1) cg_resident_kernel(Op op, CgVecs<T> v, CgResidentBufs<T> rb, TagSync ts,
+                                                            unsigned long long epoch, CgScalars *sc) {
+  extern __shared__ __align__(16) unsigned char cg_dyn[];
+  if (*(volatile int *)&sc->state != B200LA_ITERATE) return;
+  constexpr int G = Op::kLanes;
+  const int R = rb.rows;
+  T *xs = reinterpret_cast<T *>(cg_dyn), *rs = xs + R, *ps = rs + R, *aps = ps + R, *ds = aps + R;
+  int *row_of = reinterpret_cast<int *>(ds + (PRE ? R : 0));
+  const int at0 = (int)threadIdx.x / G;
+  constexpr int step = NT / G;
+  int cnt = 0;
+  op.template each_row<NT>([&](int row) {
+    const int a = at0 + cnt * step;
+    row_of[a] = row;
+    xs[a] = v.x[row];
+    rs[a] = v.r[row];
+    const T p = v.p[row];
+    ps[a] = p;
+    if (PRE) ds[a] = v.invd[row];
+    rb.z[row] = p;
+    rb.p0[row] = T(0);
+    ++cnt;
+  });
+  double rz = sc->rz, rz_prev = sc->rz_prev, rr = sc->rr, res = sc->res, beta_d = 0.0, alpha_d = 0.0, pap = 0.0;
+  const double first_res = sc->res_init;
+  const CgScalars lim = *sc;  // tolerances, maxits and the stop rule
+  int iter = lim.iter, state = B200LA_ITERATE;
+  bool first = true;
+  double s0[1] = {0.0};
+  bool ok = tag_sum<1, true>(s0, ts, ++epoch);  // z and p0 are written
+  // maxits ends the loop; the bound only guards against broken sums
+  for (int k = 0; ok && state == B200LA_ITERATE && k < lim.maxits + 2; ++k) {
+    T *pn = (k & 1) ? rb.p0 : rb.p1;
+    const T beta = (T)beta_d;
+    CgGatherEmit<T, PRE> e{ps, aps, pn, rs, ds, beta, first, at0, step};
+    op.template run_with<NT>(CgGather<T>{rb.z, (k & 1) ? rb.p1 : rb.p0, beta}, e);
+    first = false;
+    double s1[1] = {e.acc.value()};
+    ok = tag_sum<1, false>(s1, ts, ++epoch);
+    if (!ok) break;
+    pap = s1[0];
+    alpha_d = rz / pap;
+    if (!(pap != 0.0) || !isfinite(alpha_d)) {
+      state = B200LA_FAIL_BREAKDOWN;
+      break;
+    }
+    const T alpha = (T)alpha_d;
+    Acc<T> arr, arz;
+    for (int c = 0; c < cnt; ++c) {
+      const int a = at0 + c * step;
+      xs[a] = fma(alpha, ps[a], xs[a]);
+      const T r = fma(-alpha, aps[a], rs[a]);
+      rs[a] = r;
+      const T z = PRE ? r * ds[a] : r;
+      rb.z[row_of[a]] = z;
+      arr.add(r * r);
+      if (PRE) arz.add(r * z);
+    }
+    double s2[2] = {arr.value(), arz.value()};
+    ok = tag_sum<2, true>(s2, ts, ++epoch);
+    if (!ok) break;
+    rr = s2[0];
+    res = sqrt(rr);
+    ++iter;
+    state = iterate_check(iter, res, lim, first_res);
+    const double rz_new = PRE ? s2[1] : rr;
+    beta_d = rz_new / rz;
+    rz_prev = rz;
+    rz = rz_new;
+  }
+  if (ok && state == B200LA_ITERATE) state = B200LA_FAIL_BREAKDOWN;  // the guard
+  for (int c = 0; c < cnt; ++c) {
+    const int a = at0 + c * step, row = row_of[a];
+    v.x[row] = xs[a];
+    v.r[row] = rs[a];
+    v.p[row] = ps[a];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->rz = rz;
+    sc->rz_prev = rz_prev;
+    sc->pAp = pap;
+    sc->alpha = alpha_d;
+    sc->beta = beta_d;
+    sc->rr = rr;
+    sc->res = res;
+    sc->iter = iter;
+    sc->state = ok ? state : B200LA_FAIL_BREAKDOWN;
+  }
+}
+
+// ---- the whole loop on one cluster (cluster_cg.cuh) -------------------------------
+// The same recurrence, decisions and outputs as the graph of three kernels;
+// the matrix is read once, when shared memory is filled.
+template <typename M, typename T, int H, int R, bool PRE>
+__global__ void __launch_bounds__(kClThreads, 1) cg_cluster_kernel(ClMatrix<M> m, CgVecs<T> v, CgScalars *sc) {
+  extern __shared__ __align__(16) unsigned char cl_dyn[];
+  if (*(volatile int *)&sc->state != B200LA_ITERATE) return;
+  ClCg<T, H, R, PRE> g;
+  g.carve(cl_dyn, m);
+  g.fill(m);
+  g.load_window(v.p);
+  g.each([&](int j, int li) {
+    const int row = g.r0 + li;
+    g.c[j] = v.x[row];
+    g.r[j] = v.r[row];
+    if (PRE) g.d[j] = v.invd[row];
+  });
+  const CgScalars lim = *sc;  // tolerances, maxits, the stop rule and the start
+  double rz = lim.rz, rz_prev = lim.rz_prev, rr = lim.rr, res = lim.res, beta_d = 0.0, alpha_d = 0.0, pap = 0.0;
+  int iter = lim.iter, state = B200LA_ITERATE;
+  cl_barrier(g.blocks);  // every block of the cluster runs and has its window
+  // maxits ends the loop; the bound only guards against broken sums
+  for (int k = 0; state == B200LA_ITERATE && k < lim.maxits + 2; ++k) {
+    double s1[1] = {g.multiply()};
+    g.template sum<1>(s1, 0);
+    pap = s1[0];
+    alpha_d = rz / pap;
+    if (!(pap != 0.0) || !isfinite(alpha_d)) {
+      state = B200LA_FAIL_BREAKDOWN;
+      break;
+    }
+    const T alpha = (T)alpha_d;
+    double s2[2];
+    g.update(alpha, s2);
+    g.template sum<2>(s2, 1);
+    rr = s2[0];
+    res = sqrt(rr);
+    ++iter;
+    state = iterate_check(iter, res, lim, lim.res_init);
+    const double rz_new = PRE ? s2[1] : rr;
+    beta_d = rz_new / rz;
+    rz_prev = rz;
+    rz = rz_new;
+    if (state == B200LA_ITERATE)
+      g.direction((T)beta_d, true, [&](int j, T p) { g.c[j] = fma(alpha, p, g.c[j]); });
+    else
+      g.each([&](int j, int li) { g.c[j] = fma(alpha, g.pw[li + g.halo], g.c[j]); });
+  }
+  if (state == B200LA_ITERATE) state = B200LA_FAIL_BREAKDOWN;  // the guard
+  g.each([&](int j, int li) {
+    const int row = g.r0 + li;
+    v.x[row] = g.c[j];
+    v.r[row] = g.r[j];
+    v.p[row] = g.pw[li + g.halo];
+  });
+  cl_barrier(g.blocks);  // no block leaves while another may still write to its shared memory
+  if (g.rank == 0 && threadIdx.x == 0) {
+    sc->rz = rz;
+    sc->rz_prev = rz_prev;
+    sc->pAp = pap;
+    sc->alpha = alpha_d;
+    sc->beta = beta_d;
+    sc->rr = rr;
+    sc->res = res;
+    sc->iter = iter;
+    sc->state = state;
+  }
+}
+
 // ---- resume after a residual replacement: x = 0, p = z + beta p ------------------
 // Every block derives beta from the same two scalars; block 0 then resets the
 // solve's scalars for the new start (none of which the other blocks read).
@@ -329,6 +542,31 @@ static int cg_build_graph_t(b200la_cg s) {
   return B200LA_OK;
 }
 
+template <typename M, typename T, bool PRE> static int cg_size_cluster_t(b200la_cg s);
+template <typename M, typename T, bool PRE> static int cg_size_resident_t(b200la_cg s);
+static int cg_resident_buffers(b200la_cg s);
+static int cg_build_graph(b200la_cg s);
+
+// Picks the form for the matrix's current schedule: one cluster, the resident
+// kernel, or the three kernels (whose graph is built here).
+static int cg_select_form(b200la_cg s) {
+  b200la_mat A = s->A;
+  s->res_blocks = 0;
+  B_TRY(cg_types(s, [&](auto m, auto t, auto pre) -> int {
+    using M = decltype(m);
+    using T = decltype(t);
+    constexpr bool PRE = decltype(pre)::value;
+    B_TRY((cg_size_cluster_t<M, T, PRE>(s)));
+    return s->cl_blocks > 0 ? B200LA_OK : cg_size_resident_t<M, T, PRE>(s);
+  }));
+  if (s->res_blocks > 0) B_TRY(cg_resident_buffers(s));
+  if (s->cl_blocks == 0 && s->res_blocks == 0) return cg_build_graph(s);
+  s->g_format = A->format;
+  s->g_param = A->param;
+  s->g_gen = A->sched_gen;
+  return B200LA_OK;
+}
+
 static int cg_build_graph(b200la_cg s) {
   return cg_types(s, [&](auto m, auto t, auto pre) -> int {
     return cg_build_graph_t<decltype(m), decltype(t), decltype(pre)::value>(s);
@@ -394,14 +632,201 @@ static int cg_host_loop_t(b200la_cg s) {
   return B200LA_OK;
 }
 
+// Shared-memory bytes per owned row of the resident kernel: x, r, p, Ap (and
+// invD) and the row's number.
+template <typename T> static size_t cg_resident_row_bytes(bool pre) { return sizeof(T) * (pre ? 5 : 4) + sizeof(int); }
+
+constexpr int kCgResThreads = 512;
+
+// Blocks of the resident form: the sums cost 1.3 / 2.6 us (without / with
+// published stores) up to 32 blocks and about twice that on more, so more
+// blocks pay once a block's rows take longer than that.  Measured, us an
+// iteration on 32 / 64 / 100 / 148 blocks: 2D 256^2 9.0 / 11.1 / 11.4 / 12.2,
+// 400^2 15.5 / 12.9 / 12.7 / 14.2, 600^2 24 / 24 / 18.3 / 18.9; 3D 32^3
+// 12.4 / 15.0 / 12.6 / 15.2, 48^3 24.6 / 18.2 / 16.5 / 16.0.
+static int cg_resident_blocks(int64_t n, int max_row, int sms) {
+  if (n <= 72000) return 32;
+  return max_row <= 12 ? std::min(100, sms) : sms;
+}
+// Beyond this many rows the graph's three kernels win (their launches and
+// the WHILE node cost ~8 us an iteration; the resident form gathers two
+// vectors instead of one): 2D 600^2 18.3 against 23.7 us, 3D 48^3 16.0
+// against 21.3, 64^3 26.0 against 27.6.
+static int64_t cg_resident_limit(int max_row) { return max_row <= 12 ? 420000 : 280000; }
+
+// Sizes the resident form, or leaves res_blocks = 0.
+template <typename M, typename T, bool PRE> static int cg_size_resident_t(b200la_cg s) {
+  s->res_blocks = 0;
+  b200la_mat A = s->A;
+  b200la_ctx c = A->ctx;
+  int optin = 0;
+  B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  // CSR chains three dependent loads (row pointer, column, gather) behind
+  // every grid-wide sum and was slower than the graph at every size tried
+  if (!is_sliced(A->format) || s->n > cg_resident_limit(A->max_row)) return B200LA_OK;
+  return with_schedule<M, T>(A, [&](auto op) -> int {
+    using Op = decltype(op);
+    constexpr int NT = kCgResThreads;
+    const void *k = (const void *)cg_resident_kernel<Op, T, PRE, NT>;
+    const int64_t threads = op.work_items() * Op::kLanes;
+    int blocks = (int)std::min<int64_t>((threads + NT - 1) / NT, c->num_sms);
+    blocks = std::max(1, std::min(blocks, cg_resident_blocks(s->n, A->max_row, c->num_sms)));
+    const int rows = op.template rows_per_block<NT>(blocks);
+    const size_t bytes = cg_resident_row_bytes<T>(PRE) * (size_t)rows;
+    cudaFuncAttributes fa;
+    B_CUDA(cudaFuncGetAttributes(&fa, k));
+    if (bytes + fa.sharedSizeBytes > (size_t)optin) return B200LA_OK;
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    int per_sm = 0;
+    B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, bytes));
+    if (per_sm < 1) return B200LA_OK;
+    s->res_blocks = blocks;
+    s->res_rows = rows;
+    return B200LA_OK;
+  });
+}
+
+constexpr int kCgClRows = 9;  // most rows a thread of the cluster form (257 x 257 nodes on 16 blocks)
+
+// Calls f(H, R) (integral constants) for a cluster solve with `up` upper
+// offsets and `regs` rows a thread.
+template <typename T, typename F> static int cl_dispatch(int up, int regs, F &&f) {
+  auto with_r = [&](auto h) -> int {
+    if (regs <= 2) return f(h, std::integral_constant<int, 2>());
+    return f(h, std::integral_constant<int, kCgClRows>());
+  };
+  return up <= 4 ? with_r(std::integral_constant<int, 4>()) : with_r(std::integral_constant<int, kClMaxOff>());
+}
+
+static ClMatrix<char> cl_matrix_head(b200la_mat A) {
+  ClMatrix<char> m{};
+  m.n = A->nrow;
+  m.H = A->cl_H;
+  m.halo = A->cl_off[A->cl_H - 1];
+  for (int k = 0; k < A->cl_H; ++k) m.off[k] = A->cl_off[k];
+  m.rowptr = A->rowptr;
+  m.col = A->col;
+  return m;
+}
+template <typename M> static ClMatrix<M> cl_matrix(b200la_mat A) {
+  const ClMatrix<char> h = cl_matrix_head(A);
+  ClMatrix<M> m{h.n, h.H, h.halo, {}, h.rowptr, h.col, (const M *)A->val};
+  for (int k = 0; k < kClMaxOff; ++k) m.off[k] = h.off[k];
+  return m;
+}
+
+// Blocks of the cluster form: a block's rows take ~0.8 ns each (FP64, nine
+// points), the two sums of an iteration 0.5 us more on 8 blocks than on one
+// and 1.5 us on 16.  Measured, us an iteration on 1 / 2 / 4 / 8 / 16 blocks
+// (the graph of three kernels 16-18): 289 rows 2.75 / 3.2 / 3.2 / 3.5 / 4.5,
+// 2,401 rows 5.2 / 4.8 / 3.3 / 3.2 / 4.1, 10,201 rows - / - / 5.8 / 5.0 / 4.3,
+// 25,921 rows 6.5 on 8, 6.2 on 16, 66,049 rows 8.4 on 16 (- : does not fit).
+static int cg_cluster_blocks(int64_t n) { return n <= kClThreads ? 1 : n <= 6000 ? 8 : kClMaxBlocks; }
+
+// Sizes the cluster form, or leaves cl_blocks = 0.
+template <typename M, typename T, bool PRE> static int cg_size_cluster_t(b200la_cg s) {
+  s->cl_blocks = 0;
+  b200la_mat A = s->A;
+  b200la_ctx c = A->ctx;
+  if (s->n > (int64_t)kClMaxBlocks * kClThreads * kCgClRows) return B200LA_OK;
+  B_TRY(cl_detect(A));
+  if (A->cl_state != 1) return B200LA_OK;
+  int optin = 0;
+  B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  const int blocks = cg_cluster_blocks(s->n);
+  const int rpc = cl_rows_per_block((int)s->n, blocks);
+  const int need = (rpc + kClThreads - 1) / kClThreads;
+  if (need > kCgClRows) return B200LA_OK;
+  const int regs = need <= 2 ? 2 : kCgClRows;
+  const size_t smem = cl_smem_bytes(rpc, A->cl_off[A->cl_H - 1], A->cl_H, sizeof(T));
+  return cl_dispatch<T>(A->cl_H, regs, [&](auto h, auto r) -> int {
+    auto k = cg_cluster_kernel<M, T, decltype(h)::value, decltype(r)::value, PRE>;
+    cudaFuncAttributes fa;
+    B_CUDA(cudaFuncGetAttributes(&fa, k));
+    if (smem + fa.sharedSizeBytes > (size_t)optin) return B200LA_OK;
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cl_config(blocks, smem, c->stream, attr);
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();  // a cluster of this size cannot be placed: another form
+      return B200LA_OK;
+    }
+    s->cl_blocks = blocks;
+    s->cl_regs = regs;
+    s->cl_smem = smem;
+    return B200LA_OK;
+  });
+}
+
+template <typename M, typename T, bool PRE> static int cg_run_cluster_t(b200la_cg s) {
+  b200la_mat A = s->A;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = cl_config(s->cl_blocks, s->cl_smem, A->ctx->stream, attr);
+  const CgVecs<T> v{(T *)s->x, (T *)s->r, (T *)s->p, (T *)s->Ap, (const T *)s->invd, s->n};
+  const ClMatrix<M> m = cl_matrix<M>(A);
+  return cl_dispatch<T>(A->cl_H, s->cl_regs, [&](auto h, auto r) -> int {
+    B_CUDA(cudaLaunchKernelEx(&cfg, cg_cluster_kernel<M, T, decltype(h)::value, decltype(r)::value, PRE>, m, v,
+                              s->sc));
+    return B200LA_OK;
+  });
+}
+
+// Buffers of the resident form, made when it is first chosen.
+static int cg_resident_buffers(b200la_cg s) {
+  if (s->tag_slots) return B200LA_OK;
+  cudaStream_t st = s->ctx->stream;
+  const size_t vb = dtype_size(s->vdtype) * (size_t)s->n;
+  if (cudaMallocAsync(&s->zg, vb, st) != cudaSuccess || cudaMallocAsync(&s->pg[0], vb, st) != cudaSuccess ||
+      cudaMallocAsync(&s->pg[1], vb, st) != cudaSuccess ||
+      cudaMallocAsync(&s->tag_slots, kTagSlotBytes, st) != cudaSuccess)
+    return fail(B200LA_ERR_NOMEM, "cg: allocation of %zu-byte gather buffers failed", vb);
+  B_CUDA(cudaMemsetAsync(s->tag_slots, 0, kTagSlotBytes, st));
+  s->epoch = 0;
+  return B200LA_OK;
+}
+
+template <typename M, typename T, bool PRE> static int cg_run_resident_t(b200la_cg s) {
+  b200la_mat A = s->A;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = A->ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)s->res_blocks);
+  cfg.blockDim = dim3(kCgResThreads);
+  cfg.dynamicSmemBytes = cg_resident_row_bytes<T>(PRE) * (size_t)s->res_rows;
+  const CgVecs<T> v{(T *)s->x, (T *)s->r, (T *)s->p, (T *)s->Ap, (const T *)s->invd, s->n};
+  const CgResidentBufs<T> rb{(T *)s->zg, (T *)s->pg[0], (T *)s->pg[1], s->res_rows};
+  const TagSync ts{(TagSlot *)s->tag_slots, &s->sc->err};
+  const unsigned long long epoch = s->epoch;
+  s->epoch += 2ull * ((unsigned long long)s->prm.maxits + 4ull);
+  return with_schedule<M, T>(A, [&](auto op) -> int {
+    using Op = decltype(op);
+    B_CUDA(cudaLaunchKernelEx(&cfg, cg_resident_kernel<Op, T, PRE, kCgResThreads>, op, v, rb, ts, epoch, s->sc));
+    return B200LA_OK;
+  });
+}
+
 int cg_run(b200la_cg s) {
   b200la_mat A = s->A;
+  if (A->format != s->g_format || A->param != s->g_param || A->sched_gen != s->g_gen) B_TRY(cg_select_form(s));
+  if (s->cl_blocks > 0)
+    return cg_types(s, [&](auto m, auto t, auto pre) -> int {
+      return cg_run_cluster_t<decltype(m), decltype(t), decltype(pre)::value>(s);
+    });
+  if (s->res_blocks > 0)
+    return cg_types(s, [&](auto m, auto t, auto pre) -> int {
+      return cg_run_resident_t<decltype(m), decltype(t), decltype(pre)::value>(s);
+    });
   if (!A->ctx->use_graphs) {
     return cg_types(s, [&](auto m, auto t, auto pre) -> int {
       return cg_host_loop_t<decltype(m), decltype(t), decltype(pre)::value>(s);
     });
   }
-  if (A->format != s->g_format || A->param != s->g_param || A->sched_gen != s->g_gen) B_TRY(cg_build_graph(s));
   B_CUDA(cudaGraphLaunch(s->exec, A->ctx->stream));
   return B200LA_OK;
 }
@@ -411,6 +836,11 @@ int cg_fetch(b200la_cg s, CgScalars *out) {
   B_CUDA(cudaMemcpyAsync(s->sc_host, s->sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
   B_CUDA(cudaStreamSynchronize(st));
   *out = *s->sc_host;
+  if (out->err != 0) {  // the blocks left at different epochs: fresh slots for the next solve
+    B_CUDA(cudaMemsetAsync(&s->sc->err, 0, sizeof(unsigned), st));
+    B_CUDA(cudaMemsetAsync(s->tag_slots, 0, kTagSlotBytes, st));
+    return fail(B200LA_ERR_TIMEOUT, "cg: a wait of the resident kernel ran out");
+  }
   return B200LA_OK;
 }
 
@@ -469,6 +899,7 @@ int b200la_cg_profile(b200la_cg s, b200la_vec b, b200la_vec x, int iters, double
   B_CHECK(s && b && x && ms && iters >= 0, B200LA_ERR_INVALID, "cg_profile: bad argument");
   B_CHECK(b->n == s->n && x->n == s->n && s->n > 0, B200LA_ERR_INVALID, "cg_profile: sizes");
   B_CHECK(b->dtype == s->vdtype && x->dtype == s->vdtype, B200LA_ERR_DTYPE, "cg_profile: dtype");
+  if (!s->exec) B_TRY(cg_build_graph(s));  // the grids of the three kernels, whatever form the solves take
   return cg_types(s, [&](auto m, auto t, auto pre) -> int {
     return cg_profile_t<decltype(m), decltype(t), decltype(pre)::value>(s, x->d, b->d, iters, ms);
   });
@@ -532,7 +963,7 @@ int b200la::cg_create_ex(b200la_mat A, const b200la_cg_params *prm, int vdtype, 
     if (rc != B200LA_OK) return cleanup(rc);
   }
   if (s->n > 0) {
-    rc = cg_build_graph(s);
+    rc = cg_select_form(s);
     if (rc != B200LA_OK) return cleanup(rc);
   }
   *out = s;
@@ -547,7 +978,7 @@ int b200la_cg_destroy(b200la_cg s) {
   cudaStreamSynchronize(st);
   if (s->exec) cudaGraphExecDestroy(s->exec);
   if (s->graph) cudaGraphDestroy(s->graph);
-  void *bufs[] = {s->x, s->r, s->p, s->Ap, s->invd, s->part, s->sc};
+  void *bufs[] = {s->x, s->r, s->p, s->Ap, s->invd, s->part, s->sc, s->zg, s->pg[0], s->pg[1], s->tag_slots};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, st);
   if (s->sc_host) cudaFreeHost(s->sc_host);

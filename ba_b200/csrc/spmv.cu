@@ -3,6 +3,7 @@
 #include <array>
 #include <vector>
 
+#include "cluster_cg.cuh"
 #include "internal.cuh"
 #include "spmv.cuh"
 
@@ -400,6 +401,70 @@ int stencil_build(b200la_mat m, int width) {
                                                         (const float *)m->val, off, (float *)d.val);
   B_CUDA(cudaGetLastError());
   B_CUDA(cudaStreamSynchronize(s));
+  return B200LA_OK;
+}
+
+// Rows that do not fit the halved storage set *bad.
+template <typename V>
+__global__ void sym_check_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+                                 const V *__restrict__ val, int *__restrict__ bad) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+    if (!sym_row_ok(rowptr, col, val, i)) *bad = 1;
+}
+
+int cl_detect(b200la_mat m) {
+  if (m->cl_state != 0) return B200LA_OK;
+  m->cl_state = -1;
+  const int n = m->nrow, E = m->max_row;
+  if (n == 0 || n != m->ncol || E < 3 || E > 2 * kClMaxOff + 1 || !(E & 1)) return B200LA_OK;
+  cudaStream_t s = m->ctx->stream;
+  // the first longest row's number, its start and columns, and the verdict
+  int *d = nullptr;
+  B_CUDA(cudaMallocAsync(&d, sizeof(int) * 2, s));
+  const int init[2] = {INT32_MAX, 0};
+  int first = 0, start = 0, cols[2 * kClMaxOff + 1], bad = 0;
+  auto cu = [](cudaError_t e) { return e == cudaSuccess; };
+  const int grid = std::min((n + kBlock - 1) / kBlock, m->ctx->num_sms * 8);
+  bool ok = cu(cudaMemcpyAsync(d, init, sizeof(init), cudaMemcpyHostToDevice, s));
+  longest_row_kernel<<<grid, kBlock, 0, s>>>(n, m->rowptr, E, d);
+  ok = ok && cu(cudaGetLastError()) && cu(cudaMemcpyAsync(&first, d, sizeof(int), cudaMemcpyDeviceToHost, s)) &&
+       cu(cudaStreamSynchronize(s));
+  if (ok && first >= 0 && first < n)
+    ok = cu(cudaMemcpyAsync(&start, m->rowptr + first, sizeof(int), cudaMemcpyDeviceToHost, s)) &&
+         cu(cudaStreamSynchronize(s)) &&
+         cu(cudaMemcpyAsync(cols, m->col + start, sizeof(int) * E, cudaMemcpyDeviceToHost, s)) &&
+         cu(cudaStreamSynchronize(s));
+  else
+    bad = 1;
+  StencilOffsets off{};
+  int H = 0;
+  if (ok && !bad) {
+    bool asc = true;
+    for (int k = 0; k < E; ++k) {
+      off.v[k] = cols[k] - first;
+      asc = asc && (k == 0 || off.v[k] > off.v[k - 1]);
+    }
+    H = asc ? cl_offsets(off.v, E, m->cl_off) : 0;
+    if (H > 0) {
+      stencil_check_kernel<<<grid, kBlock, 0, s>>>(n, m->rowptr, m->col, off, E, d + 1);
+      if (m->dtype == B200LA_F64)
+        sym_check_kernel<double><<<grid, kBlock, 0, s>>>(n, m->rowptr, m->col, (const double *)m->val, d + 1);
+      else
+        sym_check_kernel<float><<<grid, kBlock, 0, s>>>(n, m->rowptr, m->col, (const float *)m->val, d + 1);
+      ok = cu(cudaGetLastError()) && cu(cudaMemcpyAsync(&bad, d + 1, sizeof(int), cudaMemcpyDeviceToHost, s)) &&
+           cu(cudaStreamSynchronize(s));
+    }
+  }
+  cudaFreeAsync(d, s);
+  if (!ok) {
+    m->cl_state = 0;
+    return fail(B200LA_ERR_CUDA, "symmetric structure check: %s", cudaGetErrorString(cudaGetLastError()));
+  }
+  if (H > 0 && !bad) {
+    m->cl_H = H;
+    m->cl_state = 1;
+  }
   return B200LA_OK;
 }
 

@@ -3,7 +3,7 @@
 //
 // A schedule is an "operator" type with run(x, emit): every thread block
 // walks its share of the rows (grid-stride) and calls emit(row, y_row) on
-// exactly one lane per row.  The fused kernels pass emitters that also
+// exactly one lane per row (run_with: any block size and vector loader).  The fused kernels pass emitters that also
 // accumulate dot products, so the SpMV result never makes an extra trip
 // through HBM.
 #pragma once
@@ -11,6 +11,17 @@
 #include "internal.cuh"
 
 namespace b200la {
+
+// How a schedule reads the gathered vector: ld(column).  The plain form keeps
+// it in the read-only path; a kernel that writes the vector while it runs
+// brings its own.
+// at(row) gives the loader of offsets from a row, so that a row's address is
+// formed once and its entries' offsets are added to it.
+template <typename X> struct KeepLoad {
+  const X *__restrict__ x;
+  __device__ __forceinline__ X operator()(int c) const { return ld_keep(x + c); }
+  __device__ __forceinline__ KeepLoad at(int row) const { return KeepLoad{x + row}; }
+};
 
 // ---- CSR, G lanes per row (G = 1..32) -------------------------------------
 // Each warp covers 32/G consecutive rows, so a warp's loads of val/col fall
@@ -26,14 +37,33 @@ template <typename T, int G, typename X = T> struct CsrOp {
   const T *__restrict__ val;
   int n;
   static constexpr int kRowsPerBlock = kBlock / G;
+  static constexpr int kLanes = G;  // threads per row
   __host__ __device__ int64_t work_items() const { return n; }
-  template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
-    for (int base = blockIdx.x * kRowsPerBlock; base < n; base += gridDim.x * kRowsPerBlock) {
+  template <int NT, typename Ld, typename Emit>
+  __device__ __forceinline__ void run_with(const Ld &x, Emit &emit) const {
+    constexpr int rpb = NT / G;
+    for (int base = blockIdx.x * rpb; base < n; base += gridDim.x * rpb) {
       const int row = base + (int)threadIdx.x / G;
       const bool valid = row < n;
       X y = csr_row_group<T, G, X>(rowptr, col, val, x, row, valid);
       if (valid && (threadIdx.x & (G - 1)) == 0) emit(row, y);
     }
+  }
+  template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
+    run_with<kBlock>(KeepLoad<X>{x}, emit);
+  }
+  // the rows that run_with<NT> hands to this thread's emitter, in its order
+  template <int NT, typename F> __device__ __forceinline__ void each_row(F &&f) const {
+    constexpr int rpb = NT / G;
+    if (threadIdx.x & (G - 1)) return;
+    for (int base = blockIdx.x * rpb; base < n; base += gridDim.x * rpb)
+      if (base + (int)threadIdx.x / G < n) f(base + (int)threadIdx.x / G);
+  }
+  // the most rows a block of NT threads owns in a grid of `blocks`
+  template <int NT> int rows_per_block(int blocks) const {
+    constexpr int rpb = NT / G;
+    const int64_t tiles = ((int64_t)n + rpb - 1) / rpb;
+    return (int)((tiles + blocks - 1) / blocks) * rpb;
   }
 };
 
@@ -84,12 +114,31 @@ template <typename T, int W, typename X = T> struct SellOp {
   int log2c;                 // C = 1 << log2c rows per slice
   const int *__restrict__ perm;  // row of each position, or null (identity)
   static constexpr int kRowsPerBlock = kBlock;
+  static constexpr int kLanes = 1;
   __host__ __device__ int64_t work_items() const { return n; }
   template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
+    run_with<kBlock>(KeepLoad<X>{x}, emit);
+  }
+  template <int NT, typename F> __device__ __forceinline__ void each_row(F &&f) const {
+    const int lane = threadIdx.x & 31;
+    const int C = 1 << log2c, spw = 32 >> log2c;
+    const int r = lane & (C - 1), sub = lane >> log2c;
+    for (int s0 = (blockIdx.x * (NT / 32) + ((int)threadIdx.x >> 5)) * spw; s0 < nslices;
+         s0 += gridDim.x * (NT / 32) * spw) {
+      const int s = s0 + sub, pos = s * C + r;
+      if (s < nslices && pos < n) f(perm ? __ldg(perm + pos) : pos);
+    }
+  }
+  template <int NT> int rows_per_block(int blocks) const {
+    const int64_t tiles = ((int64_t)nslices * (1 << log2c) + NT - 1) / NT;
+    return (int)((tiles + blocks - 1) / blocks) * NT;
+  }
+  template <int NT, typename Ld, typename Emit>
+  __device__ __forceinline__ void run_with(const Ld &x, Emit &emit) const {
     using VV = typename VecW<T, W>::v;
     using VI = typename VecW<T, W>::i;
     const int lane = threadIdx.x & 31;
-    const int wpb = kBlock / 32;
+    constexpr int wpb = NT / 32;
     const int C = 1 << log2c, spw = 32 >> log2c;
     const int r = lane & (C - 1), sub = lane >> log2c;
     for (int s0 = (blockIdx.x * wpb + ((int)threadIdx.x >> 5)) * spw; s0 < nslices; s0 += gridDim.x * wpb * spw) {
@@ -106,7 +155,7 @@ template <typename T, int W, typename X = T> struct SellOp {
         VV vv = ld_vec_stream(vi + c * C);
 #pragma unroll
         for (int k = 0; k < W; ++k)
-          sum = fma((X)lane_get<VV, T, W>(vv, k), ld_keep(x + lane_geti<VI, W>(cc, k)), sum);
+          sum = fma((X)lane_get<VV, T, W>(vv, k), x(lane_geti<VI, W>(cc, k)), sum);
       }
       const int pos = s * C + r;
       if (live && pos < n) emit(perm ? __ldg(perm + pos) : pos, sum);
@@ -137,12 +186,31 @@ template <typename T, int W, typename X = T> struct SellOp16 {
   int log2c;                 // C = 1 << log2c rows per slice
   const int *__restrict__ perm;  // row of each position, or null (identity)
   static constexpr int kRowsPerBlock = kBlock;
+  static constexpr int kLanes = 1;
   __host__ __device__ int64_t work_items() const { return n; }
   template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
+    run_with<kBlock>(KeepLoad<X>{x}, emit);
+  }
+  template <int NT, typename F> __device__ __forceinline__ void each_row(F &&f) const {
+    const int lane = threadIdx.x & 31;
+    const int C = 1 << log2c, spw = 32 >> log2c;
+    const int r = lane & (C - 1), sub = lane >> log2c;
+    for (int s0 = (blockIdx.x * (NT / 32) + ((int)threadIdx.x >> 5)) * spw; s0 < nslices;
+         s0 += gridDim.x * (NT / 32) * spw) {
+      const int s = s0 + sub, pos = s * C + r;
+      if (s < nslices && pos < n) f(perm ? __ldg(perm + pos) : pos);
+    }
+  }
+  template <int NT> int rows_per_block(int blocks) const {
+    const int64_t tiles = ((int64_t)nslices * (1 << log2c) + NT - 1) / NT;
+    return (int)((tiles + blocks - 1) / blocks) * NT;
+  }
+  template <int NT, typename Ld, typename Emit>
+  __device__ __forceinline__ void run_with(const Ld &x, Emit &emit) const {
     using VV = typename VecW<T, W>::v;
     using VI = typename VecS<W>::i;
     const int lane = threadIdx.x & 31;
-    const int wpb = kBlock / 32;
+    constexpr int wpb = NT / 32;
     const int C = 1 << log2c, spw = 32 >> log2c;
     const int r = lane & (C - 1), sub = lane >> log2c;
     for (int s0 = (blockIdx.x * wpb + ((int)threadIdx.x >> 5)) * spw; s0 < nslices; s0 += gridDim.x * wpb * spw) {
@@ -157,6 +225,7 @@ template <typename T, int W, typename X = T> struct SellOp16 {
       // the stored offsets are relative to the row itself; padding rows
       // past n (last slice) hold offset 0 and gather x[0]
       const int row = real ? (perm ? __ldg(perm + pos) : pos) : 0;
+      const Ld xr = x.at(row);
       X sum = X(0);
 #pragma unroll 4
       for (int c = 0; c < chunks; ++c) {
@@ -164,7 +233,7 @@ template <typename T, int W, typename X = T> struct SellOp16 {
         VV vv = ld_vec_stream(vi + c * C);
 #pragma unroll
         for (int k = 0; k < W; ++k)
-          sum = fma((X)lane_get<VV, T, W>(vv, k), ld_keep(x + row + lane_gets(cc, k)), sum);
+          sum = fma((X)lane_get<VV, T, W>(vv, k), xr(lane_gets(cc, k)), sum);
       }
       if (real) emit(row, sum);
     }
@@ -190,21 +259,37 @@ template <typename T, int W, int EP, typename X = T> struct StencilOp {
   int lo, hi;  // smallest and largest offset
   int off[EP];
   static constexpr int kRowsPerBlock = kBlock;
+  static constexpr int kLanes = 1;
   __host__ __device__ int64_t work_items() const { return n; }
   template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
+    run_with<kBlock>(KeepLoad<X>{x}, emit);
+  }
+  template <int NT, typename F> __device__ __forceinline__ void each_row(F &&f) const {
+    for (int s = blockIdx.x * (NT / 32) + ((int)threadIdx.x >> 5); s < nslices; s += gridDim.x * (NT / 32)) {
+      const int row = s * 32 + (int)(threadIdx.x & 31);
+      if (row < n) f(row);
+    }
+  }
+  template <int NT> int rows_per_block(int blocks) const {
+    const int64_t tiles = ((int64_t)nslices * 32 + NT - 1) / NT;
+    return (int)((tiles + blocks - 1) / blocks) * NT;
+  }
+  template <int NT, typename Ld, typename Emit>
+  __device__ __forceinline__ void run_with(const Ld &x, Emit &emit) const {
     using VV = typename VecW<T, W>::v;
     const int lane = threadIdx.x & 31;
-    const int wpb = kBlock / 32;
+    constexpr int wpb = NT / 32;
     for (int s = blockIdx.x * wpb + ((int)threadIdx.x >> 5); s < nslices; s += gridDim.x * wpb) {
       const int row = s * 32 + lane;
       const VV *vi = reinterpret_cast<const VV *>(val + (int64_t)s * EP * 32) + lane;
       X sum = X(0);
       if (s * 32 + lo >= 0 && s * 32 + 31 + hi < n) {
+        const Ld xr = x.at(row);
 #pragma unroll
         for (int c = 0; c < EP / W; ++c) {
           const VV vv = ld_vec_stream(vi + c * 32);
 #pragma unroll
-          for (int k = 0; k < W; ++k) sum = fma((X)lane_get<VV, T, W>(vv, k), ld_keep(x + row + off[c * W + k]), sum);
+          for (int k = 0; k < W; ++k) sum = fma((X)lane_get<VV, T, W>(vv, k), xr(off[c * W + k]), sum);
         }
       } else {
 #pragma unroll
@@ -212,7 +297,7 @@ template <typename T, int W, int EP, typename X = T> struct StencilOp {
           const VV vv = ld_vec_stream(vi + c * 32);
 #pragma unroll
           for (int k = 0; k < W; ++k)
-            sum = fma((X)lane_get<VV, T, W>(vv, k), ld_keep(x + min(max(row + off[c * W + k], 0), n - 1)), sum);
+            sum = fma((X)lane_get<VV, T, W>(vv, k), x(min(max(row + off[c * W + k], 0), n - 1)), sum);
         }
       }
       if (row < n) emit(row, sum);
@@ -313,6 +398,10 @@ int sell_build(b200la_mat m, int width, bool col16 = false, int C = 32, int sigm
 // Builds the values-only copy (B200LA_FMT_STENCIL) with `width` entries per
 // vector load; B200LA_ERR_UNSUPPORTED when the matrix has no stencil.
 int stencil_build(b200la_mat m, int width);
+// Looks once for the structure the cluster-resident solver needs (m->cl_*):
+// rows that are subsets of one symmetric offset set, values symmetric up to
+// rows that hold only their diagonal.  Waits for the stream.
+int cl_detect(b200la_mat m);
 inline bool is_sell(int format) { return format == B200LA_FMT_SELL || format == B200LA_FMT_SELL16; }
 // any schedule with a sliced copy (rebuilt when the values change)
 inline bool is_sliced(int format) { return is_sell(format) || format == B200LA_FMT_STENCIL; }

@@ -589,3 +589,75 @@ def test_stencil_copy_in_the_solvers(plat):
     fmt, prm, us = A.tune()
     assert fmt in (FMT_CSR, FMT_SELL, FMT_SELL16, FMT_STENCIL) and us > 0
 
+
+
+# Sizes where the on-chip CG forms change hands or a block's rows end: one
+# block up to 512 rows (22^2 cells: 529), 8 blocks up to 6,000 (76^2: 5,929;
+# 77^2: 6,084), 16 blocks up to 9 rows a thread (256^2 fits, 260^2 does not),
+# halos wider than a block's rows (3D), the smallest stencils, then the
+# resident form on sliced copies and its limits.
+@pytest.mark.parametrize("dim,cells,fmt", [
+    (2, 2, None), (2, 3, None), (2, 21, None), (2, 22, None), (2, 76, None), (2, 77, None), (2, 131, None),
+    (2, 256, None), (3, 2, None), (3, 4, None), (3, 11, None), (3, 25, None), (3, 29, (FMT_STENCIL, 1)),
+    (2, 260, (FMT_STENCIL, 1)), (2, 268, (FMT_SELL16, 2)), (3, 41, (FMT_SELL, 1))])
+@pytest.mark.parametrize("precond", [True, False])
+def test_cg_on_chip_forms_match_oracle(plat, dim, cells, fmt, precond):
+    s = P.q1_system(dim, cells, 70 + cells, 0.5, "onchip")
+    A = _mat(plat, s)
+    if fmt:
+        A.set_format(*fmt)
+    b, x = _vec(plat, s.b), _vec(plat, np.zeros(s.n))
+    # a fixed number of steps pins the recurrence itself: every step's alpha and
+    # beta carry the rounding of dots of n terms, n eps relative at worst for
+    # the oracle's sequential sums, so k steps move x by up to k n eps
+    steps = 40
+    tol = max(1e-10, steps * s.n * np.finfo(np.float64).eps)
+    solver = lmp.setup_CG_solver(maxits=steps, atol=0.0, rtol=1e-10, dtol=1e8, use_precond=precond)
+    solver.SetupOperator(A)
+    solver.Solve(b, x)
+    ref = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=steps, atol=0.0, rtol=1e-10, precond=precond)
+    assert abs(solver.iter() - ref.iters) <= 1
+    if solver.iter() == ref.iters:
+        assert np.linalg.norm(x.numpy() - ref.x) <= tol * np.linalg.norm(ref.x)
+    # a second solve from there on the same object ends where the oracle's full solve does
+    if s.n < 20000:
+        solver.InitControl(20000, 0.0, 1e-11, 1e8)
+        x2 = _vec(plat, np.zeros(s.n))
+        assert solver.Solve(b, x2) == lmp.kSolverSuccess
+        full = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=20000, atol=0.0, rtol=1e-12, precond=precond)
+        assert np.linalg.norm(x2.numpy() - full.x) <= 1e-9 * np.linalg.norm(full.x)
+
+
+def test_cg_on_chip_form_refuses_what_it_cannot_hold(plat):
+    """Matrices whose halved storage would lose entries take another form:
+    values that are not symmetric, columns outside one symmetric offset set,
+    a repeated column; ZeroRows after the solver was made is honoured."""
+    s = P.q1_system(2, 12, 3, 1.0, "refuse")
+    rng = np.random.default_rng(5)
+    lo = s.val.copy()
+    i = s.n // 2
+    lo[s.rowptr[i]] *= 1.5  # one entry without its mirror
+    ragged = P.random_spd(120, 4, density=0.05)
+    for rp, cl, vv, b in ((s.rowptr, s.col, lo, s.b), (ragged.rowptr, ragged.col, ragged.val, ragged.b)):
+        A = lmp.B200_CSR_lMatrix(rp, cl, vv, platform=plat)
+        x = _vec(plat, np.zeros(len(b)))
+        solver = lmp.setup_CG_solver(maxits=15, atol=0.0, rtol=1e-14, dtol=1e8)
+        solver.SetupOperator(A)
+        solver.Solve(_vec(plat, b), x)
+        ref = oracle.cg(rp, cl, vv, b, maxits=15, atol=0.0, rtol=1e-14)
+        assert np.linalg.norm(x.numpy() - ref.x) <= 1e-10 * np.linalg.norm(ref.x)
+    A = _mat(plat, s)
+    solver = lmp.setup_CG_solver(maxits=5000, atol=0.0, rtol=1e-12, dtol=1e8, use_precond=False)
+    solver.SetupOperator(A)
+    x = _vec(plat, np.zeros(s.n))
+    solver.Solve(_vec(plat, s.b), x)
+    rows = rng.choice(s.n, 9, replace=False).astype(np.int32)
+    A.ZeroRows(rows, 2.0)
+    val = s.val.copy()
+    for r in rows:
+        seg = slice(s.rowptr[r], s.rowptr[r + 1])
+        val[seg] = np.where(s.col[seg] == r, 2.0, 0.0)
+    x = _vec(plat, np.zeros(s.n))
+    solver.Solve(_vec(plat, s.b), x)
+    ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=solver.iter(), atol=0.0, rtol=1e-30, precond=False)
+    assert np.linalg.norm(x.numpy() - ref.x) <= 1e-8 * np.linalg.norm(ref.x)
