@@ -53,6 +53,12 @@
 //               p = z + beta p; if it ends, x += (double)(c + alpha p) and
 //               -> RESID (mixed) or DONE (FP64 mode)
 //   DONE    skipped by every kernel
+// Systems that fit on the SMs of one thread-block cluster (cluster_cg.cuh:
+// symmetric, structured offsets, up to ~70,000 rows) do not take part in the
+// passes below: batch_cluster_kernel walks the same phases with the matrix
+// and the Krylov vectors on chip, one cluster a system, as many passes as the
+// run allows, and leaves the state as the pass kernels would.  Which form a
+// system takes depends on the system alone, never on the batch around it.
 // One pass of the device loop is K1 K2 K3; the last block of K3 ends the
 // pass and clears the graph's WHILE condition when no system is running or
 // the pass budget is spent, so the device loop always ends.
@@ -62,6 +68,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cluster_cg.cuh"
 #include "internal.cuh"
 
 namespace b200la {
@@ -87,6 +94,8 @@ template <typename T> struct SysDesc {
   double *x;
   T *c, *r, *p, *Ap;
   const T *invd;
+  int cl_H;           // upper offsets of the symmetric set (cluster form), 0: none
+  int cl_off[kClMaxOff];
   int stencil;        // 1: values-only layout, entry k of a row at column row + soff[k] (scol unused)
   int soff[kMaxStencil];  // ascending column offsets of the stencil layout (ell of them)
 };
@@ -113,6 +122,7 @@ struct SysState {
   int itb[2];                  // inner iterations done, by pass parity
   int totb[2];                 // inner iterations over all passes, by pass parity
   double tot[3];               // ticket path totals: K1 p.Ap; K2 r.r, r.z
+  int cl_passes;               // passes of the last run on a cluster
 };
 
 struct BatchParams {
@@ -951,7 +961,7 @@ template <typename T> struct SetupJob {
 // Descriptor and fresh RESID state of every job's slot (thread per job).
 template <typename T>
 __global__ void slot_init_many_kernel(const SetupJob<T> *__restrict__ jobs, int count, SysDesc<T> *desc,
-                                      SysState *st) {
+                                      SysState *st, int *sym) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     const int s = jobs[k].slot;
     desc[s] = jobs[k].d;
@@ -959,6 +969,7 @@ __global__ void slot_init_many_kernel(const SetupJob<T> *__restrict__ jobs, int 
     z.phase = PH_RESID;
     z.bad_row = 0xffffffffu;
     st[s] = z;
+    sym[s] = jobs[k].d.cl_H > 0 ? 1 : 0;
   }
 }
 
@@ -970,6 +981,200 @@ __global__ void slot_setup_many_kernel(const SetupJob<T> *__restrict__ jobs, int
     const SetupJob<T> &j = jobs[k];
     slot_setup_rows(j.d, &st[j.slot].bad_row, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (int64_t)gridDim.x * blockDim.x, j.zero_x != 0);
+  }
+}
+
+// ---- systems on one cluster ---------------------------------------------------
+// One cluster per listed system: at most `budget` passes of the phases at the
+// top of this file (an inner iteration is a pass, a residual pass covers
+// RESID and START), with the decisions of K1, K2 and K3.  All threads of the
+// cluster hold the same scalars; block 0's thread 0 writes them back.
+template <typename T, int H, int R, bool PRE>
+__global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int *__restrict__ list,
+                                                                      const SysDesc<T> *__restrict__ desc,
+                                                                      SysState *st, BatchParams prm, int budget) {
+  extern __shared__ __align__(16) unsigned char cl_dyn[];
+  const int sys = list[cl_cluster_id()];
+  const SysDesc<T> &d = desc[sys];
+  SysState &S = st[sys];
+  int phase = *(volatile int *)&S.phase;
+  if (phase != PH_RESID && phase != PH_INNER && phase != PH_START) return;
+  ClMatrix<double> m;
+  m.n = d.n;
+  m.H = d.cl_H;
+  m.halo = d.cl_off[d.cl_H - 1];
+  for (int k = 0; k < kClMaxOff; ++k) m.off[k] = d.cl_off[k];
+  m.rowptr = d.rowptr;
+  m.col = d.col;
+  m.val = d.val64;
+  const double *b = d.b;
+  double *x = d.x;
+  ClCg<T, H, R, PRE> g;
+  g.carve(cl_dyn, m);
+  g.fill(m);
+  g.load_window(d.p);
+  g.each([&](int j, int li) {
+    const int row = g.r0 + li;
+    g.r[j] = d.r[row];
+    g.c[j] = d.c[row];
+    if (PRE) g.d[j] = d.invd[row];
+  });
+  // the state as the last kernel left it (both parities alike for systems
+  // that run here; a fresh state is zero)
+  double rz = S.rzb[0], rz_keep = S.rz_keep, res = S.res, res0 = S.res0, res_in = S.res_in, res_in0 = S.res_in0;
+  int it = S.itb[0], tot = S.totb[0], outer = S.outer, keep_p = S.keep_p, state = S.state;
+  const bool diag_ok = !prm.precond || S.bad_row == 0xffffffffu;
+  unsigned long long t_begin = S.t_begin, t_done = S.t_done;
+  int set = 0, passes = 0;
+  // START left open by a run of the pass kernels: the direction, then INNER
+  auto start = [&]() {
+    const double beta_d = keep_p ? rz / rz_keep : 0.0;
+    const bool use = keep_p && isfinite(beta_d);
+    g.direction((T)beta_d, use, [](int, T) {});
+    phase = PH_INNER;
+  };
+  if (phase == PH_START && g.blocks > 1) g.each([&](int j, int li) { g.push(li, PRE ? g.r[j] * g.d[j] : g.r[j]); });
+  cl_barrier(g.blocks);  // every block of the cluster runs and has its window
+  if (phase == PH_START) start();
+  while (phase != PH_DONE && passes < budget) {
+    ++passes;
+    if (phase == PH_RESID) {
+      // the FP64 residual from the CSR, products in stored order
+      Acc<double> rr64;
+      Acc<T> rrin, rzin;
+      g.each([&](int j, int li) {
+        const int row = g.r0 + li;
+        double y = 0.0;
+        const int e = m.rowptr[row + 1];
+        for (int q = m.rowptr[row]; q < e; ++q) y = fma(m.val[q], __ldcg(x + m.col[q]), y);
+        const double r64 = b[row] - y;
+        rr64.add(r64 * r64);
+        const T r = (T)r64;
+        g.r[j] = r;
+        g.c[j] = T(0);
+        const T z = PRE ? r * g.d[j] : r;
+        rrin.add(r * r);
+        rzin.add(r * z);
+        if (g.blocks > 1) g.push(li, z);
+      });
+      double v[3] = {rr64.value(), rrin.value(), rzin.value()};
+      g.template sum<3>(v, set);
+      set ^= 1;
+      res = sqrt(v[0]);
+      if (outer == 0) {
+        res0 = res;
+        t_begin = globaltimer();
+      }
+      int s = outer_check(res, res0, prm);
+      if (s == B200LA_ITERATE && outer >= prm.max_outer) s = B200LA_FAIL_MAXITS;
+      if (outer > 0 && sqrt(v[1]) > 2.0 * res_in) keep_p = 0;
+      if (!diag_ok) s = B200LA_FAIL_BREAKDOWN;
+      if (s != B200LA_ITERATE) {
+        state = s;
+        phase = PH_DONE;
+        t_done = globaltimer();
+        break;
+      }
+      ++outer;
+      it = 0;
+      res_in = res_in0 = sqrt(v[1]);
+      rz = PRE ? v[2] : v[1];
+      start();
+      continue;
+    }
+    double s1[1] = {g.multiply()};
+    g.template sum<1>(s1, set);
+    set ^= 1;
+    const double pap = s1[0];
+    double alpha_d = rz / pap;
+    const bool ok = pap != 0.0 && isfinite(alpha_d);
+    int fin = B200LA_ITERATE;
+    bool done = true;
+    double rz_new = rz;
+    const double rz_cur = rz;
+    if (!ok) {
+      alpha_d = 0.0;  // breakdown: no step; x takes the correction so far
+      fin = B200LA_FAIL_BREAKDOWN;
+    } else {
+      double s2[2];
+      g.update((T)alpha_d, s2);
+      g.template sum<2>(s2, set);
+      set ^= 1;
+      const double rs = sqrt(s2[0]);
+      rz_new = PRE ? s2[1] : s2[0];
+      ++it;
+      ++tot;
+      res_in = rs;
+      if (prm.mixed) {
+        const double target = fmax(prm.inner_rtol * res_in0, 0.5 * prm.rtol * res0);
+        done = rs < target || it >= prm.inner_maxits || !(rs == rs);
+      } else {
+        if (rs <= prm.atol) fin = B200LA_SUCCESS_ABS;
+        else if (rs < prm.rtol * res_in0) fin = B200LA_SUCCESS_REL;
+        else if (rs > prm.dtol * res_in0) fin = B200LA_FAIL_DIV;
+        else if (it >= prm.inner_maxits) fin = B200LA_FAIL_MAXITS;
+        done = fin != B200LA_ITERATE;
+      }
+      rz = rz_new;
+    }
+    const T alpha = (T)alpha_d;
+    if (!done) {
+      g.direction((T)(rz_new / rz_cur), true, [&](int j, T p) { g.c[j] = fma(alpha, p, g.c[j]); });
+      continue;
+    }
+    rz_keep = rz_cur;
+    keep_p = (ok && isfinite(res_in) && !prm.restart_inner) ? 1 : 0;
+    g.each([&](int j, int li) {
+      const int row = g.r0 + li;
+      x[row] = __ldcg(x + row) + (double)fma(alpha, g.pw[li + g.halo], g.c[j]);
+    });
+    if (prm.mixed) {
+      phase = PH_RESID;
+      cl_barrier(g.blocks);  // the new x, for the residual's gathers
+    } else {
+      if (ok) res = res_in;
+      state = fin;
+      phase = PH_DONE;
+      t_done = globaltimer();
+    }
+  }
+  g.each([&](int j, int li) {
+    const int row = g.r0 + li;
+    d.r[row] = g.r[j];
+    d.c[row] = g.c[j];
+    d.p[row] = g.pw[li + g.halo];
+  });
+  cl_barrier(g.blocks);  // no block leaves while another may still write to its shared memory
+  if (g.rank == 0 && threadIdx.x == 0) {
+    S.phase = phase;
+    S.state = state;
+    S.outer = outer;
+    S.inner_iter = it;
+    S.total_iter = tot;
+    S.itb[0] = S.itb[1] = it;
+    S.totb[0] = S.totb[1] = tot;
+    S.rzb[0] = S.rzb[1] = rz;
+    S.rz_keep = rz_keep;
+    S.keep_p = keep_p;
+    S.res_in = res_in;
+    S.res_in0 = res_in0;
+    S.res = res;
+    S.res0 = res0;
+    S.t_begin = t_begin;
+    S.t_done = t_done;
+    S.cl_passes = passes;
+  }
+}
+
+// Whether every row of each added system fits the cluster form's halved
+// storage (its structure has been checked): sym[slot] &= verdict.
+template <typename T>
+__global__ void sym_check_many_kernel(const SetupJob<T> *__restrict__ jobs, int count, int *sym) {
+  for (int k = blockIdx.y; k < count; k += gridDim.y) {
+    const SysDesc<T> &d = jobs[k].d;
+    if (d.cl_H == 0) continue;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n; i += gridDim.x * blockDim.x)
+      if (!sym_row_ok(d.rowptr, d.col, d.val64, i)) sym[jobs[k].slot] = 0;
   }
 }
 
@@ -1043,13 +1248,16 @@ __global__ void csr_check_init_kernel(int count, CsrCheck *c) {
   }
 }
 
-// The candidate stencil of a system: the column offsets of its middle row,
-// if that row's extent lies in [0, nnz], it has 1..kMaxStencil entries and
-// its columns ascend strictly; len 0 otherwise.  Every block derives the same
-// candidate (the row is checked before it is read).
+// The candidate stencil of a system: the column offsets of its middle row or
+// the one after it, whichever is longer (on grids with an even number of
+// nodes an axis the middle row is a boundary row), if that row's extent lies
+// in [0, nnz], it has 1..kMaxStencil entries and its columns ascend strictly;
+// len 0 otherwise.  Every block derives the same candidate (the row is
+// checked before it is read).
 __device__ int stencil_candidate(int n, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
                                  int *off) {
-  const int m = n / 2;
+  int m = n / 2;
+  if (m + 1 < n && rowptr[m + 2] - rowptr[m + 1] > rowptr[m + 1] - rowptr[m]) ++m;
   const int a = rowptr[m], b = rowptr[m + 1];
   if (a < 0 || b > nnz || b - a < 1 || b - a > kMaxStencil) return 0;
   for (int j = a; j < b; ++j) {
@@ -1159,6 +1367,9 @@ struct HostSys {
   SysDesc<float> d32{};
   double *out = nullptr;   // registered host destination of the solution
   bool out_copied = false; // its copy is queued on the transfer stream
+  int cl_H = 0;            // cluster form possible if the values are symmetric (sym_host)
+  int cl_blocks = 0, cl_rows = 0;  // blocks of its cluster, rows a thread (0: does not fit)
+  size_t cl_smem = 0;
 };
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -1220,6 +1431,14 @@ struct b200la_batch_s {
   bool rm_pending;
   bool xfer_copies;   // solution copies queued on xfer since its last wait
   bool in_flight;     // a b200la_batch_launch not yet completed
+  // systems on clusters: verdicts of the symmetry check by slot, the slots of
+  // the last launch by group, and the streams that let groups overlap
+  int *sym, *sym_host;         // device, pinned host [capacity]
+  int *cl_list;                // device [capacity]
+  std::vector<int> cl_slots;   // slots of the last launch, as listed
+  int list_passes;             // passes of the pass kernels in the last run
+  cudaStream_t cl_stream[4];
+  cudaEvent_t cl_event[5];
 };
 
 namespace {
@@ -1248,6 +1467,53 @@ size_t sell_part_bytes(int64_t n, int64_t ell, bool mixed, bool col16, bool sten
 }
 size_t slot_bytes(int64_t n, int64_t nnz, int64_t ell, bool mixed, bool col16 = false) {
   return csr_part_bytes(n, nnz, mixed) + sell_part_bytes(n, ell, mixed, col16);
+}
+
+// Rows a thread of the cluster form holds (instantiated counts, ascending):
+// r, Ap, invD and c of each live in registers, 128 a thread, so 17 FP32 or 9
+// FP64 rows at most; 27-point systems run out of shared memory first.
+template <typename T, int H> struct ClRows {
+  static constexpr int n = H > 4 ? 3 : (sizeof(T) == 4 ? 6 : 4);
+  static constexpr int at(int k) {
+    constexpr int few[6] = {2, 4, 6, 9, 13, 17};
+    constexpr int wide[3] = {2, 4, sizeof(T) == 4 ? 7 : 5};
+    return H > 4 ? wide[k] : few[k];
+  }
+};
+// The smallest instantiated count that holds `need` rows, 0 if none does.
+template <typename T, int H> int cl_rows_for(int need) {
+  for (int k = 0; k < ClRows<T, H>::n; ++k)
+    if (ClRows<T, H>::at(k) >= need) return ClRows<T, H>::at(k);
+  return 0;
+}
+// f(integral constant R) for an instantiated count.
+template <typename T, int H, int K = 0, typename F> int cl_with_rows(int rows, F &&f) {
+  if constexpr (K + 1 < ClRows<T, H>::n)
+    if (rows != ClRows<T, H>::at(K)) return cl_with_rows<T, H, K + 1>(rows, f);
+  return f(std::integral_constant<int, ClRows<T, H>::at(K)>());
+}
+
+// Picks the cluster that holds a system: the smallest one it fits on, since
+// an iteration's two barriers cost the same whatever a block's rows are and
+// other systems fill the rest of the GPU.
+template <typename T> void cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
+  h.cl_H = d.cl_H;
+  h.cl_blocks = 0;
+  if (d.cl_H == 0) return;
+  int optin = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device) != cudaSuccess) return;
+  const int halo = d.cl_off[d.cl_H - 1];
+  for (int blocks = 1; blocks <= kClMaxBlocks; blocks *= 2) {
+    const int rpc = cl_rows_per_block(d.n, blocks);
+    const int need = (rpc + kClThreads - 1) / kClThreads;
+    const int held = d.cl_H <= 4 ? cl_rows_for<T, 4>(need) : cl_rows_for<T, kClMaxOff>(need);
+    const size_t smem = cl_smem_bytes(rpc, halo, d.cl_H, sizeof(T));
+    if (held == 0 || smem + 1024 > (size_t)optin) continue;
+    h.cl_blocks = blocks;
+    h.cl_rows = held;
+    h.cl_smem = smem;
+    return;
+  }
 }
 
 // Allocates a slot's CSR part (one chunk: CSR as uploaded, b, x and the
@@ -1370,6 +1636,7 @@ int finish_stage(BatchHandle B, int slot, const CsrCheck &c, SysDesc<T> &d) {
   B_TRY(alloc_sell_part<T>(B, slot, stencil ? c.slen : std::max(c.max_row, 1), col16, d, B->xfer,
                            stencil ? c.soff : nullptr));
   d.max_off = c.max_off;
+  d.cl_H = c.stencil && c.slen >= c.max_row ? cl_offsets(c.soff, c.slen, d.cl_off) : 0;
   return B200LA_OK;
 }
 
@@ -1564,8 +1831,12 @@ int ensure_items(BatchHandle B, int k, int64_t nt) {
 
 // Both item lists over the given slots (all used slots, or only those still
 // running); writes the slot count and the SpMV's algorithmic bytes.
-int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_bytes) {
+// With `on_clusters`, systems that run on clusters are left out of the lists
+// and of the count, and noted in B->cl_slots.
+int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_bytes, bool on_clusters = false) {
   for (ItemList &L : B->lst) L.host.clear();
+  B->cl_slots.clear();
+  if (on_clusters) B_CUDA(cudaEventSynchronize(B->xfer_done));  // the adds' symmetry verdicts
   int act = 0;
   int64_t bytes = 0;
   const int64_t vb = B->kp.mixed ? 4 : 8;
@@ -1575,6 +1846,10 @@ int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_byte
     if (!h.used) continue;
     const int ph = B->st_host[s].phase;
     if (running_only && (ph == PH_DONE || ph == PH_EMPTY)) continue;
+    if (on_clusters && h.cl_blocks > 0 && B->sym_host[s]) {
+      B->cl_slots.push_back(s);
+      continue;
+    }
     ++act;
     run.push_back(s);
     bytes += (int64_t)h.nnz * (vb + 4) + (int64_t)(h.n + 1) * 4 + 2 * (int64_t)h.n * vb;
@@ -1620,6 +1895,77 @@ int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_byte
   *count = act;
   if (alg_bytes) *alg_bytes = bytes;
   return B200LA_OK;
+}
+
+// Launches the listed systems' clusters: one launch per group of equal
+// cluster size, offset count and rows a thread, the largest clusters first,
+// on side streams between two events of the context stream, so that the
+// groups share the GPU.
+template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget) {
+  std::vector<int> &sl = B->cl_slots;
+  cudaStream_t st = B->ctx->stream;
+  auto key = [&](int s) {
+    const HostSys &h = B->sys[s];
+    return h.cl_blocks * 1000 + (h.cl_H > 4 ? 500 : 0) + h.cl_rows;
+  };
+  std::stable_sort(sl.begin(), sl.end(), [&](int a, int b) {
+    const int ka = key(a), kb = key(b);
+    return ka != kb ? ka > kb : B->sys[a].n > B->sys[b].n;
+  });
+  B_CUDA(cudaMemcpyAsync(B->cl_list, sl.data(), sizeof(int) * sl.size(), cudaMemcpyHostToDevice, st));
+  B_CUDA(cudaStreamSynchronize(st));  // the list is rebuilt on the host for the next launch
+  B_CUDA(cudaEventRecord(B->cl_event[4], st));
+  int used = 0, turn = 0;
+  for (size_t a = 0; a < sl.size();) {
+    size_t e = a;
+    size_t smem = 0;
+    while (e < sl.size() && key(sl[e]) == key(sl[a])) smem = std::max(smem, B->sys[sl[e++]].cl_smem);
+    const HostSys &h = B->sys[sl[a]];
+    const int q = turn++ % 4;
+    if (q >= used) {
+      B_CUDA(cudaStreamWaitEvent(B->cl_stream[q], B->cl_event[4], 0));
+      used = q + 1;
+    }
+    auto go = [&](auto hh, auto rr) -> int {
+      auto k = batch_cluster_kernel<T, decltype(hh)::value, decltype(rr)::value, PRE>;
+      B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      cudaLaunchAttribute attr[1];
+      const cudaLaunchConfig_t cfg = cl_config(h.cl_blocks, smem, B->cl_stream[q], attr, (int)(e - a));
+      B_CUDA(cudaLaunchKernelEx(&cfg, k, (const int *)(B->cl_list + a), (const SysDesc<T> *)B->desc, B->st, B->kp,
+                                budget));
+      return B200LA_OK;
+    };
+    if (h.cl_H <= 4)
+      B_TRY((cl_with_rows<T, 4>(h.cl_rows, [&](auto rr) { return go(std::integral_constant<int, 4>(), rr); })));
+    else
+      B_TRY((cl_with_rows<T, kClMaxOff>(h.cl_rows,
+                                        [&](auto rr) { return go(std::integral_constant<int, kClMaxOff>(), rr); })));
+    a = e;
+  }
+  for (int q = 0; q < used; ++q) {
+    B_CUDA(cudaEventRecord(B->cl_event[q], B->cl_stream[q]));
+    B_CUDA(cudaStreamWaitEvent(st, B->cl_event[q], 0));
+  }
+  return B200LA_OK;
+}
+
+int launch_clusters(BatchHandle B, int budget) {
+  if (B->cl_slots.empty()) return B200LA_OK;
+  const bool pre = B->kp.precond != 0;
+  if (B->kp.mixed) return pre ? launch_clusters_t<float, true>(B, budget) : launch_clusters_t<float, false>(B, budget);
+  return pre ? launch_clusters_t<double, true>(B, budget) : launch_clusters_t<double, false>(B, budget);
+}
+
+// After the states came back: adds the cluster systems of the launch to the
+// passes it took and to the systems still running.
+void count_clusters(BatchHandle B) {
+  BatchGlobals &g = *B->glob_host;
+  B->list_passes = g.passes;
+  for (int s : B->cl_slots) {
+    g.passes = std::max(g.passes, B->st_host[s].cl_passes);
+    if (B->st_host[s].phase != PH_DONE) g.active += 1;
+  }
 }
 
 // Host globals of a launch over the current lists.
@@ -1892,6 +2238,7 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
       continue;
     }
     desc_of<T>(h) = d[k];
+    cl_plan<T>(B, h, d[k]);
     SysState &s0 = B->st_host[sl[k]];
     memset(&s0, 0, sizeof(SysState));
     s0.phase = PH_RESID;
@@ -1907,10 +2254,13 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
     void *sj_dev = (char *)B->jobs_dev + align256(sizeof(CheckJob) * B->chk_cap);
     B_CUDA(cudaMemcpyAsync(sj_dev, sj, sizeof(SetupJob<T>) * nsetup, cudaMemcpyHostToDevice, st));
     slot_init_many_kernel<T><<<(nsetup + kBlock - 1) / kBlock, kBlock, 0, st>>>(
-        (const SetupJob<T> *)sj_dev, nsetup, (SysDesc<T> *)B->desc, B->st);
+        (const SetupJob<T> *)sj_dev, nsetup, (SysDesc<T> *)B->desc, B->st, B->sym);
     const dim3 grid((unsigned)std::min((max_n + 32 + kBlock - 1) / kBlock, 256), (unsigned)std::min(nsetup, 65535));
     slot_setup_many_kernel<T><<<grid, kBlock, 0, st>>>((const SetupJob<T> *)sj_dev, nsetup, B->st);
+    sym_check_many_kernel<T><<<grid, kBlock, 0, st>>>((const SetupJob<T> *)sj_dev, nsetup, B->sym);
     B_CUDA(cudaGetLastError());
+    // read when the next run lists its systems, behind the event below
+    B_CUDA(cudaMemcpyAsync(B->sym_host, B->sym, sizeof(int) * B->capacity, cudaMemcpyDeviceToHost, st));
   }
   // later work on the context stream (runs, results, removals) follows the add
   B_CUDA(cudaEventRecord(B->xfer_done, st));
@@ -1939,7 +2289,7 @@ int b200la_batch_destroy(b200la_batch B) {
   if (B->exec) cudaGraphExecDestroy(B->exec);
   if (B->graph) cudaGraphDestroy(B->graph);
   for (HostSys &h : B->sys) free_slot_memory(B, h);
-  void *bufs[] = {B->desc, B->st, B->glob, B->chk, B->sysfirst};
+  void *bufs[] = {B->desc, B->st, B->glob, B->chk, B->sysfirst, B->sym, B->cl_list};
   for (void *p : bufs)
     if (p) cudaFreeAsync(p, st);
   for (ItemList &L : B->lst) {
@@ -1953,6 +2303,11 @@ int b200la_batch_destroy(b200la_batch B) {
   if (B->chk_host) cudaFreeHost(B->chk_host);
   if (B->jobs_host) cudaFreeHost(B->jobs_host);
   if (B->glob_host) cudaFreeHost(B->glob_host);
+  if (B->sym_host) cudaFreeHost(B->sym_host);
+  for (cudaStream_t q : B->cl_stream)
+    if (q) cudaStreamDestroy(q);
+  for (cudaEvent_t q : B->cl_event)
+    if (q) cudaEventDestroy(q);
   cudaStreamSynchronize(st);
   if (B->xfer_done) cudaEventDestroy(B->xfer_done);
   if (B->rm_done) cudaEventDestroy(B->rm_done);
@@ -2001,10 +2356,17 @@ int b200la_batch_create(b200la_ctx ctx, const b200la_batch_params *p, b200la_bat
             cudaMallocAsync(&B->sysfirst, sizeof(int) * 3 * p->capacity, st) == cudaSuccess &&
             ensure_checks(B, 64) == B200LA_OK &&
             cudaMallocHost(&B->st_host, sizeof(SysState) * p->capacity) == cudaSuccess &&
-            cudaMallocHost(&B->glob_host, sizeof(BatchGlobals)) == cudaSuccess;
+            cudaMallocHost(&B->glob_host, sizeof(BatchGlobals)) == cudaSuccess &&
+            cudaMallocAsync(&B->sym, sizeof(int) * p->capacity, st) == cudaSuccess &&
+            cudaMallocAsync(&B->cl_list, sizeof(int) * p->capacity, st) == cudaSuccess &&
+            cudaMallocHost(&B->sym_host, sizeof(int) * p->capacity) == cudaSuccess &&
+            cudaMemsetAsync(B->sym, 0, sizeof(int) * p->capacity, st) == cudaSuccess;
+  for (cudaStream_t &q : B->cl_stream) ok = ok && cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t &q : B->cl_event) ok = ok && cudaEventCreateWithFlags(&q, cudaEventDisableTiming) == cudaSuccess;
   if (ok) {
     memset(B->st_host, 0, sizeof(SysState) * p->capacity);
     memset(B->glob_host, 0, sizeof(BatchGlobals));
+    memset(B->sym_host, 0, sizeof(int) * p->capacity);
     ok = cudaMemsetAsync(B->st, 0, sizeof(SysState) * p->capacity, st) == cudaSuccess &&
          cudaMemsetAsync(B->glob, 0, sizeof(BatchGlobals), st) == cudaSuccess &&
          cudaStreamSynchronize(B->xfer) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
@@ -2071,6 +2433,20 @@ int b200la_batch_add_q1(b200la_batch B, int dim, int cells, uint64_t seed, doubl
     B_TRY(alloc_sell_part<T>(B, slot, ell, B->prm.index_bits != 32 && q1_col16(dim, cells), d, st,
                              use_stencil ? stencil : nullptr));
     d.max_off = (int)std::min<int64_t>(q1_max_off(dim, cells), INT32_MAX);
+    // assembled symmetric: both rows of a pair sum the same cells in the same
+    // order, and Dirichlet rows hold only their diagonal
+    if (cells >= 2) {
+      const int64_t mm = (int64_t)cells + 1;
+      int full[kMaxStencil], k = 0;
+      for (int dz = (dim == 3 ? -1 : 0); dz <= (dim == 3 ? 1 : 0); ++dz)
+        for (int dy = -1; dy <= 1; ++dy)
+          for (int dx = -1; dx <= 1; ++dx) full[k++] = (int)(dz * mm * mm + dy * mm + dx);
+      d.cl_H = cl_offsets(full, k, d.cl_off);
+    }
+    cl_plan<T>(B, h, d);
+    B_CUDA(cudaMemsetAsync(B->sym + slot, 0, sizeof(int), st));
+    if (d.cl_H > 0) B_CUDA(cudaMemsetAsync(B->sym + slot, 1, 1, st));  // the low byte: 1
+    B_CUDA(cudaMemcpyAsync(B->sym_host, B->sym, sizeof(int) * B->capacity, cudaMemcpyDeviceToHost, st));
     B_TRY(q1_assemble(st, B->ctx->num_sms, dim, cells, seed, sigma, (int *)d.rowptr, (int *)d.col,
                       (double *)d.val64, (double *)d.b));
     B_CUDA(cudaMemsetAsync(d.x, 0, 8 * (size_t)n, st));
@@ -2202,6 +2578,37 @@ int complete_inflight(b200la_batch B) {
   B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
   B_CUDA(cudaStreamSynchronize(st));
   B->pass_total = B->glob_host->pass_total;
+  count_clusters(B);
+  return issue_early_copies(B);
+}
+
+// One run: the cluster systems for at most cluster_passes passes, then the
+// pass kernels over the others for at most max_passes.
+int run_passes(b200la_batch B, int max_passes, int cluster_passes, int *active_out) {
+  B_TRY(complete_inflight(B));
+  cudaStream_t st = B->ctx->stream;
+  int active = 0;
+  B_TRY(upload_tiles(B, true, &active, nullptr, true));
+  BatchGlobals &g = *B->glob_host;
+  if (active == 0 && B->cl_slots.empty()) {
+    g.passes = 0;
+    if (active_out) *active_out = 0;
+    return B200LA_OK;
+  }
+  if (active > 0 && B->ctx->use_graphs && !B->exec) B_TRY(build_graph(B));
+  set_globals(B, active, max_passes);
+  B_CUDA(cudaMemcpyAsync(B->glob, &g, sizeof(BatchGlobals), cudaMemcpyHostToDevice, st));
+  B_TRY(launch_clusters(B, cluster_passes));
+  if (active > 0) {
+    if (B->ctx->use_graphs) B_CUDA(cudaGraphLaunch(B->exec, st));
+    else B_TRY(host_loop(B));
+  }
+  B_CUDA(cudaMemcpyAsync(B->st_host, B->st, sizeof(SysState) * B->capacity, cudaMemcpyDeviceToHost, st));
+  B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
+  B_CUDA(cudaStreamSynchronize(st));
+  B->pass_total = B->glob_host->pass_total;
+  count_clusters(B);
+  if (active_out) *active_out = B->glob_host->active;
   return issue_early_copies(B);
 }
 }  // namespace
@@ -2213,54 +2620,37 @@ int b200la_batch_launch(b200la_batch B, int max_passes) {
   B_TRY(complete_inflight(B));
   cudaStream_t st = B->ctx->stream;
   int active = 0;
-  B_TRY(upload_tiles(B, true, &active, nullptr));
+  B_TRY(upload_tiles(B, true, &active, nullptr, true));
   BatchGlobals &g = *B->glob_host;
-  if (active == 0) return B200LA_OK;
+  if (active == 0 && B->cl_slots.empty()) return B200LA_OK;
   if (!B->ctx->use_graphs) {  // the host loop waits on the device anyway
     int a = 0;
     return b200la_batch_run(B, max_passes, &a);
   }
-  if (!B->exec) B_TRY(build_graph(B));
+  if (active > 0 && !B->exec) B_TRY(build_graph(B));
   set_globals(B, active, max_passes);
   B_CUDA(cudaMemcpyAsync(B->glob, &g, sizeof(BatchGlobals), cudaMemcpyHostToDevice, st));
-  B_CUDA(cudaGraphLaunch(B->exec, st));
+  B_TRY(launch_clusters(B, max_passes));
+  if (active > 0) B_CUDA(cudaGraphLaunch(B->exec, st));
   B->in_flight = true;
   return B200LA_OK;
 }
 
 int b200la_batch_run(b200la_batch B, int max_passes, int *active_out) {
   B_CHECK(B && max_passes >= 1, B200LA_ERR_INVALID, "batch_run: bad argument");
-  B_TRY(complete_inflight(B));
-  cudaStream_t st = B->ctx->stream;
-  int active = 0;
-  B_TRY(upload_tiles(B, true, &active, nullptr));
-  BatchGlobals &g = *B->glob_host;
-  if (active == 0) {
-    g.passes = 0;
-    if (active_out) *active_out = 0;
-    return B200LA_OK;
-  }
-  if (B->ctx->use_graphs && !B->exec) B_TRY(build_graph(B));
-  set_globals(B, active, max_passes);
-  B_CUDA(cudaMemcpyAsync(B->glob, &g, sizeof(BatchGlobals), cudaMemcpyHostToDevice, st));
-  if (B->ctx->use_graphs) B_CUDA(cudaGraphLaunch(B->exec, st));
-  else B_TRY(host_loop(B));
-  B_CUDA(cudaMemcpyAsync(B->st_host, B->st, sizeof(SysState) * B->capacity, cudaMemcpyDeviceToHost, st));
-  B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
-  B_CUDA(cudaStreamSynchronize(st));
-  B->pass_total = B->glob_host->pass_total;
-  if (active_out) *active_out = B->glob_host->active;
-  return issue_early_copies(B);
+  return run_passes(B, max_passes, max_passes, active_out);
 }
 
 int b200la_batch_solve(b200la_batch B, int chunk_passes, int *total_passes) {
   B_CHECK(B && chunk_passes >= 1, B200LA_ERR_INVALID, "batch_solve: bad argument");
-  int active = 1, total = 0;
+  int active = 1, lists = 0, total = 0;
   // each run ends after chunk_passes passes; the next run's tile list holds
   // only the systems still running, so finished systems stop costing passes
   while (active > 0) {
-    B_TRY(b200la_batch_run(B, chunk_passes, &active));
-    total += B->glob_host->passes;
+    // systems on clusters have nothing to compact: they run to their end
+    B_TRY(run_passes(B, chunk_passes, INT32_MAX, &active));
+    lists += B->list_passes;
+    total = std::max(total, std::max(lists, B->glob_host->passes));
   }
   B->glob_host->passes = total;
   if (total_passes) *total_passes = total;

@@ -156,9 +156,23 @@ __device__ __forceinline__ unsigned cl_remote(const void *p, unsigned rank) {
 __device__ __forceinline__ void cl_store(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
-__device__ __forceinline__ void cl_store(unsigned addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+__device__ __forceinline__ void cl_store_if(bool on, unsigned addr, double v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared::cluster.f64 [%0], %1;\n\t}" ::"r"(addr),
+               "d"(v), "r"((unsigned)on)
+               : "memory");
 }
+__device__ __forceinline__ void cl_store_if(bool on, unsigned addr, float v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared::cluster.f32 [%0], %1;\n\t}" ::"r"(addr),
+               "f"(v), "r"((unsigned)on)
+               : "memory");
+}
+
+// Sums of one thread's products, in FP64 whatever T is: for FP32 a conversion
+// and an addition instead of the seven operations of a compensated FP32 sum.
+struct ClAcc {
+  double s = 0.0;
+  template <typename T> __device__ __forceinline__ void add(T v) { s += (double)v; }
+};
 
 template <typename T, int H, int R, bool PRE> struct ClCg {
   static constexpr int NT = kClThreads;
@@ -168,6 +182,7 @@ template <typename T, int H, int R, bool PRE> struct ClCg {
   int n, r0, rows, rpc, halo, VW;
   unsigned rank, blocks;
   T r[R], ap[R], d[R], c[R];
+  unsigned zh_prev, zh_next;  // zh of the neighbouring blocks (shared::cluster addresses)
   unsigned diag_only;  // bit j: own row j holds only its diagonal
 
   template <typename V> __device__ __forceinline__ void carve(unsigned char *dyn, const ClMatrix<V> &m) {
@@ -187,6 +202,11 @@ template <typename T, int H, int R, bool PRE> struct ClCg {
     size_t b = sizeof(T) * ((size_t)rpc + 2 * halo + (size_t)(H + 1) * VW + 2 * (size_t)halo);
     b = (b + 15) & ~(size_t)15;
     slots = reinterpret_cast<double *>(dyn + b);
+    zh_prev = cl_remote(zh, rank > 0 ? rank - 1 : 0);
+    zh_next = cl_remote(zh, rank + 1 < blocks ? rank + 1 : rank);
+    // rows past the block's own stay zero in the loops below
+#pragma unroll
+    for (int j = 0; j < R; ++j) r[j] = d[j] = c[j] = ap[j] = T(0);
   }
 
   // Zeroes the window arrays, then every row that reaches this block's vv
@@ -233,6 +253,7 @@ template <typename T, int H, int R, bool PRE> struct ClCg {
     for (int i = max(0, base) + (int)threadIdx.x; i < hi; i += NT) pw[i - base] = __ldcg(p + i);
   }
 
+  // f(j, li) for this thread's own rows
   template <typename F> __device__ __forceinline__ void each(F &&f) {
 #pragma unroll
     for (int j = 0; j < R; ++j) {
@@ -241,49 +262,66 @@ template <typename T, int H, int R, bool PRE> struct ClCg {
     }
   }
 
-  // ap = A p; returns this thread's share of p.Ap
+  // ap = A p; returns this thread's share of p.Ap.  Straight-line over the R
+  // rows, so that the loads of one row overlap the sums of another: rows past
+  // the block's own read what lies there in shared memory (at most NT + 31
+  // values past an array's end, the sum slots at the latest) and are then
+  // set to zero, and rows that hold only their diagonal are selected.
   __device__ __forceinline__ double multiply() {
-    Acc<T> acc;
-    each([&](int j, int li) {
+    ClAcc acc;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int li = (int)threadIdx.x + j * NT;
       const int i = li + halo;
       T y = T(0);
-      if (!((diag_only >> j) & 1u)) {
 #pragma unroll
-        for (int k = H - 1; k >= 0; --k) {
-          const int q = i - off[k];
-          y = fma(vv[(k + 1) * VW + q], pw[q], y);
-        }
-        y = fma(vv[i], pw[i], y);
-#pragma unroll
-        for (int k = 0; k < H; ++k) y = fma(vv[(k + 1) * VW + i], pw[i + off[k]], y);
-      } else {
-        y = vv[i] * pw[i];
+      for (int k = H - 1; k >= 0; --k) {
+        const int q = i - off[k];
+        y = fma(vv[(k + 1) * VW + q], pw[q], y);
       }
-      ap[j] = y;
-      acc.add(y * pw[i]);
-    });
-    return acc.value();
+      const T v0 = vv[i], p0 = pw[i];
+      y = fma(v0, p0, y);
+#pragma unroll
+      for (int k = 0; k < H; ++k) y = fma(vv[(k + 1) * VW + i], pw[i + off[k]], y);
+      y = ((diag_only >> j) & 1u) ? v0 * p0 : y;
+      const bool in = li < rows;
+      ap[j] = in ? y : T(0);
+      acc.add(in ? y * p0 : T(0));
+    }
+    return acc.s;
   }
 
   // Row li's z into the zh of every other block whose window covers the row.
+  // Windows that reach only the neighbouring blocks (halo <= rpc) take two
+  // predicated stores, so the callers' loops stay free of branches.
   __device__ __forceinline__ void push(int li, T z) {
+    if (halo <= rpc) {
+      cl_store_if(li < halo && li < rows && rank > 0, zh_prev + (unsigned)sizeof(T) * (unsigned)(halo + li), z);
+      cl_store_if(li >= rpc - halo && li < rows && rank + 1 < blocks,
+                  zh_next + (unsigned)sizeof(T) * (unsigned)(li - rpc + halo), z);
+      return;
+    }
+    if (li >= rows) return;
     for (int dd = 1, first = 0; first < halo; ++dd, first += rpc) {
       if ((int)rank - dd >= 0 && li + first < halo)
-        cl_store(cl_remote(zh + halo + li + first, rank - dd), z);
+        cl_store_if(true, cl_remote(zh + halo + li + first, rank - dd), z);
       if (rank + dd < blocks && li >= dd * rpc - halo)
-        cl_store(cl_remote(zh + (li - dd * rpc + halo), rank + dd), z);
+        cl_store_if(true, cl_remote(zh + (li - dd * rpc + halo), rank + dd), z);
     }
   }
 
   // p = z + beta p over the window (own rows from r, halo rows from zh), or
   // p = z; `before(j, p_old)` sees each own row's p first.
   template <typename F> __device__ __forceinline__ void direction(T beta, bool keep, F &&before) {
-    each([&](int j, int li) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int li = (int)threadIdx.x + j * NT;
       const T z = PRE ? r[j] * d[j] : r[j];
       const T p = pw[li + halo];
       before(j, p);
-      pw[li + halo] = keep ? fma(beta, p, z) : z;
-    });
+      const T q = keep ? fma(beta, p, z) : z;
+      if (li < rows) pw[li + halo] = q;
+    }
     // halo rows outside [0, n) hold zeros in zh and stay zero
     for (int q = threadIdx.x; q < 2 * halo; q += NT) {
       const int w = q < halo ? q : rpc + q;
@@ -323,18 +361,23 @@ template <typename T, int H, int R, bool PRE> struct ClCg {
   // One step's update after alpha: r -= alpha Ap, z pushed to the windows
   // that cover it; v = this thread's shares of r.r and r.z.
   __device__ __forceinline__ void update(T alpha, double (&v)[2]) {
-    Acc<T> rr, rz;
-    const bool edge = blocks > 1;
-    each([&](int j, int li) {
+    ClAcc rr, rz;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
       const T q = fma(-alpha, ap[j], r[j]);
       r[j] = q;
       const T z = PRE ? q * d[j] : q;
       rr.add(q * q);
       if (PRE) rz.add(q * z);
-      if (edge && (li < halo || li >= rpc - halo)) push(li, z);
-    });
-    v[0] = rr.value();
-    v[1] = rz.value();
+    }
+    // the few rows other blocks' windows cover, out of the loop above
+    if (blocks > 1) {
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (j * NT < halo || (j + 1) * NT > rpc - halo) push((int)threadIdx.x + j * NT, PRE ? r[j] * d[j] : r[j]);
+    }
+    v[0] = rr.s;
+    v[1] = rz.s;
   }
 };
 

@@ -467,3 +467,62 @@ def test_column_storages_give_the_same_bits(plat, mixed):
             a, b = out[0][k], out[bits][k]
             assert a.solver_state == lmp.kSolverSuccess and (a.iters, a.outer) == (b.iters, b.outer), (k, bits)
             np.testing.assert_array_equal(a.x, b.x)
+
+
+# Sizes where the cluster form of a batch changes hands: one block up to 17
+# FP32 (9 FP64) rows a thread, then 2, 4, 8 and 16 blocks, the rows-a-thread
+# counts between, windows wider than a block's rows (3D), the pass kernels
+# beyond.  Each system is held to the FP64 oracle and must not move by a bit
+# when others run beside it or the run is cut into pieces.
+@pytest.mark.parametrize("mixed", [True, False])
+def test_cluster_systems_match_oracle_and_are_isolated(plat, mixed):
+    shapes = [(2, 2), (2, 3), (2, 31), (2, 32), (2, 44), (2, 45), (2, 54), (2, 66), (2, 67), (2, 80), (2, 92), (2, 93),
+              (2, 131), (2, 132), (3, 2), (3, 3), (3, 9), (3, 12), (3, 17), (3, 20), (3, 26)]
+    systems = [P.q1_system(d, c, 500 + k, 1.0, "cl") for k, (d, c) in enumerate(shapes)]
+    B = Batch(len(systems), mixed=mixed, precond=True, rtol=1e-9, platform=plat)
+    slots = B.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
+    B.solve()
+    res = B.results(slots)
+    for s, r in zip(systems, res):
+        assert r.solver_state == 0, (s.name, s.n, r)
+        ref = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=100000, atol=0.0, rtol=1e-13)
+        # the residual ends at 1e-9 ||b||; Jacobi-scaled systems of these sizes keep
+        # the error within 100 times that
+        assert np.linalg.norm(r.x - ref.x) <= 1e-7 * np.linalg.norm(ref.x), (s.n, r)
+        if not mixed:
+            full = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=100000, atol=0.0, rtol=1e-9)
+            assert abs(r.iters - full.iters) <= 1, (s.n, r.iters, full.iters)
+    # cut into runs of 7 passes: the state goes through global memory
+    B.restart()
+    while B.run(7):
+        pass
+    for a, c in zip(res, B.results(slots)):
+        assert a.iters == c.iters and np.array_equal(a.x, c.x)
+    B.close()
+    # alone
+    for k in (1, 9, 13, 18):
+        s = systems[k]
+        A1 = Batch(1, mixed=mixed, precond=True, rtol=1e-9, platform=plat)
+        sl = A1.add(s.rowptr, s.col, s.val, s.b)
+        A1.solve()
+        r1 = A1.result(sl)
+        assert r1.iters == res[k].iters and np.array_equal(r1.x, res[k].x)
+        A1.close()
+
+
+def test_cluster_form_refuses_unsymmetric_values(plat):
+    """An entry without its mirror keeps a system on the pass kernels, with
+    the results they give."""
+    s = P.q1_system(2, 20, 9, 0.5, "unsym")
+    val = s.val.copy()
+    val[s.rowptr[s.n // 2]] *= 1.0 + 2.0 ** -40  # one bit pattern off
+    outs = []
+    for bits in (0, 32):
+        B = Batch(1, mixed=False, precond=True, rtol=1e-10, platform=plat, index_bits=bits)
+        sl = B.add(s.rowptr, s.col, val, s.b)
+        B.solve()
+        outs.append(B.result(sl))
+        B.close()
+    assert outs[0].solver_state == 0 and np.array_equal(outs[0].x, outs[1].x)
+    ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=10000, atol=0.0, rtol=1e-13)
+    assert np.linalg.norm(outs[0].x - ref.x) <= 1e-8 * np.linalg.norm(ref.x)
