@@ -79,8 +79,10 @@ template <typename T> struct GmBufs {
 template <typename T> struct NormResEmit {
   const T *__restrict__ b;
   Acc<T> rr;
+  T br;
+  __device__ __forceinline__ void fetch(int row) { br = b[row]; }
   __device__ __forceinline__ void operator()(int row, T y) {
-    const T r = b[row] - y;
+    const T r = br - y;
     rr.add(r * r);
   }
 };
@@ -136,10 +138,15 @@ __global__ void __launch_bounds__(kBlock) gm_update_kernel(GmBufs<T> v, GmScalar
 template <typename T, bool PRE> struct RestartV0Emit {
   GmBufs<T> v;
   T inv_res;
+  T br, dr;
+  __device__ __forceinline__ void fetch(int row) {
+    br = v.b[row];
+    if (PRE) dr = v.invd[row];
+  }
   __device__ __forceinline__ void operator()(int row, T y) {
-    const T r = (v.b[row] - y) * inv_res;  // V0 = b - A x; V0.Scale(1 / res)
+    const T r = (br - y) * inv_res;  // V0 = b - A x; V0.Scale(1 / res)
     v.V[row] = r;
-    if (PRE) v.z[row] = r * v.invd[row];
+    if (PRE) v.z[row] = r * dr;
   }
 };
 
@@ -173,9 +180,11 @@ template <typename T> struct ArnoldiSpmvEmit {
   T *__restrict__ w;
   const T *__restrict__ v0;
   Acc<T> acc;
+  T vr;
+  __device__ __forceinline__ void fetch(int row) { vr = v0[row]; }
   __device__ __forceinline__ void operator()(int row, T y) {
     w[row] = y;
-    acc.add(y * v0[row]);
+    acc.add(y * vr);
   }
 };
 
@@ -726,7 +735,8 @@ static int gm_build_graph_t(GmresState *s) {
   cudaStream_t cs;
   B_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   B_CUDA(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  int rc = gm_body_t<T, PRE, true>(s, cs, h);
+  int rc = B200LA_OK;
+  for (int k = 0; k < kWhileUnroll && rc == B200LA_OK; ++k) rc = gm_body_t<T, PRE, true>(s, cs, h);
   cudaGraph_t captured;
   cudaError_t ce = cudaStreamEndCapture(cs, &captured);
   cudaStreamDestroy(cs);

@@ -98,6 +98,12 @@ struct SellData {
   int ell = 0;
   int soff[kStencilMax] = {};
   int off_lo = 0, off_hi = 0;  // smallest and largest offset
+  // symmetric half of the values-only copy (SymStencilOp); the same for
+  // every width
+  int sym = 0;
+  int sym_pair = 0;  // offsets in triples (o - 1, o, o + 1) of one parity pattern: 1 even, 2 odd (SymPairOp); 0 not
+  int sym_ld = 0, sym_pad = 0;  // values between diagonals, zeros before a diagonal's first row
+  unsigned *sym_only = nullptr;  // [nslices] rows that hold only their diagonal
 };
 
 struct b200la_mat_s {
@@ -131,6 +137,12 @@ int64_t q1_rows(int dim, int n);
 int64_t q1_nnz(int dim, int n);
 int q1_assemble(cudaStream_t st, int num_sms, int dim, int n, uint64_t seed, double sigma, int *rowptr, int *col,
                 double *val, double *b);
+
+// Passes of a solver's loop in one body of its graph's WHILE node.  The node
+// costs ~4.5 us each time it goes round (a body of one empty kernel 5.5 us,
+// of 24 kernels 27.8 us), a kernel that finds the solve ended ~1 us, so a
+// body of four passes saves 3.4 us a pass and wastes 9 kernels at the end.
+constexpr int kWhileUnroll = 4;
 
 // Launch helpers
 int grid_for(b200la_ctx ctx, const void *kernel, int64_t work_items, int items_per_block,
@@ -226,6 +238,26 @@ __device__ __forceinline__ bool grid_sum_last(double (&v)[NV], double *part, uns
 // read-only cached loads for the gathered vector.
 template <typename T> __device__ __forceinline__ T ld_stream(const T *p) { return __ldcs(p); }
 template <typename T> __device__ __forceinline__ T ld_keep(const T *p) { return __ldg(p); }
+// Read-only load that stays where it is written, so that a batch of them is
+// in flight before the first is used.
+__device__ __forceinline__ double ld_nc(const double *p) {
+  double v;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_nc(const float *p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+// Two consecutive values, the first at an even index of an aligned array.
+__device__ __forceinline__ void ld_nc2(const double *p, double &a, double &b) {
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(p));
+}
+__device__ __forceinline__ void ld_nc2(const float *p, float &a, float &b) {
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p));
+}
 
 // One row of y = A x computed by a group of G lanes of a warp (G divides 32).
 // All 32 lanes must call it (the shuffles use the full mask); lanes whose row

@@ -76,9 +76,15 @@ template <typename T> struct JacobiEmit {
   T *__restrict__ xn;
   T w;
   Acc<T> rr;
+  T br, dr, xr;
+  __device__ __forceinline__ void fetch(int row) {
+    br = b[row];
+    dr = invd[row];
+    xr = xc[row];
+  }
   __device__ __forceinline__ void operator()(int row, T y) {
-    const T r = b[row] - y;
-    xn[row] = fma(w * invd[row], r, xc[row]);
+    const T r = br - y;
+    xn[row] = fma(w * dr, r, xr);
     rr.add(r * r);
   }
 };
@@ -145,11 +151,16 @@ template <bool PRE> __device__ __forceinline__ double bicg_eps() { return PRE ? 
 template <typename T, bool PRE> struct RestartEmit {
   BiVecs<T> v;
   Acc<T> rr;
+  T br, dr;
+  __device__ __forceinline__ void fetch(int row) {
+    br = v.b[row];
+    if (PRE) dr = v.invd[row];
+  }
   __device__ __forceinline__ void operator()(int row, T y) {
-    const T r = v.b[row] - y;  // r0.ScaleAdd(b, -1): -1*(Ax) + b
+    const T r = br - y;  // r0.ScaleAdd(b, -1): -1*(Ax) + b
     v.r0[row] = r;
     v.r[row] = r;
-    v.q[row] = PRE ? r * v.invd[row] : r;
+    v.q[row] = PRE ? r * dr : r;
     rr.add(r * r);
   }
 };
@@ -159,9 +170,11 @@ template <typename T> struct StepEmit {
   T *__restrict__ Ap;
   const T *__restrict__ r0;
   Acc<T> sig, aa;
+  T rr;
+  __device__ __forceinline__ void fetch(int row) { rr = r0[row]; }
   __device__ __forceinline__ void operator()(int row, T y) {
     Ap[row] = y;
-    sig.add(y * r0[row]);
+    sig.add(y * rr);
     aa.add(y * y);
   }
 };
@@ -238,9 +251,11 @@ template <typename T> struct TEmit {
   T *__restrict__ t;
   const T *__restrict__ s;
   Acc<T> ts, tt;
+  T sr;
+  __device__ __forceinline__ void fetch(int row) { sr = s[row]; }
   __device__ __forceinline__ void operator()(int row, T y) {
     t[row] = y;
-    ts.add(y * s[row]);
+    ts.add(y * sr);
     tt.add(y * y);
   }
 };
@@ -431,7 +446,8 @@ static int solver_build_graph_t(b200la_solver s) {
   cudaStream_t cs;
   B_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   B_CUDA(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  int rc = solver_body_t<T, PRE, true>(s, cs, h);
+  int rc = B200LA_OK;
+  for (int k = 0; k < kWhileUnroll && rc == B200LA_OK; ++k) rc = solver_body_t<T, PRE, true>(s, cs, h);
   cudaGraph_t captured;
   cudaError_t ce = cudaStreamEndCapture(cs, &captured);
   cudaStreamDestroy(cs);

@@ -41,13 +41,19 @@ template <typename Op, typename R, bool PRE> struct ResidualEmit {
   const R *__restrict__ invd;
   Acc<double> rr;
   Acc<R> rr_in, rz_in;
+  double br;
+  R dr;
+  __device__ __forceinline__ void fetch(int row) {
+    br = b[row];
+    if (PRE) dr = invd[row];
+  }
   __device__ __forceinline__ void operator()(int row, double y) {
-    const double r = b[row] - y;
+    const double r = br - y;
     const R ri = (R)r;
     rin[row] = ri;
     rr.add(r * r);
     rr_in.add(ri * ri);
-    if (PRE) rz_in.add(ri * (ri * invd[row]));
+    if (PRE) rz_in.add(ri * (ri * dr));
   }
 };
 

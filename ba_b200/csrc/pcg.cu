@@ -60,11 +60,17 @@ template <typename T, bool PRE> struct InitEmit {
   const T *__restrict__ x_user;
   CgVecs<T> v;
   Acc<T> rr, rz;
+  T br, xr, dr;
+  __device__ __forceinline__ void fetch(int row) {
+    br = b[row];
+    xr = x_user[row];
+    if (PRE) dr = v.invd[row];
+  }
   __device__ __forceinline__ void operator()(int row, T y) {
-    T r = b[row] - y;  // r.ScaleAdd(b, -1): -1*(Ax) + b
-    v.x[row] = x_user[row];
+    T r = br - y;  // r.ScaleAdd(b, -1): -1*(Ax) + b
+    v.x[row] = xr;
     v.r[row] = r;
-    T z = PRE ? r * v.invd[row] : r;
+    T z = PRE ? r * dr : r;
     v.p[row] = z;
     rr.add(r * r);
     rz.add(r * z);
@@ -122,9 +128,11 @@ template <typename T> struct SpmvDotEmit {
   T *__restrict__ Ap;
   const T *__restrict__ p;
   Acc<T> acc;
+  T pr;
+  __device__ __forceinline__ void fetch(int row) { pr = __ldg(p + row); }
   __device__ __forceinline__ void operator()(int row, T y) {
     Ap[row] = y;
-    acc.add(y * __ldg(p + row));
+    acc.add(y * pr);
   }
 };
 
@@ -255,6 +263,10 @@ template <typename T> struct CgGather {
   T beta;
   __device__ __forceinline__ T operator()(int c) const { return fma(beta, po[c], z[c]); }
   __device__ __forceinline__ CgGather at(int row) const { return CgGather{z + row, po + row, beta}; }
+  __device__ __forceinline__ void pair(int c, T &a, T &b) const {
+    a = (*this)(c);
+    b = (*this)(c + 1);
+  }
 };
 
 template <typename T> struct CgResidentBufs {
@@ -269,6 +281,7 @@ template <typename T, bool PRE> struct CgGatherEmit {
   bool first;
   int at, step;  // shared-memory index of this thread's next row
   Acc<T> acc;
+  __device__ __forceinline__ void fetch(int) {}
   __device__ __forceinline__ void operator()(int row, T y) {
     T p = ps[at];
     if (!first) p = fma(beta, p, PRE ? rs[at] * ds[at] : rs[at]);
@@ -529,7 +542,8 @@ static int cg_build_graph_t(b200la_cg s) {
   cudaStream_t cs;
   B_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   B_CUDA(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  int rc = cg_launch_body_t<M, T, PRE, true>(s, cs, h);
+  int rc = B200LA_OK;
+  for (int k = 0; k < kWhileUnroll && rc == B200LA_OK; ++k) rc = cg_launch_body_t<M, T, PRE, true>(s, cs, h);
   cudaGraph_t captured;
   cudaError_t ce = cudaStreamEndCapture(cs, &captured);
   cudaStreamDestroy(cs);

@@ -159,6 +159,7 @@ void sell_free(b200la_mat m) {
   if (d.col16p) cudaFreeAsync(d.col16p, s);
   if (d.val) cudaFreeAsync(d.val, s);
   if (d.perm) cudaFreeAsync(d.perm, s);
+  if (d.sym_only) cudaFreeAsync(d.sym_only, s);
   d = SellData();
 }
 
@@ -323,16 +324,111 @@ __global__ void stencil_fill_kernel(int n, int nslices, int EP, int W, const int
   }
 }
 
+// The symmetric half: thread per row of a slice; v_k of a row that holds only
+// its diagonal is the value of the row at i + off[k] (its mirror), unless
+// that one does too.
+template <typename T>
+__global__ void sym_stencil_fill_kernel(int n, int nslices, int H, int ld, int pad, const int *__restrict__ rowptr,
+                                        const int *__restrict__ col, const T *__restrict__ val, StencilOffsets off,
+                                        T *__restrict__ sval, unsigned *__restrict__ only) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = (int)(t >> 5), row = (int)t;
+  if (s >= nslices) return;
+  const bool real = row < n;
+  const bool diag = real && diag_only_row(rowptr, col, val, row);
+  const unsigned word = __ballot_sync(0xffffffffu, diag);
+  if ((row & 31) == 0) only[s] = word;
+  int j = real ? rowptr[row] : 0;
+  const int end = real ? rowptr[row + 1] : 0;
+  while (j < end && col[j] < row) ++j;
+  for (int k = 0; k <= H; ++k) {
+    const int c = row + off.v[H + k];
+    T v = T(0);
+    if (j < end && col[j] == c) v = val[j++];
+    if (diag && k > 0 && c < n && !diag_only_row(rowptr, col, val, c))
+      for (int q = rowptr[c]; q < rowptr[c + 1]; ++q)
+        if (col[q] == row) {
+          v = val[q];
+          break;
+        }
+    sval[(int64_t)k * ld + pad + row] = v;
+  }
+}
+
+// SymPairOp's pattern of the offsets: 1 even, 2 odd, 0 neither.
+static int sym_pair_pattern(const int *off, int E) {
+  for (int t = 0; t < E / 3; ++t)
+    if (off[3 * t] != off[3 * t + 1] - 1 || off[3 * t + 2] != off[3 * t + 1] + 1) return 0;
+  for (int odd = 0; odd < 2; ++odd) {
+    bool fits = true;
+    for (int t = 0; t < E / 3; ++t) {
+      const bool want = odd && (E == 9 ? t != 1 : (((t / 3 != 1) + (t % 3 != 1)) & 1) != 0);
+      fits = fits && ((off[3 * t + 1] & 1) != 0) == want;
+    }
+    if (fits) return 1 + odd;
+  }
+  return 0;
+}
+
 int stencil_build(b200la_mat m, int width) {
   B_CHECK(width == 1 || width == 2 || width == 4, B200LA_ERR_INVALID, "STENCIL: width %d (1, 2 or 4)", width);
   SellData &cur = m->sell;
-  if (cur.stencil && cur.width == width && cur.val) return B200LA_OK;
+  // entries the copy stands for (what get_sell reports): rows of the longest
+  // row's entries rounded up to the width, also where the halved copy stores
+  // fewer
+  const int64_t stands_for = (int64_t)((m->nrow + 31) / 32) * 32 * ((m->max_row + width - 1) / width * width);
+  if (cur.stencil && cur.val && (cur.sym || cur.width == width)) {
+    cur.width = width;
+    cur.padded = stands_for;
+    return B200LA_OK;
+  }
   B_CHECK(m->nrow == m->ncol && m->nrow > 0, B200LA_ERR_UNSUPPORTED, "STENCIL: square matrices only (%dx%d)",
           m->nrow, m->ncol);
   const int E = m->max_row;
   B_CHECK(E == 9 || E == 27, B200LA_ERR_UNSUPPORTED, "STENCIL: longest row %d (9 or 27 entries)", E);
   cudaStream_t s = m->ctx->stream;
   const int n = m->nrow;
+  B_TRY(cl_detect(m));
+  if (m->cl_state == 1 && 2 * m->cl_H + 1 == E) {
+    const int H = m->cl_H, nslices = (n + 31) / 32;
+    const int pad = (m->cl_off[H - 1] + 31) & ~31;
+    const int64_t ld = (int64_t)nslices * 32 + pad, total = ld * (H + 1);
+    if (total < INT32_MAX) {
+      sell_free(m);
+      m->sched_gen += 1;
+      SellData &d = m->sell;
+      StencilOffsets off{};
+      for (int k = 0; k < E; ++k)
+        off.v[k] = d.soff[k] = k < H ? -m->cl_off[H - 1 - k] : k == H ? 0 : m->cl_off[k - H - 1];
+      d.stencil = 1;
+      d.sym = 1;
+      d.width = width;
+      d.ell = E;
+      d.nslices = nslices;
+      d.padded = stands_for;
+      d.off_lo = off.v[0];
+      d.off_hi = off.v[E - 1];
+      d.sym_ld = (int)ld;
+      d.sym_pad = pad;
+      d.sym_pair = sym_pair_pattern(off.v, E);
+      const size_t bytes = dtype_size(m->dtype) * (size_t)total;
+      B_CUDA(cudaMallocAsync(&d.val, bytes, s));
+      B_CUDA(cudaMallocAsync(&d.sym_only, sizeof(unsigned) * (size_t)nslices, s));
+      B_CUDA(cudaMemsetAsync(d.val, 0, bytes, s));
+      const int fgrid = (int)(((int64_t)nslices * 32 + kBlock - 1) / kBlock);
+      if (m->dtype == B200LA_F64)
+        sym_stencil_fill_kernel<double><<<fgrid, kBlock, 0, s>>>(n, nslices, H, d.sym_ld, pad, m->rowptr, m->col,
+                                                                 (const double *)m->val, off, (double *)d.val,
+                                                                 d.sym_only);
+      else
+        sym_stencil_fill_kernel<float><<<fgrid, kBlock, 0, s>>>(n, nslices, H, d.sym_ld, pad, m->rowptr, m->col,
+                                                                (const float *)m->val, off, (float *)d.val,
+                                                                d.sym_only);
+      B_CUDA(cudaGetLastError());
+      B_CUDA(cudaStreamSynchronize(s));
+      return B200LA_OK;
+    }
+  }
   // the offsets of the first longest row
   int *d_tmp = nullptr;
   B_CUDA(cudaMallocAsync(&d_tmp, sizeof(int) * 2, s));
@@ -510,6 +606,7 @@ extern "C" int b200la_mat_tune(b200la_mat m, int *format, int *param, double *us
       // sliced copies cost extra HBM; skip them when they would pad badly
       // (STENCIL: when the matrix has no stencil)
       if (fp[0] == B200LA_FMT_STENCIL) {
+        if (fp[1] > 1 && m->sell.sym) continue;  // one layout whatever the width
         if (b200la_mat_set_format(m, fp[0], fp[1]) != B200LA_OK) continue;
       } else if (b200la_mat_to_sell(m, fp[2], fp[3], fp[1], fp[0] == B200LA_FMT_SELL16) != B200LA_OK) {
         continue;

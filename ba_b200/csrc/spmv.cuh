@@ -2,8 +2,12 @@
 // VectorMult entry points, the autotuner and the fused CG kernels.
 //
 // A schedule is an "operator" type with run(x, emit): every thread block
-// walks its share of the rows (grid-stride) and calls emit(row, y_row) on
-// exactly one lane per row (run_with: any block size and vector loader).  The fused kernels pass emitters that also
+// walks its share of the rows (grid-stride) and, on exactly one lane per row,
+// calls emit.fetch(row) before the row's products and emit(row, y_row) after
+// them (run_with: any block size and vector loader).  An emitter loads what
+// it needs of other vectors in fetch, so that these loads overlap the row's
+// own; loaded after the sum they cost each warp another round trip per row
+// (FP64 128^3: the CG's product and dot 94 us where the product alone takes 78).  The fused kernels pass emitters that also
 // accumulate dot products, so the SpMV result never makes an extra trip
 // through HBM.
 #pragma once
@@ -21,6 +25,8 @@ template <typename X> struct KeepLoad {
   const X *__restrict__ x;
   __device__ __forceinline__ X operator()(int c) const { return ld_keep(x + c); }
   __device__ __forceinline__ KeepLoad at(int row) const { return KeepLoad{x + row}; }
+  // x[c], x[c + 1] of a loader at an even row, c even
+  __device__ __forceinline__ void pair(int c, X &a, X &b) const { ld_nc2(x + c, a, b); }
 };
 
 // ---- CSR, G lanes per row (G = 1..32) -------------------------------------
@@ -45,6 +51,7 @@ template <typename T, int G, typename X = T> struct CsrOp {
     for (int base = blockIdx.x * rpb; base < n; base += gridDim.x * rpb) {
       const int row = base + (int)threadIdx.x / G;
       const bool valid = row < n;
+      if (valid && (threadIdx.x & (G - 1)) == 0) emit.fetch(row);
       X y = csr_row_group<T, G, X>(rowptr, col, val, x, row, valid);
       if (valid && (threadIdx.x & (G - 1)) == 0) emit(row, y);
     }
@@ -148,6 +155,10 @@ template <typename T, int W, typename X = T> struct SellOp {
       const int chunks = live ? __ldg(slice_len + s) / W : 0;
       const VI *ci = reinterpret_cast<const VI *>(col + base) + r;
       const VV *vi = reinterpret_cast<const VV *>(val + base) + r;
+      const int pos = s * C + r;
+      const bool real = live && pos < n;
+      const int row = real ? (perm ? __ldg(perm + pos) : pos) : 0;
+      if (real) emit.fetch(row);
       X sum = X(0);
 #pragma unroll 4
       for (int c = 0; c < chunks; ++c) {
@@ -157,8 +168,7 @@ template <typename T, int W, typename X = T> struct SellOp {
         for (int k = 0; k < W; ++k)
           sum = fma((X)lane_get<VV, T, W>(vv, k), x(lane_geti<VI, W>(cc, k)), sum);
       }
-      const int pos = s * C + r;
-      if (live && pos < n) emit(perm ? __ldg(perm + pos) : pos, sum);
+      if (real) emit(row, sum);
     }
   }
 };
@@ -226,6 +236,7 @@ template <typename T, int W, typename X = T> struct SellOp16 {
       // past n (last slice) hold offset 0 and gather x[0]
       const int row = real ? (perm ? __ldg(perm + pos) : pos) : 0;
       const Ld xr = x.at(row);
+      if (real) emit.fetch(row);
       X sum = X(0);
 #pragma unroll 4
       for (int c = 0; c < chunks; ++c) {
@@ -282,6 +293,7 @@ template <typename T, int W, int EP, typename X = T> struct StencilOp {
     for (int s = blockIdx.x * wpb + ((int)threadIdx.x >> 5); s < nslices; s += gridDim.x * wpb) {
       const int row = s * 32 + lane;
       const VV *vi = reinterpret_cast<const VV *>(val + (int64_t)s * EP * 32) + lane;
+      if (row < n) emit.fetch(row);
       X sum = X(0);
       if (s * 32 + lo >= 0 && s * 32 + 31 + hi < n) {
         const Ld xr = x.at(row);
@@ -316,14 +328,219 @@ template <typename Op> Op stencil_op(const void *val, int n, const SellData &s) 
   return op;
 }
 
+// ---- values-only copy, symmetric half --------------------------------------
+// The stencil copy of a matrix whose values are symmetric up to rows that
+// hold only their diagonal (sym_row_ok in cluster_cg.cuh): the diagonal and
+// the H upper diagonals, v_k(i) = a(i, i + off[k]) at (k * ld + pad + i); the
+// lower entry a(i, i - off[k]) is v_k(i - off[k]), read from L2 where its row's
+// own load left it.  DRAM moves 14 values a 27-point row instead of 27
+// (FP64 128^3: product 74 -> 51 us; FP32 46 -> 40, where the requests in
+// flight bind before the bytes do).  `only` holds a bit per row that stores
+// only its diagonal; such a row's other values are taken as the zeros it
+// stores.  Products in ascending column order: SELL's bits.
+// A row's loads are issued kBatch entries at a time before their sums.
+template <typename T, int E, typename X = T> struct SymStencilOp {
+  using XT = X;
+  static constexpr int H = E / 2, kBatch = 9;
+  const T *__restrict__ val;           // v_0(0), after the front padding of the first diagonal
+  const unsigned *__restrict__ only;   // [nslices]
+  int n, nslices, ld;
+  int hi;        // largest offset
+  int off[E];    // all offsets, ascending
+  static constexpr int kRowsPerBlock = kBlock;
+  static constexpr int kLanes = 1;
+  __host__ __device__ int64_t work_items() const { return n; }
+  template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
+    run_with<kBlock>(KeepLoad<X>{x}, emit);
+  }
+  template <int NT, typename F> __device__ __forceinline__ void each_row(F &&f) const {
+    for (int s = blockIdx.x * (NT / 32) + ((int)threadIdx.x >> 5); s < nslices; s += gridDim.x * (NT / 32)) {
+      const int row = s * 32 + (int)(threadIdx.x & 31);
+      if (row < n) f(row);
+    }
+  }
+  template <int NT> int rows_per_block(int blocks) const {
+    const int64_t tiles = ((int64_t)nslices * 32 + NT - 1) / NT;
+    return (int)((tiles + blocks - 1) / blocks) * NT;
+  }
+  // y of one row; IN: every column of the slice lies in [0, n); ONLY: the
+  // slice has rows that hold only their diagonal (`diag` if this one does)
+  template <bool IN, bool ONLY, typename Ld>
+  __device__ __forceinline__ X row_sum(const Ld &x, int row, bool diag) const {
+    const Ld xr = x.at(IN ? row : 0);
+    X sum = X(0);
+#pragma unroll
+    for (int c = 0; c < E; c += kBatch) {
+      T v[kBatch];
+      X g[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (c + k < E) {
+          const int e = c + k, q = e < H ? H - e : e - H;
+          v[k] = ld_nc(val + (int64_t)q * ld + (e < H ? row + off[e] : row));
+        }
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (c + k < E) g[k] = IN ? xr(off[c + k]) : xr(min(max(row + off[c + k], 0), n - 1));
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (c + k < E) sum = fma(ONLY && diag && c + k != H ? X(0) : (X)v[k], g[k], sum);
+    }
+    return sum;
+  }
+  template <int NT, typename Ld, typename Emit>
+  __device__ __forceinline__ void run_with(const Ld &x, Emit &emit) const {
+    const int lane = threadIdx.x & 31;
+    constexpr int wpb = NT / 32;
+    for (int s = blockIdx.x * wpb + ((int)threadIdx.x >> 5); s < nslices; s += gridDim.x * wpb) {
+      const int row = s * 32 + lane;
+      const unsigned word = __ldg(only + s);
+      if (row < n) emit.fetch(row);
+      const bool diag = (word >> lane) & 1u;
+      X sum;
+      if (s * 32 - hi >= 0 && s * 32 + 31 + hi < n) {
+        sum = word == 0 ? row_sum<true, false>(x, row, false) : row_sum<true, true>(x, row, diag);
+      } else {
+        sum = row_sum<false, true>(x, row, diag);
+      }
+      if (row < n) emit(row, sum);
+    }
+  }
+};
+
+// The same copy, two consecutive rows a lane (64 rows a warp), for offsets
+// in triples (o - 1, o, o + 1) whose middle ones follow one of two parity
+// patterns (grids with m nodes an axis: multiples of m and m^2, all even when
+// m is, else odd for odd multiples).  What bounds the one-row form in FP32 is
+// not bytes but requests in flight: 54 four-byte loads a row, 128 bytes each,
+// ~250 of them outstanding per SM (27% of the L1's request rate at 5 TB/s).
+// Pairs halve the requests: own values are 8-byte (FP64: 16-byte) loads, two
+// rows share four gathered values of a triple instead of loading six, and a
+// lower value's pair is one load where its offset is even.  Products in
+// ascending column order, so the bits do not change.
+template <typename T, int E, bool ODD, typename X = T> struct SymPairOp {
+  using XT = X;
+  SymStencilOp<T, E, X> one;
+  static constexpr int H = E / 2;
+  static constexpr int kRowsPerBlock = 2 * kBlock;
+  static constexpr int kLanes = 1;
+  __host__ __device__ int64_t work_items() const { return one.n; }
+  // whether the middle offset of triple t is odd
+  __host__ __device__ static constexpr bool odd_triple(int t) {
+    return ODD && (E == 9 ? t != 1 : (((t / 3 != 1) + (t % 3 != 1)) & 1) != 0);
+  }
+  template <typename Emit> __device__ __forceinline__ void run(const X *__restrict__ x, Emit &emit) const {
+    run_with<kBlock>(KeepLoad<X>{x}, emit);
+  }
+  template <int NT, typename F> __device__ __forceinline__ void each_row(F &&f) const {
+    for (int s = blockIdx.x * (NT / 32) + ((int)threadIdx.x >> 5); s * 2 < one.nslices; s += gridDim.x * (NT / 32)) {
+      const int row = s * 64 + 2 * (int)(threadIdx.x & 31);
+      if (row < one.n) f(row);
+      if (row + 1 < one.n) f(row + 1);
+    }
+  }
+  template <int NT> int rows_per_block(int blocks) const {
+    const int64_t tiles = ((int64_t)one.nslices * 32 + 2 * NT - 1) / (2 * NT);
+    return (int)((tiles + blocks - 1) / blocks) * 2 * NT;
+  }
+  template <bool ONLY, typename Ld>
+  __device__ __forceinline__ void pair_sum(const Ld &x, int row, bool d0, bool d1, X &y0, X &y1) const {
+    const Ld xr = x.at(row);
+    X s0 = X(0), s1 = X(0);
+#pragma unroll
+    for (int p = 0; p < E; p += 9) {
+      T v0[9], v1[9];
+      X g[3][4];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const int e = p + k;
+        if (e >= H) {
+          ld_nc2(one.val + (int64_t)(e - H) * one.ld + row, v0[k], v1[k]);
+        } else {
+          const T *q = one.val + (int64_t)(H - e) * one.ld + (row + one.off[e]);
+          if (odd_triple(e / 3) == (e % 3 == 1)) {  // odd offset
+            v0[k] = ld_nc(q);
+            v1[k] = ld_nc(q + 1);
+          } else {
+            ld_nc2(q, v0[k], v1[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const int o = one.off[p + 3 * t + 1];
+        if (odd_triple(p / 3 + t)) {
+          xr.pair(o - 1, g[t][0], g[t][1]);
+          xr.pair(o + 1, g[t][2], g[t][3]);
+        } else {
+          g[t][0] = xr(o - 1);
+          xr.pair(o, g[t][1], g[t][2]);
+          g[t][3] = xr(o + 2);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        s0 = fma(ONLY && d0 && p + k != H ? X(0) : (X)v0[k], g[k / 3][k % 3], s0);
+        s1 = fma(ONLY && d1 && p + k != H ? X(0) : (X)v1[k], g[k / 3][k % 3 + 1], s1);
+      }
+    }
+    y0 = s0;
+    y1 = s1;
+  }
+  template <int NT, typename Ld, typename Emit>
+  __device__ __forceinline__ void run_with(const Ld &x, Emit &emit) const {
+    const int lane = threadIdx.x & 31;
+    constexpr int wpb = NT / 32;
+    const int n = one.n;
+    for (int s = blockIdx.x * wpb + ((int)threadIdx.x >> 5); s * 2 < one.nslices; s += gridDim.x * wpb) {
+      const int row = s * 64 + 2 * lane;
+      const unsigned w0 = __ldg(one.only + 2 * s), w1 = 2 * s + 1 < one.nslices ? __ldg(one.only + 2 * s + 1) : 0u;
+      // the second row's vectors lie in the lines the first row's fetch brings
+      if (row < n) emit.fetch(row);
+      const unsigned bits = (lane < 16 ? w0 >> (2 * lane) : w1 >> (2 * lane - 32)) & 3u;
+      const bool d0 = bits & 1u, d1 = bits & 2u;
+      X y0, y1;
+      if (s * 64 - one.hi >= 0 && s * 64 + 63 + one.hi < n) {
+        if ((w0 | w1) == 0) pair_sum<false>(x, row, false, false, y0, y1);
+        else pair_sum<true>(x, row, d0, d1, y0, y1);
+      } else {
+        // rows past the last slice take the last row's place
+        const int last = one.nslices * 32 - 1;
+        y0 = one.template row_sum<false, true>(x, min(row, last), d0);
+        y1 = one.template row_sum<false, true>(x, min(row + 1, last), d1);
+      }
+      if (row < n) emit(row, y0);
+      if (row + 1 < n) {
+        emit.fetch(row + 1);
+        emit(row + 1, y1);
+      }
+    }
+  }
+};
+
+template <typename Op> Op sym_stencil_op(const void *val, int n, const SellData &s) {
+  Op op;
+  op.val = (decltype(op.val))val + s.sym_pad;
+  op.only = s.sym_only;
+  op.n = n;
+  op.nslices = s.nslices;
+  op.ld = s.sym_ld;
+  op.hi = s.off_hi;
+  for (int k = 0; k < (int)(sizeof(op.off) / sizeof(int)); ++k) op.off[k] = s.soff[k];
+  return op;
+}
+
 // ---- plain emitters --------------------------------------------------------
 template <typename T> struct StoreEmit {
   T *__restrict__ y;
+  __device__ __forceinline__ void fetch(int) {}
   __device__ __forceinline__ void operator()(int row, T v) { y[row] = v; }
 };
 template <typename T> struct AddEmit {
   T *__restrict__ y;
-  __device__ __forceinline__ void operator()(int row, T v) { y[row] += v; }
+  T y0;
+  __device__ __forceinline__ void fetch(int row) { y0 = y[row]; }
+  __device__ __forceinline__ void operator()(int row, T v) { y[row] = y0 + v; }
 };
 
 template <typename Op, typename T, bool ADD>
@@ -366,6 +583,22 @@ template <typename T, typename X = T, typename F> int with_schedule(b200la_mat m
   }
   if (m->format == B200LA_FMT_STENCIL) {
     const SellData &s = m->sell;
+    // FP64 requests are wide enough as they are (128^3 CG product 69 us with
+    // one row a lane, 73 with two; FP32 Jacobi sweep 96^3 31 and 25)
+    if constexpr (sizeof(T) == 4) {
+      if (s.sym_pair && s.ell == 9) {
+        const auto one = sym_stencil_op<SymStencilOp<T, 9, X>>(s.val, m->nrow, s);
+        return s.sym_pair == 2 ? f(SymPairOp<T, 9, true, X>{one}) : f(SymPairOp<T, 9, false, X>{one});
+      }
+      if (s.sym_pair) {
+        const auto one = sym_stencil_op<SymStencilOp<T, 27, X>>(s.val, m->nrow, s);
+        return s.sym_pair == 2 ? f(SymPairOp<T, 27, true, X>{one}) : f(SymPairOp<T, 27, false, X>{one});
+      }
+    }
+    if (s.sym) {
+      if (s.ell == 9) return f(sym_stencil_op<SymStencilOp<T, 9, X>>(s.val, m->nrow, s));
+      return f(sym_stencil_op<SymStencilOp<T, 27, X>>(s.val, m->nrow, s));
+    }
     const int key = m->param * 100 + s.ell;
     switch (key) {
       case 109: return f(stencil_op<StencilOp<T, 1, 9, X>>(s.val, m->nrow, s));
