@@ -9,18 +9,20 @@
 //   G2  at a (re)start: V0 = (b - A x) / res, z = P V0, reset H and g
 //   G3  w = A z (z = P V_j, or V_j itself without preconditioner), fused
 //       with the partial sums of w.V_0
-//   G4  the rest of the Arnoldi step in one cooperative kernel: for
-//       i = 0..j, h_ij from the previous partial sums (every block adds
-//       them in the same order), w -= h_ij V_i fused with the next dot
-//       (w.V_{i+1}, or w.w at the end), one grid barrier per i; then
-//       V_{j+1} = w / ||w||, z = P V_{j+1}; block 0 applies the Givens
-//       rotations, the test, and at a cycle end solves H y = g.  When w
+//   G4  the rest of the Arnoldi step in one cooperative kernel.  When w
 //       fits in the SMs' shared memory (up to ~4.3 M FP64 rows on 148
-//       SMs) it stays there for the whole step.
+//       SMs): all dots in one pass over the basis, the Gram-Schmidt
+//       coefficients from them, w - sum h_ij V_i in a second pass (two grid
+//       barriers).  Else, streaming: for i = 0..j, h_ij from the previous
+//       partial sums (every block adds them in the same order), w -= h_ij V_i
+//       fused with the next dot, one grid barrier per i.  Then
+//       V_{j+1} = w / ||w||, z = P V_{j+1}; block 0 applies the Givens
+//       rotations, the test, and at a cycle end solves H y = g.
 // The reference runs the Gram-Schmidt loop as 2 (j+1) separate BLAS-1 calls
 // with a blocking scalar read each; here one launch covers it and the host
 // never waits.  As in the reference, a restart normalises V0 by the
 // recurrence residual |g[j+1]|, not by V0's own norm.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -381,19 +383,24 @@ __global__ void __launch_bounds__(kBlock) gm_arnoldi_kernel(GmBufs<T> v, const d
 
 // Resident form: one block of kResBlock threads per SM, block b owning the
 // slice [b S, b S + S) of w (S a multiple of the 16-byte vector) in shared
-// memory for the whole step.  w is read from global memory once (G3 wrote
-// it) and V_{j+1} (and z) written once at the end; in between, projection i
-// reads only V_i, already in L2 since projection i-1's dot, and V_{i+1},
-// which projection i-1 prefetched into L2 before its grid barrier, so the
-// barrier's wait overlaps the DRAM read.  Each thread owns the 16-byte
-// chunks k = threadIdx.x + t kResBlock of the slice in every pass (so the
-// slice needs no block barrier of its own) and walks them kResUnroll at a
-// time, loads first, to keep that many loads in flight.  Same arithmetic per
-// element as the streaming form, and the same per-thread order; only the
-// partition of the dot products into partial sums differs.  (Measured on
-// the 2.1 M-row Poisson matrix: 1024 threads with 2 loads in flight beat
-// 1024 x 1 and 512 x 4, and a barrier-free all-gather of tagged partials
-// was slower than this barrier.)
+// memory for the whole step, in two passes over the basis and two grid
+// barriers whatever j is.
+//
+// What bounds the step: modified Gram-Schmidt is a chain of j + 1 dependent
+// dots, and one grid barrier each (3.4 us with its sums) was 90 us of a step
+// at j = 26 on 274,625 rows, where the basis itself streams from L2 in 4 us.
+// The chain's coefficients are the solution of a unit triangular system,
+//   h_i = V_i.w - sum_{k<i} (V_i.V_k) h_k,
+// which is what subtracting one projection after the other computes (the
+// products V_i.V_k of earlier steps are kept in G, row j's come with this
+// step's dots), so one pass gives every V_i.w and V_j.V_i, every block solves
+// the same small system, and a second pass forms w - sum h_i V_i and its norm.
+//   dots    warp q takes basis vectors q, q + 32, ...: a lane adds its chunks
+//           of the slice, one shuffle tree a vector, one partial a block
+//   solve   h = a - L h repeated until no bit changes: L is strictly lower
+//           triangular, so this is exact after at most j + 1 rounds, and two
+//           or three do when the basis is orthogonal to rounding
+//   update  thread t owns chunks t + q kResBlock of the slice
 constexpr int kResBlock = 1024;
 constexpr int kResUnroll = 2;
 
@@ -449,21 +456,12 @@ __device__ __forceinline__ bool projection_total(double v, double *set, unsigned
   return okf != 0;
 }
 
-template <typename T>
-__device__ __forceinline__ void prefetch_slice_l2(const T *p, int64_t len) {
-  const char *c = reinterpret_cast<const char *>(p);
-  const int64_t bytes = len * (int64_t)sizeof(T);
-  for (int64_t o = (int64_t)threadIdx.x * 128; o < bytes; o += (int64_t)blockDim.x * 128)
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(c + o));
-}
-
 template <typename T, bool PRE, bool IN_GRAPH>
-__global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> v, const double *part3, int n3,
-                                                                      double *part4, GmScalars *sc, int64_t S,
+__global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> v, double *part4, double *G,
+                                                                      GmScalars *sc, int64_t S, bool two,
                                                                       cudaGraphConditionalHandle loop) {
   constexpr int W = Vec16<T>::n, U = kResUnroll;
   extern __shared__ __align__(16) unsigned char gm_dyn[];
-  T *ws = reinterpret_cast<T *>(gm_dyn);
   const int phase = __ldg(&sc->phase);
   if (phase != kGmStep) {
     gm_idle<IN_GRAPH>(sc, phase, loop);
@@ -471,69 +469,157 @@ __global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> 
   }
   const int j = __ldg(&sc->j);
   const int m = __ldg(&sc->m), ldh = m + 1;
+  // shared memory: V_i.w, V_j.V_i and two rounds of h, then the slices
+  double *ash = reinterpret_cast<double *>(gm_dyn), *gsh = ash + ldh, *hsh[2] = {gsh + ldh, gsh + 2 * ldh};
+  T *ws = reinterpret_cast<T *>(gsh + 3 * ldh);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NW = kResBlock / 32;
   const int64_t lo = (int64_t)blockIdx.x * S;
   const int64_t len = lo < v.n ? (v.n - lo < S ? v.n - lo : S) : 0;
   const int64_t nv = len / W;               // whole chunks; elements nv W .. len-1 are the tail
   const int64_t bd = blockDim.x;
   const bool stall = (int)blockIdx.x == __ldg(&sc->stall_block);
   const unsigned long long bar0 = __ldg(&sc->bar_done);
-  prefetch_slice_l2(v.V + lo, len);
-  if (j > 0) prefetch_slice_l2(v.V + v.ldv + lo, len);
-  // w's slice into shared memory
+  // w's slice into shared memory, and V_j's where both fit
+  const T *vj = v.V + (int64_t)j * v.ldv + lo;
+  T *vs = two ? ws + S : nullptr;
   for (int64_t k0 = threadIdx.x; k0 < nv; k0 += U * bd) {
-    T t[U][W];
+    T t[U][W], q[U][W];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (k0 + u * bd < nv) ld<W>(v.w + lo + (k0 + u * bd) * W, t[u]);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (k0 + u * bd < nv) st<W>(ws + (k0 + u * bd) * W, t[u]);
-  }
-  for (int64_t e = nv * W + threadIdx.x; e < len; e += bd) ws[e] = v.w[lo + e];
-  double h = block_total(part3, n3);
-  for (int i = 0; i <= j; ++i) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) v.H[j * ldh + i] = h;
-    const T hi = (T)h;
-    const T *vi = v.V + (int64_t)i * v.ldv + lo;
-    const T *vn = i < j ? v.V + (int64_t)(i + 1) * v.ldv + lo : nullptr;
-    Acc<T> acc;
-    for (int64_t k0 = threadIdx.x; k0 < nv; k0 += U * bd) {
-      T a[U][W], bn[U][W];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t k = k0 + u * bd;
-        if (k < nv) {
-          ld<W>(vi + k * W, a[u]);
-          if (vn) ld<W>(vn + k * W, bn[u]);
-        }
+      if (k0 + u * bd < nv) {
+        ld<W>(v.w + lo + (k0 + u * bd) * W, t[u]);
+        if (two) ld<W>(vj + (k0 + u * bd) * W, q[u]);
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t k = k0 + u * bd;
-        if (k < nv) {
-          T wv[W];
-          ld<W>(ws + k * W, wv);
+    for (int u = 0; u < U; ++u)
+      if (k0 + u * bd < nv) {
+        st<W>(ws + (k0 + u * bd) * W, t[u]);
+        if (two) st<W>(vs + (k0 + u * bd) * W, q[u]);
+      }
+  }
+  for (int64_t e = nv * W + threadIdx.x; e < len; e += bd) {
+    ws[e] = v.w[lo + e];
+    if (two) vs[e] = vj[e];
+  }
+  __syncthreads();
+  // dots: part4 holds [2 (m + 1)][gridDim.x], column i = V_i.w, column
+  // m + 1 + i = V_i.V_j
+  const T *vjr = two ? vs : vj;
+  for (int i = warp; i <= j; i += NW) {
+    const T *vi = v.V + (int64_t)i * v.ldv + lo;
+    Acc<T> aw, ag;
+    constexpr int UD = 4;
+    for (int64_t k0 = lane; k0 < nv; k0 += UD * 32) {
+      T a[UD][W];
+#pragma unroll
+      for (int u = 0; u < UD; ++u)
+        if (k0 + u * 32 < nv) ld<W>(vi + (k0 + u * 32) * W, a[u]);
+#pragma unroll
+      for (int u = 0; u < UD; ++u)
+        if (k0 + u * 32 < nv) {
+          T wv[W], gv[W];
+          ld<W>(ws + (k0 + u * 32) * W, wv);
+          ld<W>(vjr + (k0 + u * 32) * W, gv);
 #pragma unroll
           for (int q = 0; q < W; ++q) {
-            wv[q] = fma(-hi, a[u][q], wv[q]);
-            acc.add(wv[q] * (vn ? bn[u][q] : wv[q]));
+            aw.add(wv[q] * a[u][q]);
+            ag.add(gv[q] * a[u][q]);
           }
-          st<W>(ws + k * W, wv);
         }
+    }
+    for (int64_t e = nv * W + lane; e < len; e += 32) {
+      aw.add(ws[e] * vi[e]);
+      ag.add(vjr[e] * vi[e]);
+    }
+    const double sw = warp_sum(aw.value()), sg = warp_sum(ag.value());
+    if (lane == 0) {
+      part4[(int64_t)i * gridDim.x + blockIdx.x] = sw;
+      part4[(int64_t)(ldh + i) * gridDim.x + blockIdx.x] = sg;
+    }
+  }
+  if (stall) return;  // test hook: this block never reaches the barrier
+  if (!grid_barrier_count(&sc->bar_count, (bar0 + 1ull) * gridDim.x, &sc->err)) {
+    gm_abort<IN_GRAPH>(sc, loop);
+    return;
+  }
+  // every block adds the same partials in the same order
+  for (int c = warp; c < 2 * (j + 1); c += NW) {
+    const int i = c >> 1;
+    const double *p = part4 + (int64_t)((c & 1) ? ldh + i : i) * gridDim.x;
+    double t = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
+    t = warp_sum(t);
+    if (lane == 0) {
+      if (c & 1) {
+        gsh[i] = t;
+        if (blockIdx.x == 0 && i < j) G[(int64_t)j * ldh + i] = t;
+      } else {
+        ash[i] = t;
+        hsh[0][i] = t;
       }
     }
-    for (int64_t e = nv * W + threadIdx.x; e < len; e += bd) {
-      const T wv = fma(-hi, vi[e], ws[e]);
-      acc.add(wv * (vn ? vn[e] : wv));
-      ws[e] = wv;
+  }
+  __syncthreads();
+  int cur = 0;
+  for (int round = 0; round <= j; ++round) {
+    int changed = 0;
+    for (int i = warp; i <= j; i += NW) {
+      double t = 0.0;
+      const double *row = G + (int64_t)i * ldh;
+      for (int k = lane; k < i; k += 32) t = fma(i == j ? gsh[k] : row[k], hsh[cur][k], t);
+      t = warp_sum(t);
+      const double hi = ash[i] - t;
+      changed |= !(hi == hsh[cur][i]);
+      if (lane == 0) hsh[cur ^ 1][i] = hi;
     }
-    if (i + 2 <= j) prefetch_slice_l2(v.V + (int64_t)(i + 2) * v.ldv + lo, len);
-    if (stall) return;  // test hook: this block never reaches the barrier
-    if (!projection_total(acc.value(), part4 + (i & 1) * gridDim.x, &sc->bar_count,
-                          (bar0 + (unsigned long long)i + 1ull) * gridDim.x, &sc->err, &h)) {
-      gm_abort<IN_GRAPH>(sc, loop);
-      return;
+    cur ^= 1;
+    if (!__syncthreads_or(changed)) break;
+  }
+  const double *hs = hsh[cur];
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i <= j; i += bd) v.H[j * ldh + i] = hs[i];
+  // w -= sum h_i V_i (the type's own arithmetic, in the chain's order), ||w||^2
+  Acc<T> acc;
+  for (int64_t k = threadIdx.x; k < nv; k += bd) {
+    T wv[W];
+    ld<W>(ws + k * W, wv);
+    const T *vk = v.V + lo + k * W;
+    constexpr int UV = 4;
+    int i = 0;
+    for (; i + UV <= j + 1; i += UV) {
+      T a[UV][W];
+#pragma unroll
+      for (int u = 0; u < UV; ++u) ld<W>(vk + (int64_t)(i + u) * v.ldv, a[u]);
+#pragma unroll
+      for (int u = 0; u < UV; ++u) {
+        const T hi = (T)hs[i + u];
+#pragma unroll
+        for (int q = 0; q < W; ++q) wv[q] = fma(-hi, a[u][q], wv[q]);
+      }
     }
+    for (; i <= j; ++i) {
+      T a[W];
+      ld<W>(vk + (int64_t)i * v.ldv, a);
+      const T hi = (T)hs[i];
+#pragma unroll
+      for (int q = 0; q < W; ++q) wv[q] = fma(-hi, a[q], wv[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < W; ++q) acc.add(wv[q] * wv[q]);
+    st<W>(ws + k * W, wv);
+  }
+  for (int64_t e = nv * W + threadIdx.x; e < len; e += bd) {
+    T wv = ws[e];
+    for (int i = 0; i <= j; ++i) wv = fma(-(T)hs[i], v.V[(int64_t)i * v.ldv + lo + e], wv);
+    acc.add(wv * wv);
+    ws[e] = wv;
+  }
+  double h;
+  double *norms = part4 + (int64_t)2 * ldh * gridDim.x;
+  if (!projection_total(acc.value(), norms, &sc->bar_count, (bar0 + 2ull) * gridDim.x, &sc->err, &h)) {
+    gm_abort<IN_GRAPH>(sc, loop);
+    return;
   }
   // V_{j+1} = w / ||w||, z = P V_{j+1}
   const T hn = sqrt((T)h);
@@ -569,8 +655,8 @@ __global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> 
   }
   if (blockIdx.x != 0) return;
   // every block read bar_done at its start, and block 0 gets here only after
-  // all arrived at barrier j
-  if (threadIdx.x == 0) sc->bar_done = bar0 + (unsigned long long)j + 1ull;
+  // all arrived at both barriers
+  if (threadIdx.x == 0) sc->bar_done = bar0 + 2ull;
   gm_step_end<IN_GRAPH>(v.H, v.g, v.cs, v.sn, v.y, sc, j, m, (double)hn, loop);
 }
 
@@ -597,6 +683,8 @@ struct GmresState {
   int grid_start, grid_restart, grid_spmv, grid_ew, grid_coop;
   int grid_res;              // blocks of the resident Arnoldi kernel (0: streaming form)
   int64_t res_slice;         // elements of w per block there
+  bool res_two;              // the block holds V_j's slice too
+  double *G;                 // [m + 1][m + 1]: V_i . V_k at i (m + 1) + k, k < i
 };
 
 template <typename T> static GmBufs<T> gm_bufs(const GmresState *s) {
@@ -606,6 +694,9 @@ template <typename T> static GmBufs<T> gm_bufs(const GmresState *s) {
   return GmBufs<T>{(T *)s->V, s->ldv, (T *)s->w, (T *)s->z, (T *)s->x, (const T *)s->bown, (const T *)s->invd,
                    H, g, g + ld, g + 2 * ld, g + 3 * ld, s->n};
 }
+
+// Shared memory of the resident step's small arrays (before the slices).
+static size_t gm_res_small(const GmresState *s) { return sizeof(double) * 4 * (size_t)(s->m + 1); }
 
 // The Arnoldi kernel as a cooperative launch (all blocks resident, which its
 // grid barrier needs), captured into the graph like any kernel node.
@@ -622,9 +713,9 @@ static int gm_launch_arnoldi(GmresState *s, cudaStream_t st, cudaGraphConditiona
   if (s->grid_res > 0) {
     cfg.gridDim = dim3((unsigned)s->grid_res);
     cfg.blockDim = dim3(kResBlock);
-    cfg.dynamicSmemBytes = (size_t)s->res_slice * sizeof(T);
-    B_CUDA(cudaLaunchKernelEx(&cfg, gm_arnoldi_res_kernel<T, PRE, IN_GRAPH>, v, (const double *)s->part3,
-                              s->grid_spmv, s->part4, s->sc, s->res_slice, h));
+    cfg.dynamicSmemBytes = gm_res_small(s) + (size_t)s->res_slice * sizeof(T) * (s->res_two ? 2 : 1);
+    B_CUDA(cudaLaunchKernelEx(&cfg, gm_arnoldi_res_kernel<T, PRE, IN_GRAPH>, v, s->part4, s->G, s->sc, s->res_slice,
+                              s->res_two, h));
     return B200LA_OK;
   }
   cfg.gridDim = dim3((unsigned)s->grid_coop);
@@ -655,20 +746,24 @@ static int gm_size_resident(GmresState *s) {
   B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   const void *kern[2] = {(const void *)gm_arnoldi_res_kernel<T, PRE, true>,
                          (const void *)gm_arnoldi_res_kernel<T, PRE, false>};
-  const int64_t bytes = S * (int64_t)sizeof(T);
+  const int64_t bytes = S * (int64_t)sizeof(T), small = (int64_t)gm_res_small(s);
+  bool two = true;
   for (const void *k : kern) {
     cudaFuncAttributes fa;
     B_CUDA(cudaFuncGetAttributes(&fa, k));
-    if (bytes + (int64_t)fa.sharedSizeBytes > (int64_t)optin) return B200LA_OK;
+    if (small + bytes + (int64_t)fa.sharedSizeBytes > (int64_t)optin) return B200LA_OK;
+    two = two && small + 2 * bytes + (int64_t)fa.sharedSizeBytes <= (int64_t)optin;
   }
+  const int64_t dyn = small + (two ? 2 * bytes : bytes);
   for (const void *k : kern) {
-    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     int per_sm = 0;
-    B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kResBlock, (size_t)bytes));
+    B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kResBlock, (size_t)dyn));
     if (per_sm < 1) return B200LA_OK;
   }
   s->grid_res = grid;
   s->res_slice = S;
+  s->res_two = two;
   return B200LA_OK;
 }
 
@@ -860,7 +955,7 @@ void gmres_destroy(GmresState *s) {
   cudaStreamSynchronize(st);
   if (s->exec) cudaGraphExecDestroy(s->exec);
   if (s->graph) cudaGraphDestroy(s->graph);
-  void *bufs[] = {s->V, s->w, s->z, s->x, s->bown, s->invd, s->arrays, s->part, s->part3, s->part4, s->sc};
+  void *bufs[] = {s->V, s->w, s->z, s->x, s->bown, s->invd, s->arrays, s->part, s->part3, s->part4, s->G, s->sc};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, st);
   if (s->sc_host) cudaFreeHost(s->sc_host);
@@ -885,6 +980,9 @@ int gmres_create(b200la_mat A, const b200la_solver_params *prm, GmresState **out
   const size_t vb = es * (size_t)s->ldv;
   auto cleanup = [&](int code) { gmres_destroy(s); return code; };
   const int ld = s->m + 1;
+  // the resident step's partial sums: 2 (m + 1) columns and the norm's, a
+  // value per block of at most one a SM
+  const size_t part4_res = (size_t)(2 * ld + 1) * (size_t)c->num_sms;
   if (cudaMallocAsync(&s->V, vb * (size_t)(s->m + 1), st) != cudaSuccess)
     return cleanup(fail(B200LA_ERR_NOMEM, "solver_create: GMRES basis of %d x %zu bytes does not fit", s->m + 1, vb));
   if (cudaMallocAsync(&s->w, vb, st) != cudaSuccess || cudaMallocAsync(&s->z, vb, st) != cudaSuccess ||
@@ -892,7 +990,9 @@ int gmres_create(b200la_mat A, const b200la_solver_params *prm, GmresState **out
       cudaMallocAsync(&s->arrays, sizeof(double) * ((size_t)s->m * ld + 4 * (size_t)ld), st) != cudaSuccess ||
       cudaMallocAsync(&s->part, sizeof(double) * kMaxReduceBlocks, st) != cudaSuccess ||
       cudaMallocAsync(&s->part3, sizeof(double) * kMaxReduceBlocks, st) != cudaSuccess ||
-      cudaMallocAsync(&s->part4, sizeof(double) * 2 * kMaxReduceBlocks, st) != cudaSuccess ||
+      cudaMallocAsync(&s->part4, sizeof(double) * std::max<size_t>(2 * kMaxReduceBlocks, part4_res), st) !=
+          cudaSuccess ||
+      cudaMallocAsync(&s->G, sizeof(double) * (size_t)ld * ld, st) != cudaSuccess ||
       cudaMallocAsync(&s->sc, sizeof(GmScalars), st) != cudaSuccess ||
       cudaMallocHost(&s->sc_host, sizeof(GmScalars)) != cudaSuccess)
     return cleanup(fail(B200LA_ERR_NOMEM, "solver_create: GMRES work space allocation failed"));
