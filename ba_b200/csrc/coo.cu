@@ -386,7 +386,7 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
   m->max_row = hmax;
   const double avg = nrow ? (double)nnz / nrow : 0.0;
   m->format = B200LA_FMT_CSR;
-  m->param = avg <= 3 ? 2 : avg <= 6 ? 4 : avg <= 14 ? 8 : avg <= 40 ? 16 : 32;
+  m->param = csr_start_lanes(nrow, avg, hmax, c->num_sms);
   *out = m;
   return B200LA_OK;
 }

@@ -33,9 +33,11 @@ int fail(int code, const char *fmt, ...) {
 }
 
 int grid_for(b200la_ctx ctx, const void *kernel, int64_t work_items, int items_per_block, int *grid) {
-  int per_sm = 0;
-  B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0));
-  if (per_sm < 1) per_sm = 1;
+  int &per_sm = ctx->occupancy[kernel];
+  if (per_sm < 1) {
+    B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0));
+    if (per_sm < 1) per_sm = 1;
+  }
   int64_t need = (work_items + items_per_block - 1) / items_per_block;
   int64_t cap = (int64_t)ctx->num_sms * per_sm;
   if (cap > kMaxReduceBlocks) cap = kMaxReduceBlocks;
@@ -229,9 +231,10 @@ template <typename T>
 static int launch_dot(b200la_ctx c, int64_t n, const T *a, const T *b, double *out) {
   int grid;
   B_TRY(grid_for(c, (const void *)dot_kernel<T>, (n + Vec16<T>::n - 1) / Vec16<T>::n, kBlock, &grid));
-  dot_kernel<T><<<grid, kBlock, 0, c->stream>>>(n, a, b, c->scratch.part, c->scratch.ticket, c->scratch.result);
+  // the total goes straight to pinned host memory: a copy after the kernel
+  // would be one more operation for the stream to wait for
+  dot_kernel<T><<<grid, kBlock, 0, c->stream>>>(n, a, b, c->scratch.part, c->scratch.ticket, c->host_result);
   B_CUDA(cudaGetLastError());
-  B_CUDA(cudaMemcpyAsync(c->host_result, c->scratch.result, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   B_CUDA(cudaStreamSynchronize(c->stream));
   *out = c->host_result[0];
   return B200LA_OK;
@@ -294,7 +297,6 @@ int b200la_ctx_create(int device, b200la_ctx *out) {
   }
   B_CUDA(cudaMalloc(&c->scratch.part, sizeof(double) * 4 * kMaxReduceBlocks));
   B_CUDA(cudaMalloc(&c->scratch.ticket, sizeof(unsigned) * 16));
-  B_CUDA(cudaMalloc(&c->scratch.result, sizeof(double) * 8));
   B_CUDA(cudaMemset(c->scratch.ticket, 0, sizeof(unsigned) * 16));
   B_CUDA(cudaMallocHost(&c->host_result, sizeof(double) * 8));
   // Stream-ordered allocations (batch slots, tile lists, scratch) come from
@@ -320,7 +322,6 @@ int b200la_ctx_destroy(b200la_ctx c) {
   cudaStreamSynchronize(c->stream);
   cudaFree(c->scratch.part);
   cudaFree(c->scratch.ticket);
-  cudaFree(c->scratch.result);
   cudaFreeHost(c->host_result);
   cudaStreamDestroy(c->own_stream);
   delete c;
@@ -631,7 +632,7 @@ int b200la_csr_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, const int *
   }
   double avg = nrow ? (double)nnz / nrow : 0.0;
   m->format = B200LA_FMT_CSR;
-  m->param = avg <= 3 ? 2 : avg <= 6 ? 4 : avg <= 14 ? 8 : avg <= 40 ? 16 : 32;
+  m->param = csr_start_lanes(nrow, avg, max_row, c->num_sms);
   B_CUDA(cudaStreamSynchronize(s));
   *out = m;
   return B200LA_OK;

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <unordered_map>
 
 #include "b200la.h"
 
@@ -48,7 +49,6 @@ constexpr int kMaxReduceBlocks = 4096;
 struct ReduceScratch {
   double *part;       // [4][kMaxReduceBlocks]
   unsigned *ticket;   // [16]
-  double *result;     // [8]
 };
 
 }  // namespace b200la
@@ -65,6 +65,9 @@ struct b200la_ctx_s {
   // a profiler can see each launch (ncu does not profile kernels inside
   // graphs with conditional nodes).
   bool use_graphs;
+  // resident blocks per SM of each kernel launched so far (grid_for), so a
+  // call does not ask the driver again
+  std::unordered_map<const void *, int> occupancy;
 };
 
 struct b200la_vec_s {
@@ -130,6 +133,22 @@ namespace b200la {
 
 // Host validation of a CSR structure: rowptr[0] == 0, non-decreasing,
 // rowptr[nrow] == nnz, 0 <= col < ncol.  Writes the longest row length.
+// Threads per row of the CSR schedule a matrix starts with: enough for the
+// rows' length, but on rows of nearly equal length that fill the GPU more
+// than about twice (2,048 threads a SM) only 2 (up to 14 entries) or 4 (up to
+// 40), since a lane's loads are then several consecutive entries and no lane
+// idles.  Measured, us a product on 2 / 4 / 8 / 16 threads: 9 entries a row 2D
+// 1024^2 24 / 29 / 41 / 62, 512^2 8.3 / 9.3 / 12.4 / 16.5, 256^2 6.1 / 5.4 /
+// 5.4 / 6.7; 27 entries 3D 96^3 72 / 58 / 68 / 84, 64^3 24 / 18.5 / 23 / 28,
+// 48^3 11.4 / 10.3 / 11.4 / 14.4, 32^3 6.2 on all.  Where some rows are much
+// longer, a thread that walks one holds its warp up (power-law rows of 1..200,
+// mean 5.8: 8 threads were the best).
+inline int csr_start_lanes(int64_t nrow, double avg, int max_row, int sms) {
+  const int lanes = avg <= 3 ? 2 : avg <= 6 ? 4 : avg <= 14 ? 8 : avg <= 40 ? 16 : 32;
+  if (max_row > 2.0 * avg || avg > 40 || nrow * lanes <= (int64_t)sms * 4096) return lanes;
+  return avg <= 14 ? 2 : 4;
+}
+
 int validate_csr(int nrow, int ncol, int64_t nnz, const int *rowptr, const int *col, int *max_row);
 
 // Q1 system assembly on the device (assemble.cu).
