@@ -6,22 +6,24 @@
 // and then sorts every row by column with a selection sort that keeps
 // duplicates (and, being a selection sort with swaps, does not keep them in
 // input order).  Here the same result comes from:
-//   1. a device check of every index (a bad triplet fails the upload),
-//   2. a stable radix sort of the triplets by row carrying (column, input
-//      position) pairs (input order kept within a row, as the reference's
-//      scatter keeps it),
-//   3. row offsets from the sorted rows (each row boundary writes its range),
-//   4. a gather of the values from their input positions (cast to the
-//      storage type), the columns coming with the sorted pairs,
-//   5. the row sort, one warp per row: ranks by shuffles when the row's
-//      columns are distinct (the sorted row is then unique), the
-//      reference's selection sort itself when a column repeats or the row
-//      is longer than 256 entries (rows above 32 entries go through a
-//      worklist to a second kernel),
-//   6. the diagonal positions and the longest row, as b200la_csr_upload does.
+//   1. one pass over the triplets that checks every index (a bad triplet
+//      fails the upload) and counts the rows with atomics, each entry keeping
+//      the count it met as its place in the row,
+//   2. the row pointer as the counts' prefix sum,
+//   3. a scatter of (column, input position) pairs to their places; within a
+//      row these come in the order the atomics ran in, which is never used:
+//   4. the row sort, one warp per row: when the row's columns are distinct
+//      the sorted row is unique, ranks come from shuffles and each value from
+//      its input position; when a column repeats, the entries are first put
+//      in input order (by the positions, which are distinct) and then sorted
+//      by the reference's selection sort itself; rows above 32 entries go
+//      through a worklist to a second kernel,
+//   5. the diagonal positions and the longest row, as b200la_csr_upload does.
+// What bounds it: random 32-byte sectors, one written (3) and one read (4)
+// per entry, and the atomics.  A stable radix sort by row (four passes over
+// 12-byte records) and a separate gather took 1.4 + 1.2 of 3.8 ms on 57 M
+// triplets.
 // The result is the reference's CSR bit for bit, duplicates included.
-#include <cub/device/device_radix_sort.cuh>
-
 #include <climits>
 #include <cstring>
 
@@ -29,29 +31,139 @@
 
 namespace b200la {
 
-// First bad triplet (smallest index), or all ones when every index is in range.
-__global__ void coo_check_kernel(int64_t nnz, int nrow, int ncol, const int *__restrict__ rows,
-                                 const int *__restrict__ cols, unsigned long long *bad) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-    const int r = rows[i], c = cols[i];
-    if (r < 0 || r >= nrow || c < 0 || c >= ncol) atomicMin(bad, (unsigned long long)i);
+// First bad triplet (smallest index), or all ones when every index is in
+// range; place[i] = how many entries of its row were counted before entry i.
+// Two entries in flight per thread.
+__global__ void __launch_bounds__(kBlock) coo_count_kernel(int64_t nnz, int nrow, int ncol,
+                                                           const int *__restrict__ rows,
+                                                           const int *__restrict__ cols, int *__restrict__ count,
+                                                           int *__restrict__ place, unsigned long long *bad) {
+  constexpr int U = 4;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nnz; i0 += U * stride) {
+    int r[U], c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = i0 + u * stride < nnz;
+      r[u] = in ? rows[i0 + u * stride] : 0;
+      c[u] = in ? cols[i0 + u * stride] : 0;
+    }
+    int p[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * stride;
+      if (i >= nnz) continue;
+      if (r[u] < 0 || r[u] >= nrow || c[u] < 0 || c[u] >= ncol) {
+        atomicMin(bad, (unsigned long long)i);
+        p[u] = 0;
+      } else {
+        p[u] = atomicAdd(count + r[u], 1);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * stride < nnz) place[i0 + u * stride] = p[u];
   }
 }
 
-// Sort payload of each triplet: its column in the high word and its input
-// position in the low word, so that the sort carries the column along and
-// the gather reads only the value from a random position.
-__global__ void coo_pack_kernel(int64_t n, const int *__restrict__ cols, unsigned long long *out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = ((unsigned long long)(unsigned)cols[i] << 32) | (unsigned long long)(unsigned)i;
+// ---- prefix sum of the row counts: a block's sum, the blocks' offsets, the
+// row pointer (kScanRows rows a block, kScanEach a thread)
+constexpr int kScanEach = 8;
+constexpr int kScanRows = kBlock * kScanEach;
+
+__device__ __forceinline__ int warp_scan(int v) {  // inclusive
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
 }
 
-// rowptr from the rows sorted ascending: entry i starts rows prev+1 .. r.
-__global__ void coo_rowptr_kernel(int64_t nnz, int nrow, const int *__restrict__ srow, int *rowptr) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= nnz; i += (int64_t)gridDim.x * blockDim.x) {
-    const int prev = i == 0 ? -1 : srow[i - 1];
-    const int r = i == nnz ? nrow : srow[i];
-    for (int rr = prev + 1; rr <= r; ++rr) rowptr[rr] = (int)i;
+// Exclusive prefix of v over the block's threads; *total = the block's sum.
+__device__ __forceinline__ int block_scan(int v, int *total) {
+  __shared__ int part[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+  const int inc = warp_scan(v);
+  if (lane == 31) part[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    const int s = warp_scan(lane < nw ? part[lane] : 0);
+    part[lane] = s;
+  }
+  __syncthreads();
+  const int before = warp > 0 ? part[warp - 1] : 0;
+  *total = part[nw - 1];
+  __syncthreads();
+  return before + inc - v;
+}
+
+__global__ void __launch_bounds__(kBlock) coo_block_sum_kernel(int nrow, const int *__restrict__ count,
+                                                               int *__restrict__ sums) {
+  const int64_t first = (int64_t)blockIdx.x * kScanRows + (int64_t)threadIdx.x * kScanEach;
+  int s = 0;
+#pragma unroll
+  for (int k = 0; k < kScanEach; ++k)
+    if (first + k < nrow) s += count[first + k];
+  int total;
+  block_scan(s, &total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// sums -> their exclusive prefix, one block
+__global__ void __launch_bounds__(1024) coo_scan_sums_kernel(int blocks, int *sums) {
+  int carry = 0;
+  for (int b0 = 0; b0 < blocks; b0 += (int)blockDim.x) {
+    const int i = b0 + (int)threadIdx.x;
+    const int v = i < blocks ? sums[i] : 0;
+    int total;
+    const int ex = block_scan(v, &total);
+    if (i < blocks) sums[i] = carry + ex;
+    carry += total;
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) coo_rowptr_kernel(int nrow, int nnz, const int *__restrict__ count,
+                                                            const int *__restrict__ sums, int *__restrict__ rowptr) {
+  const int64_t first = (int64_t)blockIdx.x * kScanRows + (int64_t)threadIdx.x * kScanEach;
+  int c[kScanEach], s = 0;
+#pragma unroll
+  for (int k = 0; k < kScanEach; ++k) {
+    c[k] = first + k < nrow ? count[first + k] : 0;
+    s += c[k];
+  }
+  int total;
+  int at = sums[blockIdx.x] + block_scan(s, &total);
+#pragma unroll
+  for (int k = 0; k < kScanEach; ++k) {
+    if (first + k < nrow) rowptr[first + k] = at;
+    at += c[k];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) rowptr[nrow] = nnz;
+}
+
+// Each triplet's column (high word) and input position (low word) to its
+// place in its row.
+__global__ void __launch_bounds__(kBlock) coo_scatter_kernel(int64_t nnz, const int *__restrict__ rows,
+                                                             const int *__restrict__ cols,
+                                                             const int *__restrict__ place,
+                                                             const int *__restrict__ rowptr,
+                                                             unsigned long long *__restrict__ out) {
+  constexpr int U = 4;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nnz; i0 += U * stride) {
+    int at[U], c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * stride < nnz) {
+        at[u] = __ldg(rowptr + rows[i0 + u * stride]) + place[i0 + u * stride];
+        c[u] = cols[i0 + u * stride];
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * stride < nnz)
+        out[at[u]] = ((unsigned long long)(unsigned)c[u] << 32) | (unsigned long long)(unsigned)(i0 + u * stride);
   }
 }
 
@@ -82,45 +194,19 @@ __device__ void row_selection_sort(int k, int b, int e, int *col, T *val, int *d
   diag[k] = d;
 }
 
-// Columns and values into the row-sorted order: the column comes with the
-// sorted payload, the value (cast to the storage type) from its input
-// position, a random read; each thread keeps kGatherUnroll of those in flight.
-constexpr int kGatherUnroll = 4;
-
-template <typename T, typename S>
-__global__ void __launch_bounds__(kBlock) coo_gather_kernel(int64_t nnz, const unsigned long long *__restrict__ packed,
-                                                            const S *__restrict__ vals, int *col, T *val) {
-  constexpr int U = kGatherUnroll;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t k0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k0 < nnz; k0 += U * stride) {
-    unsigned long long q[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) q[u] = k0 + u * stride < nnz ? packed[k0 + u * stride] : 0ull;
-    S vv[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (k0 + u * stride < nnz) vv[u] = vals[(unsigned)q[u]];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (k0 + u * stride < nnz) {
-        col[k0 + u * stride] = (int)(q[u] >> 32);
-        val[k0 + u * stride] = (T)vv[u];
-      }
-  }
-}
-
-// Row sort, one warp per row of up to 32 entries (lane l holds entry l, in
-// input order as gathered).  When the row's columns are distinct the sorted
-// row is unique, so each entry goes straight to b + (number of smaller
-// columns), ranks taken with shuffles; that equals the reference's selection
-// sort.  A row with a repeated column (found by __match_any_sync) is sorted
-// by the selection sort itself (lane 0), because there the order of equal
-// columns depends on its swaps.  Longer rows are appended to a worklist for
+// Row sort, one warp per row of up to 32 entries (lane l holds one of them).
+// When the row's columns are distinct the sorted row is unique, so each entry
+// goes straight to b + (number of smaller columns), ranks taken with shuffles;
+// that equals the reference's selection sort.  A row with a repeated column
+// (found by __match_any_sync) is first put in input order, then sorted by the
+// selection sort itself (lane 0), because there the order of equal columns
+// depends on its swaps.  Longer rows are appended to a worklist for
 // coo_long_rows_kernel.  Also the diagonal positions and the longest row.
-template <typename T>
-__global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int *__restrict__ rowptr, int *col,
-                                                             T *val, int *diag, int *max_row, int *long_rows,
-                                                             int *n_long) {
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int *__restrict__ rowptr,
+                                                             const unsigned long long *__restrict__ packed,
+                                                             const S *__restrict__ vals, int *col, T *val, int *diag,
+                                                             int *max_row, int *long_rows, int *n_long) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -134,11 +220,20 @@ __global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int
       continue;
     }
     const bool valid = lane < L;
-    const int c = valid ? col[b + lane] : INT_MAX;  // columns are < ncol <= INT_MAX
+    const unsigned long long q = valid ? packed[b + lane] : 0ull;
+    const int c = valid ? (int)(q >> 32) : INT_MAX;  // columns are < ncol <= INT_MAX
+    const unsigned pos = (unsigned)q;
     T v = T(0);
-    if (valid) v = val[b + lane];
+    if (valid) v = (T)vals[pos];
     const unsigned same = __match_any_sync(0xffffffffu, c);
     if (__any_sync(0xffffffffu, valid && __popc(same) > 1)) {
+      int r = 0;
+      for (int j = 0; j < L; ++j) r += __shfl_sync(0xffffffffu, pos, j) < pos ? 1 : 0;
+      if (valid) {
+        col[b + r] = c;
+        val[b + r] = v;
+      }
+      __syncwarp();
       if (lane == 0) row_selection_sort(k, b, e, col, val, diag);
       __syncwarp();
       continue;
@@ -161,13 +256,16 @@ __global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int
 }
 
 // Rows longer than 32 entries (from coo_rowsort_kernel's worklist), one warp
-// per row: lane l holds entries l, l + 32, ... (up to kMaxQ * 32 = 256) and
-// the ranks come from shuffles as above; a repeated column or a longer row
-// takes the selection sort (lane 0).
+// per row: the entries go to col / val in input order first (each lane counts
+// the smaller positions of its entries); then lane l holds entries l, l + 32,
+// ... (up to kMaxQ * 32 = 256) and the ranks come from shuffles as above; a
+// repeated column or a longer row takes the selection sort (lane 0).
 constexpr int kMaxQ = 8;
 
-template <typename T>
-__global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__restrict__ rowptr, int *col, T *val,
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__restrict__ rowptr,
+                                                               const unsigned long long *__restrict__ packed,
+                                                               const S *__restrict__ vals, int *col, T *val,
                                                                int *diag, const int *__restrict__ long_rows,
                                                                const int *__restrict__ n_long) {
   const int lane = threadIdx.x & 31;
@@ -177,6 +275,15 @@ __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__rest
   for (int64_t w = warp; w < count; w += nwarps) {
     const int k = long_rows[w];
     const int b = rowptr[k], e = rowptr[k + 1], L = e - b;
+    for (int i = lane; i < L; i += 32) {
+      const unsigned long long q = packed[b + i];
+      const unsigned pos = (unsigned)q;
+      int r = 0;
+      for (int t = 0; t < L; ++t) r += (unsigned)packed[b + t] < pos ? 1 : 0;
+      col[b + r] = (int)(q >> 32);
+      val[b + r] = (T)vals[pos];
+    }
+    __syncwarp();
     if (L > kMaxQ * 32) {
       if (lane == 0) row_selection_sort(k, b, e, col, val, diag);
       __syncwarp();
@@ -238,13 +345,6 @@ static int grid_1d(b200la_ctx c, int64_t work) {
   return (int)(g < 1 ? 1 : g);
 }
 
-// Number of bits that hold values 0 .. n-1.
-static int bits_for(int n) {
-  int b = 1;
-  while (b < 31 && (1LL << b) < (long long)n) ++b;
-  return b;
-}
-
 }  // namespace b200la
 
 using namespace b200la;
@@ -261,10 +361,10 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
   cudaStream_t s = c->stream;
   const size_t nz = (size_t)(nnz > 0 ? nnz : 1);
   const size_t vsz = dtype_size(val_dtype);
-  // scratch: device triplets (when given host arrays), sorted rows, permutation
-  int *d_rows = nullptr, *d_cols = nullptr, *srow = nullptr;
-  unsigned long long *idx = nullptr, *perm = nullptr;  // sort payload in and out
-  void *d_vals = nullptr, *cub_tmp = nullptr;
+  // scratch: device triplets (when given host arrays), pairs by row, block sums
+  int *d_rows = nullptr, *d_cols = nullptr, *sums = nullptr;
+  unsigned long long *packed = nullptr;
+  void *d_vals = nullptr;
   unsigned long long *bad = nullptr;
   int *max_row_d = nullptr, *n_long_d = nullptr, *long_rows = nullptr;
   b200la_mat m = new b200la_mat_s();
@@ -312,8 +412,12 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
       c_in = d_cols;
       v_in = d_vals;
     }
-    const int g = grid_1d(c, nnz);
-    coo_check_kernel<<<g, kBlock, 0, s>>>(nnz, nrow, ncol, r_in, c_in, bad);
+    // the diagonal positions' buffer holds the row counts and the columns'
+    // the entries' places until the row sort writes them
+    int *count = m->diag, *place = m->col;
+    const int g = grid_1d(c, (nnz + 3) / 4);
+    if (nrow > 0 && !cu(cudaMemsetAsync(count, 0, sizeof(int) * (size_t)nrow, s), "memset")) break;
+    coo_count_kernel<<<g, kBlock, 0, s>>>(nnz, nrow, ncol, r_in, c_in, count, place, bad);
     unsigned long long hbad = 0;
     if (!cu(cudaGetLastError(), "check") ||
         !cu(cudaMemcpyAsync(&hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, s), "copy") ||
@@ -323,50 +427,30 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
       rc = fail(B200LA_ERR_MATRIX, "coo_upload: triplet %llu has an index out of range", hbad);
       break;
     }
-    // stable sort by row: keys rows, values input positions
-    if (!cu(cudaMallocAsync(&srow, sizeof(int) * nz, s), "allocation") ||
-        !cu(cudaMallocAsync(&idx, sizeof(unsigned long long) * nz, s), "allocation") ||
-        !cu(cudaMallocAsync(&perm, sizeof(unsigned long long) * nz, s), "allocation"))
+    const int blocks = (int)(((int64_t)nrow + kScanRows - 1) / kScanRows);  // nrow > 0: every index is in range
+    if (!cu(cudaMallocAsync(&sums, sizeof(int) * (size_t)blocks, s), "allocation") ||
+        !cu(cudaMallocAsync(&packed, sizeof(unsigned long long) * nz, s), "allocation") ||
+        !cu(cudaMallocAsync(&long_rows, sizeof(int) * (size_t)nrow, s), "allocation"))
       break;
-    coo_pack_kernel<<<g, kBlock, 0, s>>>(nnz, c_in, idx);
-    size_t tmp_bytes = 0;
-    const int end_bit = bits_for(nrow);
-    if (!cu(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, r_in, srow, idx, perm, (int)nnz, 0, end_bit, s),
-            "sort size") ||
-        !cu(cudaMallocAsync(&cub_tmp, tmp_bytes > 0 ? tmp_bytes : 1, s), "allocation") ||
-        !cu(cub::DeviceRadixSort::SortPairs(cub_tmp, tmp_bytes, r_in, srow, idx, perm, (int)nnz, 0, end_bit, s),
-            "sort"))
-      break;
-    coo_rowptr_kernel<<<grid_1d(c, nnz + 1), kBlock, 0, s>>>(nnz, nrow, srow, m->rowptr);
+    coo_block_sum_kernel<<<blocks, kBlock, 0, s>>>(nrow, count, sums);
+    coo_scan_sums_kernel<<<1, 1024, 0, s>>>(blocks, sums);
+    coo_rowptr_kernel<<<blocks, kBlock, 0, s>>>(nrow, (int)nnz, count, sums, m->rowptr);
+    coo_scatter_kernel<<<g, kBlock, 0, s>>>(nnz, r_in, c_in, place, m->rowptr, packed);
+    const int gr = grid_1d(c, (int64_t)nrow * 32);
+    auto sort_rows = [&](auto t, auto u) {
+      using T = decltype(t);
+      using S = decltype(u);
+      coo_rowsort_kernel<T, S><<<gr, kBlock, 0, s>>>(nrow, m->rowptr, packed, (const S *)v_in, m->col, (T *)m->val,
+                                                     m->diag, max_row_d, long_rows, n_long_d);
+      coo_long_rows_kernel<T, S><<<c->num_sms * 8, kBlock, 0, s>>>(m->rowptr, packed, (const S *)v_in, m->col,
+                                                                   (T *)m->val, m->diag, long_rows, n_long_d);
+    };
     if (dtype == B200LA_F64) {
-      if (val_dtype == B200LA_F64)
-        coo_gather_kernel<double, double><<<g, kBlock, 0, s>>>(nnz, perm, (const double *)v_in, m->col,
-                                                               (double *)m->val);
-      else
-        coo_gather_kernel<double, float><<<g, kBlock, 0, s>>>(nnz, perm, (const float *)v_in, m->col,
-                                                              (double *)m->val);
+      if (val_dtype == B200LA_F64) sort_rows(double(), double());
+      else sort_rows(double(), float());
     } else {
-      if (val_dtype == B200LA_F64)
-        coo_gather_kernel<float, double><<<g, kBlock, 0, s>>>(nnz, perm, (const double *)v_in, m->col,
-                                                              (float *)m->val);
-      else
-        coo_gather_kernel<float, float><<<g, kBlock, 0, s>>>(nnz, perm, (const float *)v_in, m->col,
-                                                             (float *)m->val);
-    }
-    if (nrow > 0) {
-      if (!cu(cudaMallocAsync(&long_rows, sizeof(int) * (size_t)nrow, s), "allocation")) break;
-      const int gr = grid_1d(c, (int64_t)nrow * 32);
-      if (dtype == B200LA_F64) {
-        coo_rowsort_kernel<double><<<gr, kBlock, 0, s>>>(nrow, m->rowptr, m->col, (double *)m->val, m->diag,
-                                                         max_row_d, long_rows, n_long_d);
-        coo_long_rows_kernel<double><<<c->num_sms * 8, kBlock, 0, s>>>(m->rowptr, m->col, (double *)m->val,
-                                                                       m->diag, long_rows, n_long_d);
-      } else {
-        coo_rowsort_kernel<float><<<gr, kBlock, 0, s>>>(nrow, m->rowptr, m->col, (float *)m->val, m->diag,
-                                                        max_row_d, long_rows, n_long_d);
-        coo_long_rows_kernel<float><<<c->num_sms * 8, kBlock, 0, s>>>(m->rowptr, m->col, (float *)m->val, m->diag,
-                                                                      long_rows, n_long_d);
-      }
+      if (val_dtype == B200LA_F64) sort_rows(float(), double());
+      else sort_rows(float(), float());
     }
     cu(cudaGetLastError(), "kernels");
   } while (false);
@@ -375,7 +459,7 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
     cu(cudaMemcpyAsync(&hmax, max_row_d, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
     cu(cudaStreamSynchronize(s), "sync");
   }
-  void *scratch[] = {d_rows, d_cols, d_vals, srow, idx, perm, cub_tmp, bad, long_rows};
+  void *scratch[] = {d_rows, d_cols, d_vals, sums, packed, bad, long_rows};
   for (void *p : scratch)
     if (p) cudaFreeAsync(p, s);
   if (rc != B200LA_OK) {

@@ -159,3 +159,29 @@ def test_bad_triplets_are_refused(plat):
     # the context stays usable
     A = lmp.B200_CSR_lMatrix.TransformFromCOO(*LMP_TEST_COO, 3, 3, platform=plat)
     assert A.get_nnz() == 7
+
+
+# Row counts at the prefix sum's block edges (2,048 rows a block) and rows at
+# the row sort's limits (32 a warp, 256 in registers), each with distinct
+# columns, with a repeated one and with many, the triplets shuffled.
+@pytest.mark.parametrize("nrow", [1, 31, 2047, 2048, 2049, 6149])
+@pytest.mark.parametrize("dup", [0, 1, 7])
+def test_row_and_block_edges_match_oracle(plat, nrow, dup):
+    rng = np.random.default_rng(nrow + dup)
+    lengths = [0, 1, 2, 31, 32, 33, 255, 256, 257, 300]
+    rows, cols = [], []
+    for i in range(min(nrow, 40)):
+        r = (i * 997) % nrow
+        L = lengths[i % len(lengths)]
+        c = rng.permutation(400)[:L]
+        if L > dup:
+            c[:dup] = c[dup]
+        rows += [r] * L
+        cols += list(c)
+    order = rng.permutation(len(rows))
+    rows, cols = np.asarray(rows, np.int32)[order], np.asarray(cols, np.int32)[order]
+    vals = rng.standard_normal(len(rows))
+    ref = oracle.coo_to_csr(nrow, 400, rows, cols, vals)
+    A = lmp.B200_CSR_lMatrix.TransformFromCOO(rows, cols, vals, nrow, 400, platform=plat)
+    for got, want in zip(A.csr(), ref):
+        np.testing.assert_array_equal(got, want)
