@@ -195,7 +195,8 @@ int b200la_mat_inv_diag(b200la_mat m, b200la_vec out);
  * of it (checked on the device), and it must have 9 or 27 entries, else
  * B200LA_ERR_UNSUPPORTED.  Each row stores one value per offset (0 where it
  * has no entry; the list is padded with offset 0 to a multiple of `param`),
- * so the copy holds values only; a row's products are added in ascending
+ * so the copy holds values only (only the upper half of them where the values
+ * are symmetric up to rows that hold only their diagonal); a row's products are added in ascending
  * column order, its stored order, so the results are SELL's bits (the
  * absent entries add 0 * x at a column the row does not read: a non-finite
  * x there makes the row's sum NaN where CSR would not). */
@@ -255,15 +256,19 @@ typedef struct {
 } b200la_cg_result;
 
 /* SetupOperator + (optional) SetupPreconditioner: builds the solver's
- * resident work vectors, the Jacobi inverse diagonal, and the CUDA graph that
- * runs the whole iteration on the device (no host round trip per step). */
+ * resident work vectors, the Jacobi inverse diagonal, and the form in which
+ * the whole iteration runs on the device (no host round trip per step): a
+ * CUDA graph of three kernels, or, for systems that fit, one kernel that keeps
+ * matrix and vectors on the SMs of one cluster, or the vectors on resident
+ * blocks.  A resident block's wait that runs out ends the solve with
+ * B200LA_ERR_TIMEOUT. */
 int b200la_cg_create(b200la_mat A, const b200la_cg_params *params, b200la_cg *out);
 int b200la_cg_destroy(b200la_cg s);
 /* Solve(b, &x): x holds the start value on entry and the solution on exit. */
 int b200la_cg_solve(b200la_cg s, b200la_vec b, b200la_vec x, b200la_cg_result *result);
 /* Instrumentation: from the start value x, runs `iters` iterations as
- * separate launches with CUDA events between the kernels (same kernels as the
- * graph) and writes the mean milliseconds per launch of
+ * separate launches with CUDA events between the kernels (the graph's three
+ * kernels, whatever form the solves take) and writes the mean milliseconds per launch of
  * ms[0] = SpMV + p.Ap, ms[1] = update + r.r/r.z, ms[2] = direction.
  * x is not modified. */
 int b200la_cg_profile(b200la_cg s, b200la_vec b, b200la_vec x, int iters, double *ms);
@@ -295,7 +300,8 @@ int b200la_pcg_solve(b200la_mat A, b200la_vec b, b200la_vec x, const b200la_cg_p
  * GMRES<LAD, PreLAD> (linear_solver/gmres.h:143-746), restarted after
  * size_basis steps, modified Gram-Schmidt, no or right (Jacobi)
  * preconditioning: per step one SpMV (fused with w.V_0) and one cooperative
- * kernel that runs the whole Gram-Schmidt sweep with grid barriers (every
+ * kernel that runs the whole Gram-Schmidt sweep, its dots in one pass over the
+ * basis, with grid barriers (every
  * wait bounded: a wait that runs out ends the solve with B200LA_ERR_TIMEOUT),
  * normalises the new basis vector and applies the Givens rotations and the
  * test; at a cycle end one pass applies x += P V y.  The basis takes
@@ -420,7 +426,11 @@ int b200la_mp_solve(b200la_mp s, b200la_vec b, b200la_vec x, b200la_mp_result *r
  * Each system follows the Jacobi-PCG recurrence of CG<LAD>
  * (linear_solver/cg.h:165-246), either in FP64 (mixed = 0) or as FP32 inner
  * solves inside FP64 refinement (mixed = 1, MPIR structure, mpir.cc:52-230).
- * Systems can be added and removed between runs (continuous batching). */
+ * Systems can be added and removed between runs (continuous batching).
+ * Systems with a symmetric, structured matrix that fits on the SMs of one
+ * thread-block cluster (up to ~70,000 rows of nine entries in mixed mode) are
+ * iterated there, one cluster a system, instead of by the swept kernels; a run
+ * takes them the same number of passes. */
 typedef struct {
   int capacity;       /* system slots */
   int mixed;          /* 1: FP32 inner PCG + FP64 refinement; 0: FP64 PCG */
