@@ -501,8 +501,8 @@ def run_batch(args, rank, local_rank, world, torch, dist, barrier):
                 "precision": f"FP32 Jacobi-PCG inner solves (FP32 matrix values and vectors, compensated FP32 "
                              f"dots) inside FP64 refinement: the FP64 residual replaces the inner one every "
                              f"{inner_rtol:g}x reduction, the search direction is kept",
-                "spmv_schedule": ("sliced ELL, 32 rows per slice, one row per lane; values only (columns = row + the "
-                                  "system's 9 stencil offsets), p window staged in shared memory"),
+                "spmv_schedule": ("one thread-block cluster a system, symmetric half of the values and the p window in "
+                                  "shared memory; the profiled pass kernels: sliced ELL, values only"),
                 "p50_latency_ms": float(np.percentile(lat, 50)), "p99_latency_ms": float(np.percentile(lat, 99)),
                 "latency": "per-system device time from its first residual to its finish inside the step",
                 "converged": f"{ok}/{len(systems)}", "worst_true_rel_residual_sampled": worst,
@@ -519,7 +519,9 @@ def run_batch(args, rank, local_rank, world, torch, dist, barrier):
                                     "speedup_of_mixed_pcg": value / world / pcg_value}},
             "clocks": clk,
             "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-            "gpu_launches": args.steps + 3 * passes_tot + (passes_tot + CHUNK - 1) // CHUNK,
+            # a restart and at least one launch of clusters a step (one per group of equal cluster
+            # size); the pass kernels launch only for systems that no cluster holds
+            "gpu_launches": 2 * args.steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": profile_traffic("batch1024/f32/spmv"), "peak_source": peak_kind,
                          "kernel": "batch_spmv_kernel<float> (K1: sliced-ELL SpMV + p.Ap) over an inner pass of "
@@ -1626,13 +1628,13 @@ def run_coo(args, rank, local_rank, world, torch, dist, barrier):
             "config": {"workload": f"TransformFromCOO of the 3d q1 poisson {args.cells}^3 matrix, triplets shuffled",
                        "n": s.n, "nnz": s.nnz, "matches_generator_csr": ok, "parallelism": f"replicas x{world}",
                        "l2": "inputs larger than L2 (913 MB of triplets)",
-                       "launches": "6 of ours per conversion (check, iota, row offsets, gather, row sort, long "
-                                   "rows) and 5 of the CUB radix sort",
+                       "launches": "7 of ours per conversion (check and count, three of the prefix sum, scatter, "
+                                   "row sort, long rows)",
                        "e2e_host_buffers": "pinned"},
             "clocks": clk,
             "e2e": {"value": e2e_value, "unit": "conversions/s", "h2d_bytes_per_step": s.nnz * 16,
                     "d2h_bytes_per_step": s.nnz * 12 + (s.n + 1) * 4},
-            "gpu_launches": args.steps * 6,
+            "gpu_launches": args.steps * 7,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": peak_kind,
                          "kernel": "whole conversion (check, radix sort by row, row offsets, gather, row sort)",
