@@ -109,7 +109,7 @@ struct SysState {
   double rz, pAp, alpha, beta;
   double res_in, res_in0;      // inner recurrence residual and its start value
   double res, res0;            // FP64 true residual and the initial one
-  unsigned long long t_begin;  // %globaltimer at the system's first residual
+  unsigned long long t_begin;  // %globaltimer at the system's first residual (on a cluster: at its run's start)
   unsigned long long t_done;   // %globaltimer when the system finished
   int state;                   // B200LA_* iterate state at the end
   unsigned bad_row;            // first row without a usable diagonal (Jacobi), else ~0u
@@ -1024,7 +1024,7 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
   double rz = S.rzb[0], rz_keep = S.rz_keep, res = S.res, res0 = S.res0, res_in = S.res_in, res_in0 = S.res_in0;
   int it = S.itb[0], tot = S.totb[0], outer = S.outer, keep_p = S.keep_p, state = S.state;
   const bool diag_ok = !prm.precond || S.bad_row == 0xffffffffu;
-  unsigned long long t_begin = S.t_begin, t_done = S.t_done;
+  unsigned long long t_done = S.t_done;
   int set = 0, passes = 0;
   // START left open by a run of the pass kernels: the direction, then INNER
   auto start = [&]() {
@@ -1061,10 +1061,7 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
       g.template sum<3>(v, set);
       set ^= 1;
       res = sqrt(v[0]);
-      if (outer == 0) {
-        res0 = res;
-        t_begin = globaltimer();
-      }
+      if (outer == 0) res0 = res;
       int s = outer_check(res, res0, prm);
       if (s == B200LA_ITERATE && outer >= prm.max_outer) s = B200LA_FAIL_MAXITS;
       if (outer > 0 && sqrt(v[1]) > 2.0 * res_in) keep_p = 0;
@@ -1160,9 +1157,19 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
     S.res_in0 = res_in0;
     S.res = res;
     S.res0 = res0;
-    S.t_begin = t_begin;
     S.t_done = t_done;
     S.cl_passes = passes;
+  }
+}
+
+// The start of the listed systems that have not run yet, as the first pass of
+// the pass kernels records it: a system that waits for the SMs of others has
+// begun.
+__global__ void cluster_begin_kernel(const int *__restrict__ list, int count, SysState *st) {
+  const unsigned long long now = globaltimer();
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+    SysState &S = st[list[k]];
+    if (S.phase == PH_RESID && S.outer == 0) S.t_begin = now;
   }
 }
 
@@ -1914,6 +1921,8 @@ template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget)
   });
   B_CUDA(cudaMemcpyAsync(B->cl_list, sl.data(), sizeof(int) * sl.size(), cudaMemcpyHostToDevice, st));
   B_CUDA(cudaStreamSynchronize(st));  // the list is rebuilt on the host for the next launch
+  cluster_begin_kernel<<<((int)sl.size() + kBlock - 1) / kBlock, kBlock, 0, st>>>(B->cl_list, (int)sl.size(), B->st);
+  B_CUDA(cudaGetLastError());
   B_CUDA(cudaEventRecord(B->cl_event[4], st));
   int used = 0, turn = 0;
   for (size_t a = 0; a < sl.size();) {

@@ -526,3 +526,17 @@ def test_cluster_form_refuses_unsymmetric_values(plat):
     assert outs[0].solver_state == 0 and np.array_equal(outs[0].x, outs[1].x)
     ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=10000, atol=0.0, rtol=1e-13)
     assert np.linalg.norm(outs[0].x - ref.x) <= 1e-8 * np.linalg.norm(ref.x)
+
+
+def test_latency_counts_the_wait_for_sms(plat):
+    """device_us runs from the start of the solve: of many equal systems more
+    than fit on the GPU at once, the last to be placed has waited for the
+    others.  400 clusters of at least one SM each on at most 148 SMs take three
+    waves or more, so the longest time is at least twice the shortest."""
+    s = P.q1_system(2, 60, 11, 1.0, "queue")
+    B = Batch(400, mixed=True, precond=True, rtol=1e-8, platform=plat)
+    slots = B.add_many([(s.rowptr, s.col, s.val, s.b)] * 400)
+    B.solve()
+    us = [r.device_us for r in B.results(slots, with_x=False)]
+    B.close()
+    assert max(us) >= 2.0 * min(us), (min(us), max(us))
