@@ -2601,6 +2601,7 @@ int run_passes(b200la_batch B, int max_passes, int cluster_passes, int *active_o
   BatchGlobals &g = *B->glob_host;
   if (active == 0 && B->cl_slots.empty()) {
     g.passes = 0;
+    B->list_passes = 0;
     if (active_out) *active_out = 0;
     return B200LA_OK;
   }

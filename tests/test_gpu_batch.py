@@ -540,3 +540,18 @@ def test_latency_counts_the_wait_for_sms(plat):
     us = [r.device_us for r in B.results(slots, with_x=False)]
     B.close()
     assert max(us) >= 2.0 * min(us), (min(us), max(us))
+
+
+@pytest.mark.parametrize("mirror", [True, False])
+def test_a_finished_batch_takes_no_passes(plat, mirror):
+    """solve() with nothing left to run returns 0, whichever form the systems
+    took (an entry without its mirror keeps them on the pass kernels)."""
+    s = P.q1_system(2, 20, 9, 0.5, "done")
+    val = s.val.copy()
+    if not mirror:
+        val[s.rowptr[s.n // 2]] *= 1.0 + 1e-3
+    B = Batch(2, mixed=False, precond=True, rtol=1e-10, platform=plat)
+    B.add(s.rowptr, s.col, val, s.b)
+    assert B.solve() > 0
+    assert B.solve() == 0 and B.last_passes() == 0
+    B.close()
