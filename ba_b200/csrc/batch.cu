@@ -64,7 +64,9 @@
 // the pass budget is spent, so the device loop always ends.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
+#include <string>
 #include <type_traits>
 #include <vector>
 
@@ -1446,6 +1448,7 @@ struct b200la_batch_s {
   int list_passes;             // passes of the pass kernels in the last run
   cudaStream_t cl_stream[4];
   cudaEvent_t cl_event[5];
+  int test_fail_group;         // test hook: this group's launch fails, once (-1: none)
 };
 
 namespace {
@@ -1904,6 +1907,31 @@ int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_byte
   return B200LA_OK;
 }
 
+// Puts the side streams a launch has used in front of the context stream's
+// later work, on every way out: after an error too, the caller may read the
+// states, run again or destroy the batch.
+struct SideStreams {
+  BatchHandle B;
+  int used = 0;  // streams 0 .. used - 1 carry clusters
+  int join() {
+    cudaError_t bad = cudaSuccess;
+    for (int q = 0; q < used; ++q) {
+      cudaError_t e = cudaEventRecord(B->cl_event[q], B->cl_stream[q]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(B->ctx->stream, B->cl_event[q], 0);
+      if (e != cudaSuccess) cudaStreamSynchronize(B->cl_stream[q]);
+      if (bad == cudaSuccess) bad = e;
+    }
+    used = 0;
+    B_CUDA(bad);
+    return B200LA_OK;
+  }
+  ~SideStreams() {
+    if (used == 0) return;
+    const std::string first = b200la_last_error();
+    if (join() != B200LA_OK) fail(B200LA_ERR_CUDA, "%s", first.c_str());  // the first error stays
+  }
+};
+
 // Launches the listed systems' clusters: one launch per group of equal
 // cluster size, offset count and rows a thread, the largest clusters first,
 // on side streams between two events of the context stream, so that the
@@ -1924,16 +1952,21 @@ template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget)
   cluster_begin_kernel<<<((int)sl.size() + kBlock - 1) / kBlock, kBlock, 0, st>>>(B->cl_list, (int)sl.size(), B->st);
   B_CUDA(cudaGetLastError());
   B_CUDA(cudaEventRecord(B->cl_event[4], st));
-  int used = 0, turn = 0;
+  SideStreams side{B};
+  int turn = 0;
   for (size_t a = 0; a < sl.size();) {
     size_t e = a;
     size_t smem = 0;
     while (e < sl.size() && key(sl[e]) == key(sl[a])) smem = std::max(smem, B->sys[sl[e++]].cl_smem);
     const HostSys &h = B->sys[sl[a]];
+    if (B->test_fail_group >= 0 && turn == B->test_fail_group) {
+      B->test_fail_group = -1;
+      return fail(B200LA_ERR_CUDA, "batch: launch of cluster group %d refused by the test hook", turn);
+    }
     const int q = turn++ % 4;
-    if (q >= used) {
+    if (q >= side.used) {
       B_CUDA(cudaStreamWaitEvent(B->cl_stream[q], B->cl_event[4], 0));
-      used = q + 1;
+      side.used = q + 1;
     }
     auto go = [&](auto hh, auto rr) -> int {
       auto k = batch_cluster_kernel<T, decltype(hh)::value, decltype(rr)::value, PRE>;
@@ -1952,11 +1985,7 @@ template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget)
                                         [&](auto rr) { return go(std::integral_constant<int, kClMaxOff>(), rr); })));
     a = e;
   }
-  for (int q = 0; q < used; ++q) {
-    B_CUDA(cudaEventRecord(B->cl_event[q], B->cl_stream[q]));
-    B_CUDA(cudaStreamWaitEvent(st, B->cl_event[q], 0));
-  }
-  return B200LA_OK;
+  return side.join();
 }
 
 int launch_clusters(BatchHandle B, int budget) {
@@ -2376,6 +2405,8 @@ int b200la_batch_create(b200la_ctx ctx, const b200la_batch_params *p, b200la_bat
     memset(B->st_host, 0, sizeof(SysState) * p->capacity);
     memset(B->glob_host, 0, sizeof(BatchGlobals));
     memset(B->sym_host, 0, sizeof(int) * p->capacity);
+    const char *hook = getenv("B200LA_TEST_FAIL_GROUP");
+    B->test_fail_group = hook && hook[0] ? atoi(hook) : -1;
     ok = cudaMemsetAsync(B->st, 0, sizeof(SysState) * p->capacity, st) == cudaSuccess &&
          cudaMemsetAsync(B->glob, 0, sizeof(BatchGlobals), st) == cudaSuccess &&
          cudaStreamSynchronize(B->xfer) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;

@@ -555,3 +555,31 @@ def test_a_finished_batch_takes_no_passes(plat, mirror):
     assert B.solve() > 0
     assert B.solve() == 0 and B.last_passes() == 0
     B.close()
+
+
+def test_a_failed_cluster_launch_leaves_nothing_running(plat, monkeypatch):
+    """When the second group's launch fails, the call raises and the first
+    group's clusters, already launched on a side stream, are in front of the
+    context stream's later work: a wait for that stream finds their solution
+    written, and the next solve ends every system with the usual bits."""
+    big, small = P.q1_system(2, 250, 3, 1.0, "big"), P.q1_system(2, 20, 4, 1.0, "small")
+    items = [(s.rowptr, s.col, s.val, s.b) for s in (big, small)]
+    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=plat)
+    A = Batch(2, **kw)
+    sa = A.add_many(items)
+    A.solve()
+    ref = A.results(sa)
+    monkeypatch.setenv("B200LA_TEST_FAIL_GROUP", "1")
+    B = Batch(2, **kw)
+    monkeypatch.delenv("B200LA_TEST_FAIL_GROUP")
+    sb = B.add_many(items)
+    with pytest.raises(lmp.B200LAError, match="cluster group 1"):
+        B.launch(1 << 30)
+    plat.synchronize()
+    np.testing.assert_array_equal(B.result(sb[0]).x, ref[0].x)
+    B.solve()
+    for a, b in zip(ref, B.results(sb)):
+        assert b.solver_state == lmp.kSolverSuccess and b.iters == a.iters
+        np.testing.assert_array_equal(b.x, a.x)
+    A.close()
+    B.close()
