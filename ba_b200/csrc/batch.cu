@@ -1448,6 +1448,7 @@ struct b200la_batch_s {
   int list_passes;             // passes of the pass kernels in the last run
   cudaStream_t cl_stream[4];
   cudaEvent_t cl_event[5];
+  std::unordered_map<int, bool> cl_ready;  // kernel instances prepared (cl_prepare)
   int test_fail_group;         // test hook: this group's launch fails, once (-1: none)
 };
 
@@ -1503,15 +1504,49 @@ template <typename T, int H, int K = 0, typename F> int cl_with_rows(int rows, F
   return f(std::integral_constant<int, ClRows<T, H>::at(K)>());
 }
 
+// Calls f(kernel) with the instance for `up` upper offsets and `rows` rows a
+// thread.
+template <typename T, typename F> int cl_with_kernel(BatchHandle B, int up, int rows, F &&f) {
+  auto with_h = [&](auto h) -> int {
+    return cl_with_rows<T, decltype(h)::value>(rows, [&](auto r) -> int {
+      return B->kp.precond ? f(batch_cluster_kernel<T, decltype(h)::value, decltype(r)::value, true>)
+                           : f(batch_cluster_kernel<T, decltype(h)::value, decltype(r)::value, false>);
+    });
+  };
+  return up <= 4 ? with_h(std::integral_constant<int, 4>()) : with_h(std::integral_constant<int, kClMaxOff>());
+}
+
+int cl_instance(const HostSys &h) { return h.cl_blocks * 1000 + (h.cl_H > 4 ? 500 : 0) + h.cl_rows; }
+
+// Prepares a system's instance when the batch first meets it: the attributes
+// belong to the kernel on the device and not to a batch, so every batch, in
+// whatever thread, sets the same values (the largest block the device
+// allows), and none is touched at a launch.
+template <typename T> int cl_prepare(BatchHandle B, const HostSys &h) {
+  bool &ready = B->cl_ready[cl_instance(h)];
+  if (ready) return B200LA_OK;
+  int optin = 0;
+  B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device));
+  B_TRY((cl_with_kernel<T>(B, h.cl_H, h.cl_rows, [&](auto k) -> int {
+    cudaFuncAttributes fa;
+    B_CUDA(cudaFuncGetAttributes(&fa, k));
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return B200LA_OK;
+  })));
+  ready = true;
+  return B200LA_OK;
+}
+
 // Picks the cluster that holds a system: the smallest one it fits on, since
 // an iteration's two barriers cost the same whatever a block's rows are and
 // other systems fill the rest of the GPU.
-template <typename T> void cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
+template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
   h.cl_H = d.cl_H;
   h.cl_blocks = 0;
-  if (d.cl_H == 0) return;
+  if (d.cl_H == 0) return B200LA_OK;
   int optin = 0;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device) != cudaSuccess) return;
+  B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device));
   const int halo = d.cl_off[d.cl_H - 1];
   for (int blocks = 1; blocks <= kClMaxBlocks; blocks *= 2) {
     const int rpc = cl_rows_per_block(d.n, blocks);
@@ -1522,8 +1557,9 @@ template <typename T> void cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &
     h.cl_blocks = blocks;
     h.cl_rows = held;
     h.cl_smem = smem;
-    return;
+    return cl_prepare<T>(B, h);
   }
+  return B200LA_OK;
 }
 
 // Allocates a slot's CSR part (one chunk: CSR as uploaded, b, x and the
@@ -1936,13 +1972,10 @@ struct SideStreams {
 // cluster size, offset count and rows a thread, the largest clusters first,
 // on side streams between two events of the context stream, so that the
 // groups share the GPU.
-template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget) {
+template <typename T> int launch_clusters_t(BatchHandle B, int budget) {
   std::vector<int> &sl = B->cl_slots;
   cudaStream_t st = B->ctx->stream;
-  auto key = [&](int s) {
-    const HostSys &h = B->sys[s];
-    return h.cl_blocks * 1000 + (h.cl_H > 4 ? 500 : 0) + h.cl_rows;
-  };
+  auto key = [&](int s) { return cl_instance(B->sys[s]); };
   std::stable_sort(sl.begin(), sl.end(), [&](int a, int b) {
     const int ka = key(a), kb = key(b);
     return ka != kb ? ka > kb : B->sys[a].n > B->sys[b].n;
@@ -1968,21 +2001,13 @@ template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget)
       B_CUDA(cudaStreamWaitEvent(B->cl_stream[q], B->cl_event[4], 0));
       side.used = q + 1;
     }
-    auto go = [&](auto hh, auto rr) -> int {
-      auto k = batch_cluster_kernel<T, decltype(hh)::value, decltype(rr)::value, PRE>;
-      B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    B_TRY((cl_with_kernel<T>(B, h.cl_H, h.cl_rows, [&](auto k) -> int {
       cudaLaunchAttribute attr[1];
       const cudaLaunchConfig_t cfg = cl_config(h.cl_blocks, smem, B->cl_stream[q], attr, (int)(e - a));
       B_CUDA(cudaLaunchKernelEx(&cfg, k, (const int *)(B->cl_list + a), (const SysDesc<T> *)B->desc, B->st, B->kp,
                                 budget));
       return B200LA_OK;
-    };
-    if (h.cl_H <= 4)
-      B_TRY((cl_with_rows<T, 4>(h.cl_rows, [&](auto rr) { return go(std::integral_constant<int, 4>(), rr); })));
-    else
-      B_TRY((cl_with_rows<T, kClMaxOff>(h.cl_rows,
-                                        [&](auto rr) { return go(std::integral_constant<int, kClMaxOff>(), rr); })));
+    })));
     a = e;
   }
   return side.join();
@@ -1990,9 +2015,7 @@ template <typename T, bool PRE> int launch_clusters_t(BatchHandle B, int budget)
 
 int launch_clusters(BatchHandle B, int budget) {
   if (B->cl_slots.empty()) return B200LA_OK;
-  const bool pre = B->kp.precond != 0;
-  if (B->kp.mixed) return pre ? launch_clusters_t<float, true>(B, budget) : launch_clusters_t<float, false>(B, budget);
-  return pre ? launch_clusters_t<double, true>(B, budget) : launch_clusters_t<double, false>(B, budget);
+  return B->kp.mixed ? launch_clusters_t<float>(B, budget) : launch_clusters_t<double>(B, budget);
 }
 
 // After the states came back: adds the cluster systems of the launch to the
@@ -2268,7 +2291,8 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
   for (int k = 0; k < count; ++k) {
     if (sl[k] < 0) continue;
     HostSys &h = B->sys[sl[k]];
-    const int rc = finish_stage<T>(B, sl[k], B->chk_host[k], d[k]);
+    int rc = finish_stage<T>(B, sl[k], B->chk_host[k], d[k]);
+    if (rc == B200LA_OK) rc = cl_plan<T>(B, h, d[k]);
     if (rc != B200LA_OK) {
       free_slot_memory(B, h);
       h = HostSys();
@@ -2276,7 +2300,6 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
       continue;
     }
     desc_of<T>(h) = d[k];
-    cl_plan<T>(B, h, d[k]);
     SysState &s0 = B->st_host[sl[k]];
     memset(&s0, 0, sizeof(SysState));
     s0.phase = PH_RESID;
@@ -2483,7 +2506,7 @@ int b200la_batch_add_q1(b200la_batch B, int dim, int cells, uint64_t seed, doubl
           for (int dx = -1; dx <= 1; ++dx) full[k++] = (int)(dz * mm * mm + dy * mm + dx);
       d.cl_H = cl_offsets(full, k, d.cl_off);
     }
-    cl_plan<T>(B, h, d);
+    B_TRY((cl_plan<T>(B, h, d)));
     B_CUDA(cudaMemsetAsync(B->sym + slot, 0, sizeof(int), st));
     if (d.cl_H > 0) B_CUDA(cudaMemsetAsync(B->sym + slot, 1, 1, st));  // the low byte: 1
     B_CUDA(cudaMemcpyAsync(B->sym_host, B->sym, sizeof(int) * B->capacity, cudaMemcpyDeviceToHost, st));

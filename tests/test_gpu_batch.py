@@ -583,3 +583,37 @@ def test_a_failed_cluster_launch_leaves_nothing_running(plat, monkeypatch):
         np.testing.assert_array_equal(b.x, a.x)
     A.close()
     B.close()
+
+
+def test_batches_of_two_threads_share_the_gpu(plat):
+    """Two contexts, one thread each, run batches whose systems take the same
+    kernel instance with different amounts of shared memory (8,281 and 8,649
+    rows: 17 FP32 rows a thread of one block).  Neither may lower a limit the
+    other's launch relies on."""
+    import threading
+    errors, results = [], {}
+
+    def work(cells, reps=400):
+        try:
+            pf = lmp.Platform(0)
+            s = P.q1_system(2, cells, cells, 0.0, "thr")
+            B = Batch(1, mixed=True, precond=True, rtol=1e-2, platform=pf)
+            sl = B.add(s.rowptr, s.col, s.val, s.b)
+            out = []
+            for _ in range(reps):
+                B.restart()
+                B.run()
+            out = B.result(sl)
+            B.close()
+            results[cells] = (s, out)
+        except Exception as e:  # noqa: BLE001  (reported by the test's thread)
+            errors.append((cells, e))
+
+    ts = [threading.Thread(target=work, args=(c,)) for c in (90, 92)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for s, r in results.values():
+        assert r.solver_state == lmp.kSolverSuccess and _true_rel_res(s, r.x) < 1.001e-2
