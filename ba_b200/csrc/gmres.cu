@@ -756,7 +756,11 @@ static int gm_size_resident(GmresState *s) {
   }
   const int64_t dyn = small + (two ? 2 * bytes : bytes);
   for (const void *k : kern) {
-    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    // the limit is the kernel's, not this solver's: always the largest, so
+    // that a smaller solver made later does not lower it
+    cudaFuncAttributes fa;
+    B_CUDA(cudaFuncGetAttributes(&fa, k));
+    B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
     int per_sm = 0;
     B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kResBlock, (size_t)dyn));
     if (per_sm < 1) return B200LA_OK;

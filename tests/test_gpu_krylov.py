@@ -429,3 +429,26 @@ def test_gmres_barrier_wait_runs_out(plat, monkeypatch):
     solver, st, x = _solve_gmres(plat, s, True, 100)
     assert st == lmp.kSolverSuccess
     assert np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, s.val, x)) <= 2e-10 * np.linalg.norm(s.b)
+
+
+def test_gmres_solvers_of_several_sizes_live_together(plat):
+    """A solver launches with the shared memory its own size needs also after
+    a smaller one was made (the kernel's limit is shared by all of them).
+    Host-loop launches: the launch itself checks the limit."""
+    pf = lmp.Platform(0)
+    pf.set_graphs(False)
+    big, small = P.poisson_3d(64), P.poisson_3d(16)
+    made = []
+    for s in (big, small):
+        g = lmp.GMRES()
+        g.InitParameter(20, "NoPreconditioning")
+        g.SetupOperator(lmp.B200_CSR_lMatrix(s.rowptr, s.col, s.val, platform=pf))
+        g.InitControl(20, 0.0, 1e-30, 1e30)
+        g._ensure()
+        made.append((s, g))
+    for s, g in made:
+        b = lmp.B200_lVector.from_numpy(s.b, platform=pf)
+        x = lmp.B200_lVector(s.n, platform=pf)
+        g.Solve(b, x)
+        assert g.iter() == 20
+        assert np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, s.val, x.numpy())) < np.linalg.norm(s.b)
