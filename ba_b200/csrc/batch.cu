@@ -1448,7 +1448,9 @@ struct b200la_batch_s {
   int list_passes;             // passes of the pass kernels in the last run
   cudaStream_t cl_stream[4];
   cudaEvent_t cl_event[5];
-  std::unordered_map<int, bool> cl_ready;  // kernel instances prepared (cl_prepare)
+  // kernel instances prepared (cl_prepare): 1 can be placed, -1 not
+  std::unordered_map<int, signed char> cl_ready;
+  int test_max_cluster;        // test hook: clusters of more blocks count as not placeable
   int test_fail_group;         // test hook: this group's launch fails, once (-1: none)
 };
 
@@ -1521,26 +1523,38 @@ int cl_instance(const HostSys &h) { return h.cl_blocks * 1000 + (h.cl_H > 4 ? 50
 // Prepares a system's instance when the batch first meets it: the attributes
 // belong to the kernel on the device and not to a batch, so every batch, in
 // whatever thread, sets the same values (the largest block the device
-// allows), and none is touched at a launch.
-template <typename T> int cl_prepare(BatchHandle B, const HostSys &h) {
-  bool &ready = B->cl_ready[cl_instance(h)];
-  if (ready) return B200LA_OK;
-  int optin = 0;
+// allows), and none is touched at a launch.  *fits = whether the device can
+// place a cluster of that many blocks with that much shared memory each.
+template <typename T> int cl_prepare(BatchHandle B, const HostSys &h, bool *fits) {
+  signed char &ready = B->cl_ready[cl_instance(h)];
+  *fits = ready > 0;
+  if (ready != 0) return B200LA_OK;
+  int optin = 0, clusters = 0;
   B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device));
   B_TRY((cl_with_kernel<T>(B, h.cl_H, h.cl_rows, [&](auto k) -> int {
     cudaFuncAttributes fa;
     B_CUDA(cudaFuncGetAttributes(&fa, k));
     B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
     B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg =
+        cl_config(h.cl_blocks, (size_t)optin - fa.sharedSizeBytes, B->ctx->stream, attr);
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
+      cudaGetLastError();  // not a size this device has
+      clusters = 0;
+    }
     return B200LA_OK;
   })));
-  ready = true;
+  if (h.cl_blocks > B->test_max_cluster) clusters = 0;
+  *fits = clusters > 0;
+  ready = *fits ? 1 : -1;
   return B200LA_OK;
 }
 
 // Picks the cluster that holds a system: the smallest one it fits on, since
 // an iteration's two barriers cost the same whatever a block's rows are and
-// other systems fill the rest of the GPU.
+// other systems fill the rest of the GPU.  A system that fits on none, or only
+// on clusters the device cannot place, stays with the pass kernels.
 template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
   h.cl_H = d.cl_H;
   h.cl_blocks = 0;
@@ -1557,8 +1571,11 @@ template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d
     h.cl_blocks = blocks;
     h.cl_rows = held;
     h.cl_smem = smem;
-    return cl_prepare<T>(B, h);
+    bool fits = false;
+    B_TRY(cl_prepare<T>(B, h, &fits));
+    if (fits) return B200LA_OK;
   }
+  h.cl_blocks = 0;  // the pass kernels
   return B200LA_OK;
 }
 
@@ -2428,6 +2445,8 @@ int b200la_batch_create(b200la_ctx ctx, const b200la_batch_params *p, b200la_bat
     memset(B->st_host, 0, sizeof(SysState) * p->capacity);
     memset(B->glob_host, 0, sizeof(BatchGlobals));
     memset(B->sym_host, 0, sizeof(int) * p->capacity);
+    const char *cap = getenv("B200LA_TEST_MAX_CLUSTER");
+    B->test_max_cluster = cap && cap[0] ? atoi(cap) : kClMaxBlocks;
     const char *hook = getenv("B200LA_TEST_FAIL_GROUP");
     B->test_fail_group = hook && hook[0] ? atoi(hook) : -1;
     ok = cudaMemsetAsync(B->st, 0, sizeof(SysState) * p->capacity, st) == cudaSuccess &&

@@ -617,3 +617,21 @@ def test_batches_of_two_threads_share_the_gpu(plat):
     assert not errors, errors
     for s, r in results.values():
         assert r.solver_state == lmp.kSolverSuccess and _true_rel_res(s, r.x) < 1.001e-2
+
+
+@pytest.mark.parametrize("mixed", [True, False])
+def test_systems_whose_cluster_cannot_be_placed_use_the_pass_kernels(plat, monkeypatch, mixed):
+    """Where the device cannot place clusters above some size (here said by
+    the hook: above 1, then 4 blocks, then none at all), systems that need
+    them are solved by the pass kernels in the same batch."""
+    systems = [P.q1_system(d, c, 600 + c, 1.0, f"pl{c}") for d, c in ((2, 30), (2, 110), (2, 200), (3, 10), (3, 20))]
+    for cap in (0, 1, 4):
+        monkeypatch.setenv("B200LA_TEST_MAX_CLUSTER", str(cap))
+        B = Batch(len(systems), mixed=mixed, precond=True, rtol=1e-9, platform=plat)
+        slots = B.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
+        B.solve()
+        assert B.last_passes() > 0
+        for s, r in zip(systems, B.results(slots)):
+            assert r.solver_state == lmp.kSolverSuccess, (cap, s.name, r)
+            assert _true_rel_res(s, r.x) < (1.001e-9 if mixed else 2e-9), (cap, s.name)
+        B.close()
