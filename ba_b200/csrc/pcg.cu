@@ -869,6 +869,15 @@ static int cg_profile_t(b200la_cg s, const void *x_user, const void *b, int iter
   b200la_mat A = s->A;
   cudaStream_t st = A->ctx->stream;
   CgVecs<T> v{(T *)s->x, (T *)s->r, (T *)s->p, (T *)s->Ap, (const T *)s->invd, s->n};
+  // the grids of the three kernels on the matrix's present schedule, whatever
+  // form the solves take; what the solver has selected stays untouched
+  int grid_spmv = 0, grid_ew = 0;
+  B_TRY(grid_for(A->ctx, (const void *)cg_update_kernel<T, PRE>, (s->n + Vec16<T>::n - 1) / Vec16<T>::n, kBlock,
+                 &grid_ew));
+  B_TRY((with_schedule<M, T>(A, [&](auto op) -> int {
+    using Op = decltype(op);
+    return grid_for(A->ctx, (const void *)cg_spmv_kernel<Op, T>, op.work_items(), Op::kRowsPerBlock, &grid_spmv);
+  })));
   B_TRY((cg_launch_init_t<M, T, PRE>(s, x_user, b)));
   // every pass is queued before the first wait, after one untimed pass, so
   // the timed kernels run back to back and no host launch gap falls between
@@ -880,13 +889,13 @@ static int cg_profile_t(b200la_cg s, const void *x_user, const void *b, int iter
     if (e) cudaEventRecord(e[0], st);
     B_TRY((with_schedule<M, T>(A, [&](auto op) -> int {
       using Op = decltype(op);
-      cg_spmv_kernel<Op, T><<<s->grid_spmv, kBlock, 0, st>>>(op, v, s->part, s->sc);
+      cg_spmv_kernel<Op, T><<<grid_spmv, kBlock, 0, st>>>(op, v, s->part, s->sc);
       return B200LA_OK;
     })));
     if (e) cudaEventRecord(e[1], st);
-    cg_update_kernel<T, PRE><<<s->grid_ew, kBlock, 0, st>>>(v, s->part, s->sc);
+    cg_update_kernel<T, PRE><<<grid_ew, kBlock, 0, st>>>(v, s->part, s->sc);
     if (e) cudaEventRecord(e[2], st);
-    cg_direction_kernel<T, PRE, false><<<s->grid_ew, kBlock, 0, st>>>(v, s->sc, 0);
+    cg_direction_kernel<T, PRE, false><<<grid_ew, kBlock, 0, st>>>(v, s->sc, 0);
     if (e) cudaEventRecord(e[3], st);
     return B200LA_OK;
   };
@@ -915,7 +924,6 @@ int b200la_cg_profile(b200la_cg s, b200la_vec b, b200la_vec x, int iters, double
   B_CHECK(s && b && x && ms && iters >= 0, B200LA_ERR_INVALID, "cg_profile: bad argument");
   B_CHECK(b->n == s->n && x->n == s->n && s->n > 0, B200LA_ERR_INVALID, "cg_profile: sizes");
   B_CHECK(b->dtype == s->vdtype && x->dtype == s->vdtype, B200LA_ERR_DTYPE, "cg_profile: dtype");
-  if (!s->exec) B_TRY(cg_build_graph(s));  // the grids of the three kernels, whatever form the solves take
   return cg_types(s, [&](auto m, auto t, auto pre) -> int {
     return cg_profile_t<decltype(m), decltype(t), decltype(pre)::value>(s, x->d, b->d, iters, ms);
   });

@@ -5,6 +5,7 @@ tests/cg_test.cc: 3x3 known answers, tolerance 1e-12) and extends them to the
 generated FE systems: iteration counts equal to the reference's CG within +-1
 (FP64) and solutions within 1e-10 relative of the FP64 oracle.
 """
+import ctypes as C
 import json
 import os
 
@@ -14,7 +15,7 @@ import pytest
 import oracle
 from ba_b200 import lmp
 from ba_b200 import problems as P
-from ba_b200._lib import FMT_CSR, FMT_SELL, FMT_SELL16, FMT_STENCIL, B200LAError
+from ba_b200._lib import FMT_CSR, FMT_SELL, FMT_SELL16, FMT_STENCIL, B200LAError, call
 
 pytestmark = pytest.mark.gpu
 
@@ -661,3 +662,30 @@ def test_cg_on_chip_form_refuses_what_it_cannot_hold(plat):
     solver.Solve(_vec(plat, s.b), x)
     ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=solver.iter(), atol=0.0, rtol=1e-30, precond=False)
     assert np.linalg.norm(x.numpy() - ref.x) <= 1e-8 * np.linalg.norm(ref.x)
+
+
+def test_cg_profile_between_a_schedule_change_and_a_solve(plat):
+    """profile() leaves the form of the solves alone: after the schedule
+    changed under a solver, the next solve is sized for the new one.  FP32,
+    110,224 rows: the resident form holds 1,536 rows a block on SELL and
+    2,048 on the values-only copy, whose lanes take two rows."""
+    s = P.q1_system(2, 331, 5, 0.5, "prof")
+    b = _vec(plat, s.b, np.float32)
+    xs = []
+    for first in (FMT_SELL, FMT_STENCIL):
+        A = _mat(plat, s, np.float32)
+        A.set_format(first, 1)
+        solver = lmp.setup_CG_solver(maxits=30, atol=0.0, rtol=1e-30, dtol=1e30)
+        solver.SetupOperator(A)
+        x = _vec(plat, np.zeros(s.n), np.float32)
+        if first == FMT_SELL:
+            solver.Solve(b, x)
+            A.set_format(FMT_STENCIL, 1)
+            ms = (C.c_double * 3)()
+            call("b200la_cg_profile", solver._solver, b.handle, x.handle, 3, ms)
+            assert min(ms) > 0.0
+            x = _vec(plat, np.zeros(s.n), np.float32)
+        solver.Solve(b, x)
+        assert solver.iter() == 30
+        xs.append(x.numpy())
+    np.testing.assert_array_equal(xs[0], xs[1])
