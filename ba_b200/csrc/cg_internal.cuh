@@ -26,6 +26,7 @@ struct CgScalars {
   int stop_rule;    // B200LA_STOP_ITERATE_CONTROL or B200LA_STOP_LMP_CG
   unsigned ticket[4];
   unsigned err;     // a wait of the resident form ran out
+  int stall_block;  // test hook: this block of the resident form never joins a sum (-1: none)
 };
 
 }  // namespace b200la

@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(NT, 1) cg_resident_kernel(Op op, CgVecs<T> v, 
   const double first_res = sc->res_init;
   const CgScalars lim = *sc;  // tolerances, maxits and the stop rule
   int iter = lim.iter, state = B200LA_ITERATE;
+  if ((int)blockIdx.x == lim.stall_block) return;  // test hook: this block never joins a sum
   bool first = true;
   double s0[1] = {0.0};
   bool ok = tag_sum<1, true>(s0, ts, ++epoch);  // z and p0 are written
@@ -976,6 +977,11 @@ int b200la::cg_create_ex(b200la_mat A, const b200la_cg_params *prm, int vdtype, 
   init.maxits = prm->maxits;
   init.stop_rule = prm->stop_rule;
   init.state = B200LA_ITERATE;
+  // B200LA_TEST_STALL_BARRIER=b makes block b of the resident kernel leave
+  // before its first sum, so that the others' waits run out and the solve
+  // ends with B200LA_ERR_TIMEOUT (as in GMRES; never set in normal use)
+  const char *stall = getenv("B200LA_TEST_STALL_BARRIER");
+  init.stall_block = stall && stall[0] ? atoi(stall) : -1;
   if (cudaMemcpyAsync(s->sc, &init, sizeof(init), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return cleanup(fail(B200LA_ERR_CUDA, "cg_create: scalar upload failed"));

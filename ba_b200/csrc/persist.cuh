@@ -130,8 +130,11 @@ __device__ __forceinline__ bool tag_sum(double (&v)[NV], const TagSync &ts, unsi
       const int members = min(gs, B - g * gs);
       ok = tag_gather<NV>(s1, g * gs + lane, lane < members, epoch, ts.err, v);
       TagSlot *s2 = s1 + 2 * kTagMaxVals * kTagMaxBlocks;
+      // what each lane's slot published goes on with this block's own slot:
+      // every polling lane fences, then lane 0 stores after all of them
+      if (PUBLISH) __threadfence();
+      __syncwarp();
       if (lane == 0) {
-        if (PUBLISH) __threadfence();
 #pragma unroll
         for (int k = 0; k < NV; ++k) tag_store(s2 + k * kTagMaxBlocks + b, v[k], epoch);
       }

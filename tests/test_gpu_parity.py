@@ -689,3 +689,31 @@ def test_cg_profile_between_a_schedule_change_and_a_solve(plat):
         assert solver.iter() == 30
         xs.append(x.numpy())
     np.testing.assert_array_equal(xs[0], xs[1])
+
+
+@pytest.mark.parametrize("cells,blocks", [(160, "one level"), (331, "two levels")])
+def test_cg_resident_wait_runs_out(plat, monkeypatch, cells, blocks):
+    """One block of the resident CG leaves before its first grid-wide sum:
+    the others' waits run out (32 blocks sum in one level, 100 in two), the
+    solve returns B200LA_ERR_TIMEOUT, and the context and a new solver work.
+    An entry without its mirror keeps the smaller system off the cluster."""
+    s = P.q1_system(2, cells, 5, 0.5, "stall")
+    val = s.val.copy()
+    val[s.rowptr[s.n // 2]] *= 1.0 + 1e-3
+    A = lmp.B200_CSR_lMatrix(s.rowptr, s.col, val, platform=plat)
+    A.set_format(FMT_SELL, 1)
+    b, x = _vec(plat, s.b), _vec(plat, np.zeros(s.n))
+    monkeypatch.setenv("B200LA_TEST_STALL_BARRIER", "13")
+    solver = lmp.setup_CG_solver(maxits=5, atol=0.0, rtol=1e-12, dtol=1e8)
+    solver.SetupOperator(A)
+    with pytest.raises(B200LAError) as e:
+        solver.Solve(b, x)
+    assert e.value.status == -6 and "ran out" in str(e.value)
+    monkeypatch.delenv("B200LA_TEST_STALL_BARRIER")
+    solver = lmp.setup_CG_solver(maxits=40, atol=0.0, rtol=1e-12, dtol=1e8)
+    solver.SetupOperator(A)
+    x = _vec(plat, np.zeros(s.n))
+    solver.Solve(b, x)
+    ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=40, atol=0.0, rtol=1e-12)
+    # 40 steps of n-term sums, n eps relative each at worst (the on-chip test above)
+    assert np.linalg.norm(x.numpy() - ref.x) <= 40 * s.n * np.finfo(np.float64).eps * np.linalg.norm(ref.x)
