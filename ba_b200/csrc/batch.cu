@@ -1000,7 +1000,8 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
   const SysDesc<T> &d = desc[sys];
   SysState &S = st[sys];
   int phase = *(volatile int *)&S.phase;
-  if (phase != PH_RESID && phase != PH_INNER && phase != PH_START) return;
+  // a run ends between passes, so START never waits for a later one here
+  if (phase != PH_RESID && phase != PH_INNER) return;
   ClMatrix<double> m;
   m.n = d.n;
   m.H = d.cl_H;
@@ -1021,23 +1022,22 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
     g.c[j] = d.c[row];
     if (PRE) g.d[j] = d.invd[row];
   });
-  // the state as the last kernel left it (both parities alike for systems
-  // that run here; a fresh state is zero)
+  // the state as the last run left it (both parities alike: a system listed
+  // here never runs in the pass kernels, whose timings end with a restart)
   double rz = S.rzb[0], rz_keep = S.rz_keep, res = S.res, res0 = S.res0, res_in = S.res_in, res_in0 = S.res_in0;
   int it = S.itb[0], tot = S.totb[0], outer = S.outer, keep_p = S.keep_p, state = S.state;
   const bool diag_ok = !prm.precond || S.bad_row == 0xffffffffu;
   unsigned long long t_done = S.t_done;
   int set = 0, passes = 0;
-  // START left open by a run of the pass kernels: the direction, then INNER
+  // the new direction from a replaced residual, whose halo the residual pass
+  // has pushed, then INNER
   auto start = [&]() {
     const double beta_d = keep_p ? rz / rz_keep : 0.0;
     const bool use = keep_p && isfinite(beta_d);
     g.direction((T)beta_d, use, [](int, T) {});
     phase = PH_INNER;
   };
-  if (phase == PH_START && g.blocks > 1) g.each([&](int j, int li) { g.push(li, PRE ? g.r[j] * g.d[j] : g.r[j]); });
   cl_barrier(g.blocks);  // every block of the cluster runs and has its window
-  if (phase == PH_START) start();
   while (phase != PH_DONE && passes < budget) {
     ++passes;
     if (phase == PH_RESID) {
