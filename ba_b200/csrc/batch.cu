@@ -1566,7 +1566,7 @@ template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d
     const int rpc = cl_rows_per_block(d.n, blocks);
     const int need = (rpc + kClThreads - 1) / kClThreads;
     const int held = d.cl_H <= 4 ? cl_rows_for<T, 4>(need) : cl_rows_for<T, kClMaxOff>(need);
-    const size_t smem = cl_smem_bytes(rpc, halo, d.cl_H, sizeof(T));
+    const size_t smem = cl_smem_bytes(rpc, halo, d.cl_H, held, sizeof(T));
     if (held == 0 || smem + 1024 > (size_t)optin) continue;
     h.cl_blocks = blocks;
     h.cl_rows = held;

@@ -64,13 +64,24 @@ inline int cl_offsets(const int *off, int len, int *up) {
   return H;
 }
 
-// Dynamic shared memory of one block: p window, values, halo z, sum slots.
-inline size_t cl_smem_bytes(int rpc, int halo, int H, size_t ts) {
-  const int HP = H <= 4 ? 4 : kClMaxOff;
-  size_t b = ts * ((size_t)rpc + 2 * halo) + ts * (size_t)(HP + 1) * (rpc + halo) + ts * 2 * (size_t)halo;
+// Dynamic shared memory of one block whose threads hold `held` rows each
+// (the instance's count): p window, values, halo z, sum slots.  The product
+// loop also reads, and discards, the held * kClThreads - rpc rows past the
+// block's own (multiply()); what follows the values takes that, and where it
+// would not, the block gets the difference.
+constexpr size_t cl_smem_bytes(int rpc, int halo, int H, int held, size_t ts) {
+  const size_t HP = H <= 4 ? 4 : kClMaxOff;
+  const size_t values = ts * ((size_t)rpc + 2 * (size_t)halo) + ts * (HP + 1) * ((size_t)rpc + halo);
+  size_t b = values + ts * 2 * (size_t)halo;
   b = (b + 15) & ~(size_t)15;
-  return b + sizeof(double) * 2 * kClSums * kClMaxBlocks * kClWarps;
+  b += sizeof(double) * 2 * kClSums * kClMaxBlocks * kClWarps;
+  const size_t past = values + ts * ((size_t)held * kClThreads - (size_t)rpc);
+  return b > past ? b : past;
 }
+// 3,104 FP64 rows on instances of 9: 1,504 values past the end; with rows of
+// 1 a thread on instances of 4 the block is enlarged.
+static_assert(cl_smem_bytes(3104, 1, 4, 9, 8) >= 8 * (3106 + 4 * 3105 + 9 * kClThreads + 1), "reads past the block");
+static_assert(cl_smem_bytes(32, 1, 4, 4, 8) >= 8 * (34 + 4 * 33 + 4 * kClThreads + 1), "reads past the block");
 inline int cl_rows_per_block(int n, int blocks) { return ((n + blocks - 1) / blocks + 31) & ~31; }
 
 // Launch configuration of `systems` clusters of `blocks` blocks (attr must
@@ -264,9 +275,9 @@ template <typename T, int H, int R, bool PRE> struct ClCg {
 
   // ap = A p; returns this thread's share of p.Ap.  Straight-line over the R
   // rows, so that the loads of one row overlap the sums of another: rows past
-  // the block's own read what lies there in shared memory (at most NT + 31
-  // values past an array's end, the sum slots at the latest) and are then
-  // set to zero, and rows that hold only their diagonal are selected.
+  // the block's own read what lies there in shared memory (R NT - rpc values
+  // past an array's end at most, inside the block: cl_smem_bytes) and are
+  // then set to zero, and rows that hold only their diagonal are selected.
   __device__ __forceinline__ double multiply() {
     ClAcc acc;
 #pragma unroll

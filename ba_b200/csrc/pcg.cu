@@ -703,13 +703,16 @@ template <typename M, typename T, bool PRE> static int cg_size_resident_t(b200la
 
 constexpr int kCgClRows = 9;  // most rows a thread of the cluster form (257 x 257 nodes on 16 blocks)
 
+// Rows a thread of the instance that holds `need` of them (<= kCgClRows).
+static int cg_cluster_rows(int need) { return need <= 1 ? 1 : need <= 3 ? 3 : need <= 6 ? 6 : kCgClRows; }
+
 // Calls f(H, R) (integral constants) for a cluster solve with `up` upper
-// offsets and `regs` rows a thread.
+// offsets and `regs` (a value of cg_cluster_rows) rows a thread.
 template <typename T, typename F> static int cl_dispatch(int up, int regs, F &&f) {
   auto with_r = [&](auto h) -> int {
-    if (regs <= 1) return f(h, std::integral_constant<int, 1>());
-    if (regs <= 3) return f(h, std::integral_constant<int, 3>());
-    if (regs <= 6) return f(h, std::integral_constant<int, 6>());
+    if (regs == 1) return f(h, std::integral_constant<int, 1>());
+    if (regs == 3) return f(h, std::integral_constant<int, 3>());
+    if (regs == 6) return f(h, std::integral_constant<int, 6>());
     return f(h, std::integral_constant<int, kCgClRows>());
   };
   return up <= 4 ? with_r(std::integral_constant<int, 4>()) : with_r(std::integral_constant<int, kClMaxOff>());
@@ -754,8 +757,8 @@ template <typename M, typename T, bool PRE> static int cg_size_cluster_t(b200la_
   const int rpc = cl_rows_per_block((int)s->n, blocks);
   const int need = (rpc + kClThreads - 1) / kClThreads;
   if (need > kCgClRows) return B200LA_OK;
-  const int regs = need;
-  const size_t smem = cl_smem_bytes(rpc, A->cl_off[A->cl_H - 1], A->cl_H, sizeof(T));
+  const int regs = cg_cluster_rows(need);
+  const size_t smem = cl_smem_bytes(rpc, A->cl_off[A->cl_H - 1], A->cl_H, regs, sizeof(T));
   return cl_dispatch<T>(A->cl_H, regs, [&](auto h, auto r) -> int {
     auto k = cg_cluster_kernel<M, T, decltype(h)::value, decltype(r)::value, PRE>;
     cudaFuncAttributes fa;
