@@ -16,6 +16,7 @@ F64, F32 = 0, 1
 FMT_CSR, FMT_SELL, FMT_SELL16, FMT_STENCIL = 1, 4, 5, 6
 FORMAT_NAMES = {FMT_CSR: "csr", FMT_SELL: "sell", FMT_SELL16: "sell16", FMT_STENCIL: "stencil"}
 ITERATE, SUCCESS_ABS, SUCCESS_REL, FAIL_DIV, FAIL_MAXITS, FAIL_BREAKDOWN, DONE_FIXED = range(7)
+FORM_KERNELS, FORM_CLUSTER, FORM_RESIDENT = 0, 1, 2
 METHOD_JACOBI, METHOD_BICGSTAB, METHOD_GMRES = 1, 2, 3
 SOLVER_SUCCESS, SOLVER_EXCEEDED, SOLVER_ERROR = range(3)
 STATUS_NAMES = {0: "OK", -1: "ERR_INVALID", -2: "ERR_CUDA", -3: "ERR_NOMEM", -4: "ERR_DTYPE",
@@ -104,6 +105,7 @@ _SIGS = {
     "b200la_ctx_get_stream": [_vp, _P(_vp)],
     "b200la_ctx_synchronize": [_vp],
     "b200la_ctx_set_graphs": [_vp, _i],
+    "b200la_ctx_set_onchip": [_vp, _i],
     "b200la_ctx_num_sms": [_vp, _P(_i)],
     "b200la_vec_create": [_vp, _i64, _i, _P(_vp)],
     "b200la_vec_wrap": [_vp, _i64, _i, _vp, _P(_vp)],
@@ -145,6 +147,7 @@ _SIGS = {
     "b200la_cg_create": [_vp, _P(CgParams), _P(_vp)],
     "b200la_cg_destroy": [_vp],
     "b200la_cg_solve": [_vp, _vp, _vp, _P(CgResult)],
+    "b200la_cg_form": [_vp, _P(_i)],
     "b200la_cg_profile": [_vp, _vp, _vp, _i, _P(_d)],
     "b200la_pcg_solve": [_vp, _vp, _vp, _P(CgParams), _P(CgResult)],
     "b200la_solver_create": [_vp, _P(SolverParams), _P(_vp)],
@@ -174,6 +177,7 @@ _SIGS = {
     "b200la_batch_add_q1": [_vp, _i, _i, C.c_uint64, _d, _P(_i)],
     "b200la_batch_add_many": [_vp, _i, _P(_i), _P(_i64), _P(_vp), _P(_vp), _P(_vp), _P(_vp), _P(_vp), _P(_i), _P(_i)],
     "b200la_batch_get_system": [_vp, _i, _vp, _vp, _vp, _vp],
+    "b200la_batch_form": [_vp, _i, _P(_i)],
     "b200la_batch_slot_size": [_vp, _i, _P(_i), _P(_i64)],
     "b200la_server_start": [_vp, _P(ServerParams), _P(_vp)],
     "b200la_server_stop": [_vp],

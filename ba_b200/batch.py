@@ -203,6 +203,12 @@ class Batch:
         return [SystemResult(r.state, r.solver_state, r.iters, r.outer, bool(r.phase_done), r.res, r.res_init,
                              r.res_rel, r.device_us, None if xs is None else xs[j]) for j, r in enumerate(rs)]
 
+    def form(self, slot: int) -> int:
+        """FORM_CLUSTER for a system solved on a cluster, else FORM_KERNELS."""
+        f = C.c_int()
+        call("b200la_batch_form", self.handle, int(slot), C.byref(f))
+        return f.value
+
     def slot_n(self, slot: int) -> int:
         return self._sizes[slot]
 

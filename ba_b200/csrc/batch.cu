@@ -1558,7 +1558,7 @@ template <typename T> int cl_prepare(BatchHandle B, const HostSys &h, bool *fits
 template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
   h.cl_H = d.cl_H;
   h.cl_blocks = 0;
-  if (d.cl_H == 0) return B200LA_OK;
+  if (d.cl_H == 0 || !B->ctx->use_onchip) return B200LA_OK;
   int optin = 0;
   B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device));
   const int halo = d.cl_off[d.cl_H - 1];
@@ -2572,6 +2572,13 @@ int b200la_batch_slot_size(b200la_batch B, int slot, int *n, int64_t *nnz) {
   B_CHECK(B && slot >= 0 && slot < B->capacity && B->sys[slot].used, B200LA_ERR_INVALID, "batch_slot_size: slot");
   if (n) *n = B->sys[slot].n;
   if (nnz) *nnz = B->sys[slot].nnz;
+  return B200LA_OK;
+}
+
+int b200la_batch_form(b200la_batch B, int slot, int *form) {
+  B_CHECK(B && form && slot >= 0 && slot < B->capacity && B->sys[slot].used, B200LA_ERR_INVALID, "batch_form: slot");
+  B_CUDA(cudaEventSynchronize(B->xfer_done));  // the symmetry verdict of an add
+  *form = B->sys[slot].cl_blocks > 0 && B->sym_host[slot] ? B200LA_FORM_CLUSTER : B200LA_FORM_KERNELS;
   return B200LA_OK;
 }
 

@@ -46,6 +46,7 @@ struct b200la_cg_s {
   cudaGraphExec_t exec;
   int g_format, g_param;       // schedule baked into the graph
   int g_gen;                   // the matrix's schedule generation at capture
+  bool g_onchip;               // the context's on-chip switch when the form was picked
   int grid_spmv, grid_ew;
   // cluster form (cg_cluster_kernel): 0 blocks = not used
   int cl_blocks, cl_regs;      // blocks of the cluster, rows a thread

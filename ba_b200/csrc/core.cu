@@ -294,6 +294,7 @@ int b200la_ctx_create(int device, b200la_ctx *out) {
   {
     const char *g = getenv("B200LA_GRAPHS");
     c->use_graphs = !(g && g[0] == '0');
+    c->use_onchip = true;
   }
   B_CUDA(cudaMalloc(&c->scratch.part, sizeof(double) * 4 * kMaxReduceBlocks));
   B_CUDA(cudaMalloc(&c->scratch.ticket, sizeof(unsigned) * 16));
@@ -343,6 +344,12 @@ int b200la_ctx_get_stream(b200la_ctx c, void **stream) {
 int b200la_ctx_set_graphs(b200la_ctx c, int on) {
   B_CHECK(c, B200LA_ERR_INVALID, "ctx_set_graphs: null ctx");
   c->use_graphs = on != 0;
+  return B200LA_OK;
+}
+
+int b200la_ctx_set_onchip(b200la_ctx c, int on) {
+  B_CHECK(c, B200LA_ERR_INVALID, "ctx_set_onchip: null ctx");
+  c->use_onchip = on != 0;
   return B200LA_OK;
 }
 

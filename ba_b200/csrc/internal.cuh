@@ -65,6 +65,7 @@ struct b200la_ctx_s {
   // a profiler can see each launch (ncu does not profile kernels inside
   // graphs with conditional nodes).
   bool use_graphs;
+  bool use_onchip;  // CG and batch systems that fit run on chip
   // resident blocks per SM of each kernel launched so far (grid_for), so a
   // call does not ask the driver again
   std::unordered_map<const void *, int> occupancy;

@@ -566,7 +566,9 @@ static int cg_build_graph(b200la_cg s);
 // kernel, or the three kernels (whose graph is built here).
 static int cg_select_form(b200la_cg s) {
   b200la_mat A = s->A;
-  s->res_blocks = 0;
+  s->cl_blocks = s->res_blocks = 0;
+  s->g_onchip = A->ctx->use_onchip;
+  if (!s->g_onchip) return cg_build_graph(s);
   B_TRY(cg_types(s, [&](auto m, auto t, auto pre) -> int {
     using M = decltype(m);
     using T = decltype(t);
@@ -833,7 +835,9 @@ template <typename M, typename T, bool PRE> static int cg_run_resident_t(b200la_
 
 int cg_run(b200la_cg s) {
   b200la_mat A = s->A;
-  if (A->format != s->g_format || A->param != s->g_param || A->sched_gen != s->g_gen) B_TRY(cg_select_form(s));
+  if (A->format != s->g_format || A->param != s->g_param || A->sched_gen != s->g_gen ||
+      A->ctx->use_onchip != s->g_onchip)
+    B_TRY(cg_select_form(s));
   if (s->cl_blocks > 0)
     return cg_types(s, [&](auto m, auto t, auto pre) -> int {
       return cg_run_cluster_t<decltype(m), decltype(t), decltype(pre)::value>(s);
@@ -923,6 +927,12 @@ static int cg_profile_t(b200la_cg s, const void *x_user, const void *b, int iter
 }  // namespace b200la
 
 extern "C" {
+
+int b200la_cg_form(b200la_cg s, int *form) {
+  B_CHECK(s && form, B200LA_ERR_INVALID, "cg_form: null argument");
+  *form = s->cl_blocks > 0 ? B200LA_FORM_CLUSTER : s->res_blocks > 0 ? B200LA_FORM_RESIDENT : B200LA_FORM_KERNELS;
+  return B200LA_OK;
+}
 
 int b200la_cg_profile(b200la_cg s, b200la_vec b, b200la_vec x, int iters, double *ms) {
   B_CHECK(s && b && x && ms && iters >= 0, B200LA_ERR_INVALID, "cg_profile: bad argument");

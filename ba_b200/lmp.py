@@ -62,6 +62,11 @@ class Platform:
         False, launch the same kernels one by one from a host loop."""
         call("b200la_ctx_set_graphs", self.handle, 1 if on else 0)
 
+    def set_onchip(self, on: bool):
+        """Let CG solves and batch systems that fit run on chip (default) or,
+        with False, keep to the streamed kernels."""
+        call("b200la_ctx_set_onchip", self.handle, 1 if on else 0)
+
     @property
     def num_sms(self) -> int:
         n = C.c_int()
@@ -455,6 +460,13 @@ class CG:
         self.iter_, self.state_ = r.iters, r.state
         self.res_, self.res_init_, self.res_rel_ = r.res, r.res_init, r.res_rel
         return r.solver_state
+
+    def form(self) -> int:
+        """How the last solve ran: FORM_KERNELS, FORM_CLUSTER or FORM_RESIDENT."""
+        self._ensure()
+        f = C.c_int()
+        call("b200la_cg_form", self._solver, C.byref(f))
+        return f.value
 
     def iter(self) -> int:
         return self.iter_

@@ -338,3 +338,28 @@ def random_spd(n: int, seed: int, density: float = 0.1, empty_rows: int = 0) -> 
     b = rng.random(n)
     return CSRSystem(0, 0, rowptr, cols.astype(np.int32), a[rows, cols].astype(np.float64), b,
                      np.zeros(n, dtype=bool), f"random_spd_{n}")
+
+
+def offsets_spd(n: int, offs, seed: int) -> CSRSystem:
+    """Symmetric diagonally dominant matrix whose rows' columns are the row
+    plus a subset of +-offs, for edge-case parity: one entry pair in 30 is
+    absent, the middle rows have them all."""
+    rng = np.random.default_rng(seed)
+    rows, cols, vals = [], [], []
+    for o in offs:
+        i = np.arange(n - o)
+        w = -rng.uniform(0.5, 1.5, n - o)
+        mid = n // 2
+        keep = (rng.random(n - o) >= 1.0 / 30.0) | (np.abs(i - mid) <= 1) | (np.abs(i + o - mid) <= 1)
+        i, w = i[keep], w[keep]
+        rows += [i, i + o]
+        cols += [i + o, i]
+        vals += [w, w]
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    diag = np.bincount(r, weights=-v, minlength=n) + rng.uniform(0.001, 0.01, n)
+    r, c, v = np.concatenate([r, np.arange(n)]), np.concatenate([c, np.arange(n)]), np.concatenate([v, diag])
+    order = np.lexsort((c, r))
+    rowptr = np.zeros(n + 1, dtype=np.int32)
+    np.cumsum(np.bincount(r, minlength=n), out=rowptr[1:])
+    return CSRSystem(0, 0, rowptr, c[order].astype(np.int32), v[order], rng.random(n), np.zeros(n, dtype=bool),
+                     f"offsets_spd_{n}")

@@ -87,6 +87,11 @@ int b200la_ctx_get_stream(b200la_ctx ctx, void **stream);
  * loop lets a profiler or a launch record see every kernel.  Takes effect at
  * the next solve or run. */
 int b200la_ctx_set_graphs(b200la_ctx ctx, int on);
+/* CG solves and batch systems that fit run on chip (one launch, see
+ * b200la_cg_form, b200la_batch_form); with on = 0 this context keeps to the
+ * streamed kernels: CG from its next solve, a batch for the systems it adds
+ * from then on. */
+int b200la_ctx_set_onchip(b200la_ctx ctx, int on);
 int b200la_ctx_synchronize(b200la_ctx ctx);
 int b200la_ctx_num_sms(b200la_ctx ctx, int *out);
 
@@ -266,6 +271,14 @@ int b200la_cg_create(b200la_mat A, const b200la_cg_params *params, b200la_cg *ou
 int b200la_cg_destroy(b200la_cg s);
 /* Solve(b, &x): x holds the start value on entry and the solution on exit. */
 int b200la_cg_solve(b200la_cg s, b200la_vec b, b200la_vec x, b200la_cg_result *result);
+/* How the solver's last solve ran (before the first: how it would run):
+ * FORM_KERNELS three kernels an iteration, FORM_CLUSTER one launch with matrix
+ * and vectors on one cluster, FORM_RESIDENT one launch with the vectors on
+ * resident blocks. */
+#define B200LA_FORM_KERNELS 0
+#define B200LA_FORM_CLUSTER 1
+#define B200LA_FORM_RESIDENT 2
+int b200la_cg_form(b200la_cg s, int *form);
 /* Instrumentation: from the start value x, runs `iters` iterations as
  * separate launches with CUDA events between the kernels (the graph's three
  * kernels, whatever form the solves take) and writes the mean milliseconds per launch of
@@ -493,6 +506,9 @@ int b200la_batch_add_many(b200la_batch b, int count, const int *n, const int64_t
 /* Copy a slot's system back to the host (any pointer may be NULL). */
 int b200la_batch_get_system(b200la_batch b, int slot, int *rowptr, int *col, double *val, double *rhs);
 int b200la_batch_slot_size(b200la_batch b, int slot, int *n, int64_t *nnz);
+/* Whether the slot's system is solved by the swept kernels (FORM_KERNELS) or
+ * on a cluster (FORM_CLUSTER). */
+int b200la_batch_form(b200la_batch b, int slot, int *form);
 /* Frees a slot (stream-ordered: after the work already queued; no wait). */
 int b200la_batch_remove(b200la_batch b, int slot);
 /* Frees `count` slots at once (all must be in use and distinct, else nothing

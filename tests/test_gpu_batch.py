@@ -14,6 +14,7 @@ import pytest
 import oracle
 from ba_b200 import lmp
 from ba_b200 import problems as P
+from ba_b200._lib import FORM_CLUSTER, FORM_KERNELS
 from ba_b200.batch import Batch
 
 pytestmark = pytest.mark.gpu
@@ -22,6 +23,16 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture(scope="module")
 def plat():
     return lmp.init_platform(0)
+
+
+@pytest.fixture(scope="module", params=["clusters", "pass kernels"])
+def either(request):
+    """A context whose small structured systems run on clusters, and one that
+    keeps every system on the pass kernels."""
+    pf = lmp.Platform(0)
+    pf.set_onchip(request.param == "clusters")
+    pf.want = FORM_CLUSTER if request.param == "clusters" else FORM_KERNELS
+    return pf
 
 
 def _mix(seed=1, count=12):
@@ -34,9 +45,9 @@ def _mix(seed=1, count=12):
     return out
 
 
-def test_fp64_batch_matches_reference_cg(plat):
+def test_fp64_batch_matches_reference_cg(either):
     systems = _mix()
-    B = Batch(len(systems), mixed=False, precond=True, rtol=1e-10, atol=0.0, dtol=1e8, platform=plat)
+    B = Batch(len(systems), mixed=False, precond=True, rtol=1e-10, atol=0.0, dtol=1e8, platform=either)
     slots = [B.add_system(s) for s in systems]
     assert B.run() == 0
     for s, sl in zip(systems, slots):
@@ -83,10 +94,10 @@ def _true_rel_res(s, x):
     return np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, s.val, x)) / np.linalg.norm(s.b)
 
 
-def test_mixed_batch_reaches_tolerance(plat):
+def test_mixed_batch_reaches_tolerance(either):
     sizes = P.batch_sizes(24, lo=16, hi=64, seed=5)
     systems = [P.q1_system(2, int(n), 500 + k, 1.0, f"b{k}") for k, n in enumerate(sizes)]
-    B = Batch(32, mixed=True, precond=True, rtol=1e-8, platform=plat)
+    B = Batch(32, mixed=True, precond=True, rtol=1e-8, platform=either)
     B.tune()
     slots = [B.add_system(s) for s in systems]
     assert B.run() == 0
@@ -103,7 +114,7 @@ def test_mixed_batch_reaches_tolerance(plat):
 
 
 @pytest.mark.parametrize("restart", [False, True])
-def test_mixed_batch_passes_match_oracle(plat, restart):
+def test_mixed_batch_passes_match_oracle(either, restart):
     """Mixed mode per system against the oracle's restatement of the same
     refinement: with kept directions (default; oracle.mpcg_kept) and
     restarted per pass (oracle.mpir, MPIR's form), both with the batch's
@@ -113,7 +124,7 @@ def test_mixed_batch_passes_match_oracle(plat, restart):
     systems = _mix(seed=7, count=9)
     irt = 1e-4 if restart else 0.1
     B = Batch(16, mixed=True, precond=True, rtol=1e-9, inner_rtol=irt, restart_inner=restart, max_outer=40,
-              platform=plat)
+              platform=either)
     slots = B.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
     B.solve()
     rows = []
@@ -131,10 +142,10 @@ def test_mixed_batch_passes_match_oracle(plat, restart):
     assert not bad, rows
 
 
-def test_isolation_alone_vs_mix_vs_late_admission(plat):
+def test_isolation_alone_vs_mix_vs_late_admission(either):
     systems = _mix(seed=3, count=9)
     probe = systems[4]
-    kw = dict(mixed=True, precond=True, rtol=1e-9, platform=plat)
+    kw = dict(mixed=True, precond=True, rtol=1e-9, platform=either)
     # alone
     A = Batch(1, **kw)
     a = A.add_system(probe)
@@ -228,14 +239,14 @@ def test_malformed_csr_is_refused_on_the_device_check(plat):
     assert r.solver_state == lmp.kSolverSuccess and _true_rel_res(good, r.x) < 1.001e-8
 
 
-def test_add_many_matches_single_adds_and_reports_per_system_status(plat):
+def test_add_many_matches_single_adds_and_reports_per_system_status(either):
     """The bulk add gives each system the result it gets from a single add
     (bit for bit) and reports a malformed one on its own."""
     systems = _mix(seed=4, count=5)
-    A = Batch(8, mixed=True, rtol=1e-8, platform=plat)
+    A = Batch(8, mixed=True, rtol=1e-8, platform=either)
     one = [A.add_system(s) for s in systems]
     A.solve()
-    M = Batch(8, mixed=True, rtol=1e-8, platform=plat)
+    M = Batch(8, mixed=True, rtol=1e-8, platform=either)
     bad = (np.array([0, 2, 3], np.int32), np.array([0, 9, 1], np.int32), np.ones(3), np.ones(2))
     items = [(s.rowptr, s.col, s.val, s.b) for s in systems]
     items.insert(2, bad)
@@ -282,13 +293,13 @@ def test_large_system_ticket_path_isolated_and_converged(plat):
         assert np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, s.val, r.x)) <= 1.001e-8 * np.linalg.norm(s.b)
 
 
-def test_adds_overlapping_launches_match_the_plain_solve(plat):
+def test_adds_overlapping_launches_match_the_plain_solve(either):
     # systems added in chunks while earlier chunks already iterate (adds on the
     # batch's transfer stream, launches asynchronous) end bit for bit as when
     # all are added first: a system's arithmetic does not depend on when it
     # joined or on what else runs
     systems = _mix(seed=5, count=12)
-    kw = dict(mixed=True, precond=True, rtol=1e-9, platform=plat)
+    kw = dict(mixed=True, precond=True, rtol=1e-9, platform=either)
     A = Batch(16, **kw)
     A.set_items(128, 512, 512, adaptive=False)
     slots_a = A.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
@@ -312,14 +323,14 @@ def test_adds_overlapping_launches_match_the_plain_solve(plat):
         np.testing.assert_array_equal(g.x, r.x)
 
 
-def test_initial_guesses_in_one_add_many(plat):
+def test_initial_guesses_in_one_add_many(either):
     # one add_many call mixing systems with an initial guess (copied to x) and
     # without (x zeroed by the setup kernel): the latter repeat a plain run bit
     # for bit, the former start from their guess (res_init is its residual)
     # and reach the tolerance relative to it
     sizes = P.batch_sizes(8, lo=16, hi=48, seed=9)
     systems = [P.q1_system(2, int(n), 900 + k, 1.0, f"g{k}") for k, n in enumerate(sizes)]
-    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=plat)
+    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=either)
     A = Batch(8, **kw)
     sa = A.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
     A.solve(16)
@@ -342,7 +353,7 @@ def test_initial_guesses_in_one_add_many(plat):
     B.close()
 
 
-def test_registered_outputs_are_copied_as_systems_finish(plat):
+def test_registered_outputs_are_copied_as_systems_finish(either):
     # solutions registered with set_outputs are copied out on the transfer
     # stream when a run sees their system finished; results(out=...) then
     # only waits.  They equal the plain read bit for bit; status-only reads
@@ -350,7 +361,7 @@ def test_registered_outputs_are_copied_as_systems_finish(plat):
     import torch
     sizes = P.batch_sizes(12, lo=16, hi=96, seed=21)
     systems = [P.q1_system(2, int(n), 40 + k, 1.0, f"o{k}") for k, n in enumerate(sizes)]
-    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=plat)
+    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=either)
     A = Batch(12, **kw)
     sa = A.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
     A.solve(8)
@@ -403,7 +414,7 @@ def test_remove_many(plat):
     ref.close()
 
 
-def test_remove_and_reuse_slots_while_a_launch_is_in_flight(plat):
+def test_remove_and_reuse_slots_while_a_launch_is_in_flight(either):
     # running systems are removed while an asynchronous launch is in flight and
     # new systems are added into the freed slots at once.  The removal clears
     # the slots' states on the solve stream after the launch; the adds run on
@@ -413,7 +424,7 @@ def test_remove_and_reuse_slots_while_a_launch_is_in_flight(plat):
     # must end with the bits it gets when solved alone.
     first = [P.q1_system(2, c, 300 + k, 1.0, f"f{k}") for k, c in enumerate((160, 200, 180, 220))]
     second = [P.q1_system(2, c, 400 + k, 1.0, f"s{k}") for k, c in enumerate((40, 64, 90))]
-    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=plat)
+    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=either)
 
     def alone(s):
         A = Batch(1, **kw)
@@ -444,21 +455,23 @@ def test_remove_and_reuse_slots_while_a_launch_is_in_flight(plat):
 
 
 @pytest.mark.parametrize("mixed", [True, False])
-def test_column_storages_give_the_same_bits(plat, mixed):
+def test_column_storages_give_the_same_bits(either, mixed):
     # the sliced copy stores no columns (values-only stencil layout, Q1
     # systems), int16 offsets or int32 columns: each row adds the same
     # products in the same order whatever the storage, so every system --
     # uploaded CSR (stencil found by the device check), device-assembled Q1
     # (stencil known), and a random matrix (no stencil) -- ends bit for bit
-    # the same in all three
+    # the same in all three.  On the pass kernels the storages are what the
+    # kernels read; systems on clusters read the CSR whatever the storage
     systems = _mix(seed=9, count=9) + [P.random_spd(300, 4, density=0.02)]
     q1 = [(2, 37, 5, 1.0), (3, 9, 6, 2.0), (2, 3, 7, 0.5)]
     out = {}
     for bits in (0, 16, 32):
-        B = Batch(16, mixed=mixed, precond=True, rtol=1e-9, index_bits=bits, platform=plat)
+        B = Batch(16, mixed=mixed, precond=True, rtol=1e-9, index_bits=bits, platform=either)
         B.set_items(128, 512, 512, adaptive=False)
         slots = B.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
         slots += [B.add_q1(*a) for a in q1]
+        assert B.form(slots[0]) == either.want and B.form(slots[len(systems) - 1]) == FORM_KERNELS
         B.solve(16)
         out[bits] = B.results(slots)
         B.close()
@@ -471,8 +484,7 @@ def test_column_storages_give_the_same_bits(plat, mixed):
 
 # Sizes where the cluster form of a batch changes hands: one block up to 17
 # FP32 (9 FP64) rows a thread, then 2, 4, 8 and 16 blocks, the rows-a-thread
-# counts between, windows wider than a block's rows (3D), the pass kernels
-# beyond.  Each system is held to the FP64 oracle and must not move by a bit
+# counts between, the pass kernels beyond (3D 26 in FP64).  Each system is held to the FP64 oracle and must not move by a bit
 # when others run beside it or the run is cut into pieces.
 @pytest.mark.parametrize("mixed", [True, False])
 def test_cluster_systems_match_oracle_and_are_isolated(plat, mixed):
@@ -483,7 +495,11 @@ def test_cluster_systems_match_oracle_and_are_isolated(plat, mixed):
     slots = B.add_many([(s.rowptr, s.col, s.val, s.b) for s in systems])
     B.solve()
     res = B.results(slots)
-    for s, r in zip(systems, res):
+    for s, sl, r in zip(systems, slots, res):
+        # 3D: 27^3 FP64 rows fit no cluster; of 4^3 nodes both middle rows, where
+        # the offsets are looked for, lie on the boundary
+        fits = s.dim == 2 or (s.n != 64 and (mixed or s.n <= 10000))
+        assert B.form(sl) == (FORM_CLUSTER if fits else FORM_KERNELS), (s.dim, s.n)
         assert r.solver_state == 0, (s.name, s.n, r)
         ref = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=100000, atol=0.0, rtol=1e-13)
         # the residual ends at 1e-9 ||b||; Jacobi-scaled systems of these sizes keep
@@ -510,23 +526,59 @@ def test_cluster_systems_match_oracle_and_are_isolated(plat, mixed):
         A1.close()
 
 
-def test_cluster_form_refuses_unsymmetric_values(plat):
-    """An entry without its mirror keeps a system on the pass kernels, with
-    the results they give."""
-    s = P.q1_system(2, 20, 9, 0.5, "unsym")
-    val = s.val.copy()
-    val[s.rowptr[s.n // 2]] *= 1.0 + 2.0 ** -40  # one bit pattern off
-    outs = []
-    for bits in (0, 32):
-        B = Batch(1, mixed=False, precond=True, rtol=1e-10, platform=plat, index_bits=bits)
-        sl = B.add(s.rowptr, s.col, val, s.b)
-        B.solve()
-        outs.append(B.result(sl))
-        B.close()
-    assert outs[0].solver_state == 0 and np.array_equal(outs[0].x, outs[1].x)
-    ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=10000, atol=0.0, rtol=1e-13)
-    assert np.linalg.norm(outs[0].x - ref.x) <= 1e-8 * np.linalg.norm(ref.x)
+# Offset sets other than a grid's (3 to 11 entries a row) and one offset pair
+# so far that a block's window reaches beyond its neighbours: 30,000 FP32 rows
+# on 16 blocks of 1,888 (halo 4,500), 15,000 FP64 rows on 16 of 960 (2,250).
+@pytest.mark.parametrize("mixed,n,offs", [
+    (True, 600, (1,)), (False, 600, (1,)), (True, 5000, (1, 45)), (False, 5000, (1, 7, 60)), (True, 9000, (1, 2, 3, 50)),
+    (False, 4000, (1, 2, 9, 30, 77)), (True, 30000, (1, 4500)), (False, 15000, (1, 2250))])
+def test_cluster_systems_of_other_offset_sets(plat, mixed, n, offs):
+    s = P.offsets_spd(n, offs, 23)
+    got = []
+    try:
+        for onchip in (True, False):
+            plat.set_onchip(onchip)
+            B = Batch(1, mixed=mixed, precond=True, rtol=1e-9, platform=plat)
+            sl = B.add(s.rowptr, s.col, s.val, s.b)
+            assert B.form(sl) == (FORM_CLUSTER if onchip else FORM_KERNELS)
+            B.solve()
+            r = B.result(sl)
+            assert r.solver_state == lmp.kSolverSuccess
+            # FP64 mode ends on the recurrence's residual, within rounding of the true one
+            assert _true_rel_res(s, r.x) < 1.01e-9
+            got.append(r)
+            B.close()
+    finally:
+        plat.set_onchip(True)
+    assert abs(got[0].iters - got[1].iters) <= max(2, 0.05 * got[1].iters), [g.iters for g in got]
 
+
+def test_cluster_form_refuses_unsymmetric_values(plat):
+    """An entry that differs from its mirror keeps a system on the pass
+    kernels.  The halved storage would take the one for the other: the two
+    symmetric matrices it could mean have other solutions than this one."""
+    s = P.q1_system(2, 20, 9, 0.5, "unsym")
+    at = int(s.rowptr[s.n // 2])
+    other = int(s.col[at])
+    mirror = int(s.rowptr[other] + np.flatnonzero(s.col[s.rowptr[other]:s.rowptr[other + 1]] == s.n // 2)[0])
+    vals = {k: s.val.copy() for k in ("unsym", "both", "last bit")}
+    vals["unsym"][at] *= 1.0 + 1e-3
+    vals["both"][[at, mirror]] *= 1.0 + 1e-3
+    vals["last bit"][at] = np.nextafter(vals["last bit"][at], 0.0)
+    ref = {k: oracle.cg(s.rowptr, s.col, v, s.b, maxits=10000, atol=0.0, rtol=1e-13).x for k, v in vals.items()}
+    ref["none"] = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=10000, atol=0.0, rtol=1e-13).x
+    B = Batch(3, mixed=False, precond=True, rtol=1e-12, platform=plat)
+    slots = {k: B.add(s.rowptr, s.col, v, s.b) for k, v in vals.items()}
+    B.solve()
+    rel = lambda a, b: np.linalg.norm(a - b) / np.linalg.norm(b)  # noqa: E731
+    for k, sl in slots.items():
+        assert B.form(sl) == (FORM_CLUSTER if k == "both" else FORM_KERNELS), k
+        r = B.result(sl)
+        assert r.solver_state == lmp.kSolverSuccess
+        # residuals at 1e-12 ||b||, the matrix's condition below 1e3
+        assert rel(r.x, ref[k]) <= 1e-9, k
+    assert min(rel(ref["unsym"], ref["both"]), rel(ref["unsym"], ref["none"])) > 1e-7
+    B.close()
 
 def test_latency_counts_the_wait_for_sms(plat):
     """device_us runs from the start of the solve: of many equal systems more

@@ -15,7 +15,8 @@ import pytest
 import oracle
 from ba_b200 import lmp
 from ba_b200 import problems as P
-from ba_b200._lib import FMT_CSR, FMT_SELL, FMT_SELL16, FMT_STENCIL, B200LAError, call
+from ba_b200._lib import (FMT_CSR, FMT_SELL, FMT_SELL16, FMT_STENCIL, FORM_CLUSTER, FORM_KERNELS, FORM_RESIDENT,
+                          B200LAError, call)
 
 pytestmark = pytest.mark.gpu
 
@@ -32,6 +33,14 @@ SPMV_RTOL_F32 = 1e-5
 @pytest.fixture(scope="module")
 def plat():
     return lmp.init_platform(0)
+
+
+@pytest.fixture(scope="module")
+def streamed():
+    """A context that keeps to the streamed kernels."""
+    pf = lmp.Platform(0)
+    pf.set_onchip(False)
+    return pf
 
 
 def _mat(plat, s, dtype=np.float64):
@@ -541,25 +550,28 @@ def test_stencil_copy_gives_the_sell_bits(plat, dtype):
                                    rtol=1e-5 if dtype == np.float32 else 1e-13, atol=1e-6)
 
 
-def test_stencil_copy_in_the_solvers(plat):
+def test_stencil_copy_in_the_solvers(plat, streamed):
     """CG on the values-only copy takes the SELL16 path's iterations and
-    solution bits (3D Q1, FP64, Jacobi); ZeroRows rebuilds the copy with the
+    solution bits (3D Q1, FP64, Jacobi, in the graph of three kernels, where
+    the schedules differ, and again off the switch); ZeroRows rebuilds the copy with the
     new values; the tuner may pick it on a Q1 matrix and CG then matches the
     oracle."""
     s = P.q1_system(3, 14, 11, 1.0)
-    b = _vec(plat, s.b)
-    out = []
-    for fmt, w in ((FMT_SELL16, 1), (FMT_STENCIL, 1), (FMT_STENCIL, 4)):
-        A = _mat(plat, s)
-        A.set_format(fmt, w)
-        x = _vec(plat, np.zeros(s.n))
-        solver = lmp.setup_CG_solver(maxits=5000, atol=0.0, rtol=1e-10, dtol=1e8)
-        solver.SetupOperator(A)
-        assert solver.Solve(b, x) == lmp.kSolverSuccess
-        out.append((solver.iter(), x.numpy()))
-    for it, xs in out[1:]:
-        assert it == out[0][0]
-        np.testing.assert_array_equal(xs, out[0][1])
+    for pf, form in ((plat, FORM_CLUSTER), (streamed, FORM_KERNELS)):
+        b = _vec(pf, s.b)
+        out = []
+        for fmt, w in ((FMT_SELL16, 1), (FMT_STENCIL, 1), (FMT_STENCIL, 4)):
+            A = _mat(pf, s)
+            A.set_format(fmt, w)
+            x = _vec(pf, np.zeros(s.n))
+            solver = lmp.setup_CG_solver(maxits=5000, atol=0.0, rtol=1e-10, dtol=1e8)
+            solver.SetupOperator(A)
+            assert solver.Solve(b, x) == lmp.kSolverSuccess
+            assert solver.form() == form
+            out.append((solver.iter(), x.numpy()))
+        for it, xs in out[1:]:
+            assert it == out[0][0]
+            np.testing.assert_array_equal(xs, out[0][1])
     ref = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=5000, atol=0.0, rtol=1e-10, precond=True)
     assert abs(out[0][0] - ref.iters) <= 1
     # ZeroRows on the values-only schedule: the copy follows the new values
@@ -594,15 +606,17 @@ def test_stencil_copy_in_the_solvers(plat):
 
 # Sizes where the on-chip CG forms change hands or a block's rows end: one
 # block up to 512 rows (22^2 cells: 529), 8 blocks up to 6,000 (76^2: 5,929;
-# 77^2: 6,084), 16 blocks up to 9 rows a thread (256^2 fits, 260^2 does not),
-# halos wider than a block's rows (3D), the smallest stencils, then the
-# resident form on sliced copies and its limits.
-@pytest.mark.parametrize("dim,cells,fmt", [
-    (2, 2, None), (2, 3, None), (2, 21, None), (2, 22, None), (2, 76, None), (2, 77, None), (2, 131, None),
-    (2, 256, None), (3, 2, None), (3, 4, None), (3, 11, None), (3, 25, None), (3, 29, (FMT_STENCIL, 1)),
-    (2, 260, (FMT_STENCIL, 1)), (2, 268, (FMT_SELL16, 2)), (3, 41, (FMT_SELL, 1))])
+# 77^2: 6,084), 16 blocks up to 9 rows a thread (256^2 and 24^3 fit, 260^2 and
+# 25^3 do not), the smallest stencils, then the resident form on sliced copies
+# and its limits, and systems that no on-chip form takes.
+@pytest.mark.parametrize("dim,cells,fmt,form", [
+    (2, 2, None, FORM_CLUSTER), (2, 3, None, FORM_CLUSTER), (2, 21, None, FORM_CLUSTER), (2, 22, None, FORM_CLUSTER),
+    (2, 76, None, FORM_CLUSTER), (2, 77, None, FORM_CLUSTER), (2, 131, None, FORM_CLUSTER),
+    (2, 256, None, FORM_CLUSTER), (3, 2, None, FORM_CLUSTER), (3, 4, None, FORM_CLUSTER), (3, 11, None, FORM_CLUSTER),
+    (3, 24, None, FORM_CLUSTER), (3, 25, None, FORM_KERNELS), (3, 29, (FMT_STENCIL, 1), FORM_RESIDENT), (2, 260, (FMT_STENCIL, 1), FORM_RESIDENT),
+    (2, 268, (FMT_SELL16, 2), FORM_RESIDENT), (3, 41, (FMT_SELL, 1), FORM_RESIDENT), (2, 260, None, FORM_KERNELS)])
 @pytest.mark.parametrize("precond", [True, False])
-def test_cg_on_chip_forms_match_oracle(plat, dim, cells, fmt, precond):
+def test_cg_on_chip_forms_match_oracle(plat, dim, cells, fmt, form, precond):
     s = P.q1_system(dim, cells, 70 + cells, 0.5, "onchip")
     A = _mat(plat, s)
     if fmt:
@@ -616,6 +630,7 @@ def test_cg_on_chip_forms_match_oracle(plat, dim, cells, fmt, precond):
     solver = lmp.setup_CG_solver(maxits=steps, atol=0.0, rtol=1e-10, dtol=1e8, use_precond=precond)
     solver.SetupOperator(A)
     solver.Solve(b, x)
+    assert solver.form() == form
     ref = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=steps, atol=0.0, rtol=1e-10, precond=precond)
     assert abs(solver.iter() - ref.iters) <= 1
     if solver.iter() == ref.iters:
@@ -627,6 +642,29 @@ def test_cg_on_chip_forms_match_oracle(plat, dim, cells, fmt, precond):
         assert solver.Solve(b, x2) == lmp.kSolverSuccess
         full = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=20000, atol=0.0, rtol=1e-12, precond=precond)
         assert np.linalg.norm(x2.numpy() - full.x) <= 1e-9 * np.linalg.norm(full.x)
+
+
+# Offset sets other than a grid's: 3, 5, 7, 9 and 11 entries a row, and one
+# offset pair so far that a block's window reaches beyond its neighbours
+# (2,000 rows on 8 blocks of 256: halo 900; 15,000 on 16 of 960: halo 2,250).
+OFFSET_SETS = [(600, (1,)), (2000, (1, 45)), (3001, (1, 7, 60)), (2500, (1, 2, 3, 50)), (4000, (1, 2, 9, 30, 77)),
+               (2000, (1, 900)), (2000, (1, 2, 3, 850)), (15000, (1, 2250))]
+
+
+@pytest.mark.parametrize("n,offs", OFFSET_SETS)
+@pytest.mark.parametrize("precond", [True, False])
+def test_cg_cluster_form_on_other_offset_sets(plat, n, offs, precond):
+    s = P.offsets_spd(n, offs, 17)
+    A = _mat(plat, s)
+    b, x = _vec(plat, s.b), _vec(plat, np.zeros(s.n))
+    solver = lmp.setup_CG_solver(maxits=40, atol=0.0, rtol=1e-14, dtol=1e8, use_precond=precond)
+    solver.SetupOperator(A)
+    solver.Solve(b, x)
+    assert solver.form() == FORM_CLUSTER
+    ref = oracle.cg(s.rowptr, s.col, s.val, s.b, maxits=solver.iter(), atol=0.0, rtol=1e-30, precond=precond)
+    # k steps of n-term sums, n eps relative each at worst, as above
+    tol = 40 * n * np.finfo(np.float64).eps
+    assert np.linalg.norm(x.numpy() - ref.x) <= max(1e-10, tol) * np.linalg.norm(ref.x)
 
 
 def test_cg_on_chip_form_refuses_what_it_cannot_hold(plat):
@@ -645,6 +683,7 @@ def test_cg_on_chip_form_refuses_what_it_cannot_hold(plat):
         solver = lmp.setup_CG_solver(maxits=15, atol=0.0, rtol=1e-14, dtol=1e8)
         solver.SetupOperator(A)
         solver.Solve(_vec(plat, b), x)
+        assert solver.form() == FORM_KERNELS
         ref = oracle.cg(rp, cl, vv, b, maxits=15, atol=0.0, rtol=1e-14)
         assert np.linalg.norm(x.numpy() - ref.x) <= 1e-10 * np.linalg.norm(ref.x)
     A = _mat(plat, s)
@@ -660,6 +699,7 @@ def test_cg_on_chip_form_refuses_what_it_cannot_hold(plat):
         val[seg] = np.where(s.col[seg] == r, 2.0, 0.0)
     x = _vec(plat, np.zeros(s.n))
     solver.Solve(_vec(plat, s.b), x)
+    assert solver.form() == FORM_CLUSTER
     ref = oracle.cg(s.rowptr, s.col, val, s.b, maxits=solver.iter(), atol=0.0, rtol=1e-30, precond=False)
     assert np.linalg.norm(x.numpy() - ref.x) <= 1e-8 * np.linalg.norm(ref.x)
 
