@@ -33,7 +33,7 @@ namespace b200la {
 
 // First bad triplet (smallest index), or all ones when every index is in
 // range; place[i] = how many entries of its row were counted before entry i.
-// Two entries in flight per thread.
+// Four entries in flight per thread.
 __global__ void __launch_bounds__(kBlock) coo_count_kernel(int64_t nnz, int nrow, int ncol,
                                                            const int *__restrict__ rows,
                                                            const int *__restrict__ cols, int *__restrict__ count,
@@ -171,27 +171,43 @@ __global__ void __launch_bounds__(kBlock) coo_scatter_kernel(int64_t nnz, const 
 // col[b, e) / val[b, e) in place, then the first diagonal entry.
 template <typename T>
 __device__ void row_selection_sort(int k, int b, int e, int *col, T *val, int *diag) {
+  const int lane = threadIdx.x & 31;
   for (int i = b; i != e; ++i) {
-    int mi = i, mc = col[i];
-    for (int j = i + 1; j < e; ++j)
+    // the first of the smallest columns (columns are < ncol <= INT_MAX)
+    int mi = INT_MAX, mc = INT_MAX;
+    for (int j = i + lane; j < e; j += 32)
       if (col[j] < mc) {
         mi = j;
         mc = col[j];
       }
-    const int tc = col[i];
-    col[i] = col[mi];
-    col[mi] = tc;
-    const T tv = val[i];
-    val[i] = val[mi];
-    val[mi] = tv;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const int oi = __shfl_xor_sync(0xffffffffu, mi, o), oc = __shfl_xor_sync(0xffffffffu, mc, o);
+      if (oc < mc || (oc == mc && oi < mi)) {
+        mi = oi;
+        mc = oc;
+      }
+    }
+    if (lane == 0) {
+      const int tc = col[i];
+      col[i] = col[mi];
+      col[mi] = tc;
+      const T tv = val[i];
+      val[i] = val[mi];
+      val[mi] = tv;
+    }
+    __syncwarp();
   }
-  int d = -1;
-  for (int i = b; i != e; ++i)
+  int d = INT_MAX;
+  for (int i = b + lane; i < e; i += 32)
     if (col[i] == k) {
       d = i;
       break;
     }
-  diag[k] = d;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) d = min(d, __shfl_xor_sync(0xffffffffu, d, o));
+  if (lane == 0) diag[k] = d == INT_MAX ? -1 : d;
+  __syncwarp();
 }
 
 // Row sort, one warp per row of up to 32 entries (lane l holds one of them).
@@ -199,8 +215,8 @@ __device__ void row_selection_sort(int k, int b, int e, int *col, T *val, int *d
 // goes straight to b + (number of smaller columns), ranks taken with shuffles;
 // that equals the reference's selection sort.  A row with a repeated column
 // (found by __match_any_sync) is first put in input order, then sorted by the
-// selection sort itself (lane 0), because there the order of equal columns
-// depends on its swaps.  Longer rows are appended to a worklist for
+// selection sort itself, because there the order of equal columns depends on
+// its swaps.  Longer rows are appended to a worklist for
 // coo_long_rows_kernel.  Also the diagonal positions and the longest row.
 template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int *__restrict__ rowptr,
@@ -234,8 +250,7 @@ __global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int
         val[b + r] = v;
       }
       __syncwarp();
-      if (lane == 0) row_selection_sort(k, b, e, col, val, diag);
-      __syncwarp();
+      row_selection_sort(k, b, e, col, val, diag);
       continue;
     }
     int r = 0;
@@ -256,11 +271,43 @@ __global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int
 }
 
 // Rows longer than 32 entries (from coo_rowsort_kernel's worklist), one warp
-// per row: the entries go to col / val in input order first (each lane counts
-// the smaller positions of its entries); then lane l holds entries l, l + 32,
-// ... (up to kMaxQ * 32 = 256) and the ranks come from shuffles as above; a
-// repeated column or a longer row takes the selection sort (lane 0).
+// per row: lane l holds entries l, l + 32, ... (up to kMaxQ * 32 = 256) and the
+// ranks come from shuffles as above.  A repeated column or a longer row takes
+// the selection sort, after its entries were put in input order; only those
+// rows pay for the ranks of the positions.  Measured, us for the conversion of
+// shuffled triplets (every row's positions ranked and the selection sort on one
+// lane in brackets): 100,000 rows of 100 entries 1,465 (1,641), 40,000 of 256
+// 1,492 (1,820), 20,000 of 300 1,925 (5,490).
 constexpr int kMaxQ = 8;
+
+// Row b .. e of the pairs to col / val in input order: lane l ranks kMaxQ of
+// its entries per pass over the row's positions.
+template <typename T, typename S>
+__device__ __forceinline__ void row_in_input_order(int b, int e, const unsigned long long *__restrict__ packed,
+                                                   const S *__restrict__ vals, int *col, T *val) {
+  const int lane = threadIdx.x & 31, L = e - b;
+  for (int i0 = lane; i0 < L; i0 += 32 * kMaxQ) {
+    unsigned long long own[kMaxQ];
+    int rank[kMaxQ];
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q) {
+      own[q] = i0 + q * 32 < L ? packed[b + i0 + q * 32] : 0ull;
+      rank[q] = 0;
+    }
+    for (int t = 0; t < L; ++t) {
+      const unsigned pos = (unsigned)packed[b + t];
+#pragma unroll
+      for (int q = 0; q < kMaxQ; ++q) rank[q] += pos < (unsigned)own[q] ? 1 : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q)
+      if (i0 + q * 32 < L) {
+        col[b + rank[q]] = (int)(own[q] >> 32);
+        val[b + rank[q]] = (T)vals[(unsigned)own[q]];
+      }
+  }
+  __syncwarp();
+}
 
 template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__restrict__ rowptr,
@@ -275,18 +322,9 @@ __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__rest
   for (int64_t w = warp; w < count; w += nwarps) {
     const int k = long_rows[w];
     const int b = rowptr[k], e = rowptr[k + 1], L = e - b;
-    for (int i = lane; i < L; i += 32) {
-      const unsigned long long q = packed[b + i];
-      const unsigned pos = (unsigned)q;
-      int r = 0;
-      for (int t = 0; t < L; ++t) r += (unsigned)packed[b + t] < pos ? 1 : 0;
-      col[b + r] = (int)(q >> 32);
-      val[b + r] = (T)vals[pos];
-    }
-    __syncwarp();
     if (L > kMaxQ * 32) {
-      if (lane == 0) row_selection_sort(k, b, e, col, val, diag);
-      __syncwarp();
+      row_in_input_order<T, S>(b, e, packed, vals, col, val);
+      row_selection_sort(k, b, e, col, val, diag);
       continue;
     }
     const int nq = (L + 31) >> 5;
@@ -296,8 +334,9 @@ __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__rest
     for (int q = 0; q < kMaxQ; ++q) {
       const int i = q * 32 + lane;
       const bool ok = q < nq && i < L;
-      c[q] = ok ? col[b + i] : INT_MAX;
-      v[q] = ok ? val[b + i] : T(0);
+      const unsigned long long own = ok ? packed[b + i] : 0ull;
+      c[q] = ok ? (int)(own >> 32) : INT_MAX;
+      v[q] = ok ? (T)vals[(unsigned)own] : T(0);
       rank[q] = 0;
     }
     bool dup = false;
@@ -316,12 +355,10 @@ __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__rest
       }
     }
     if (__any_sync(0xffffffffu, dup)) {
-      __syncwarp();
-      if (lane == 0) row_selection_sort(k, b, e, col, val, diag);
-      __syncwarp();
+      row_in_input_order<T, S>(b, e, packed, vals, col, val);
+      row_selection_sort(k, b, e, col, val, diag);
       continue;
     }
-    __syncwarp();
     int d = INT_MAX;
 #pragma unroll
     for (int q = 0; q < kMaxQ; ++q) {
