@@ -395,14 +395,27 @@ __global__ void __launch_bounds__(kBlock) gm_arnoldi_kernel(GmBufs<T> v, const d
 // products V_i.V_k of earlier steps are kept in G, row j's come with this
 // step's dots), so one pass gives every V_i.w and V_j.V_i, every block solves
 // the same small system, and a second pass forms w - sum h_i V_i and its norm.
-//   dots    warp q takes basis vectors q, q + 32, ...: a lane adds its chunks
-//           of the slice, one shuffle tree a vector, one partial a block
+//   dots    tasks of one basis vector and one part of the slice, a warp each,
+//           round robin: a lane adds its chunks, one shuffle tree a task, the
+//           parts of a vector in order, one partial a block.  A vector is cut
+//           into parts while they fit the tasks' slots: with one warp a vector
+//           a step of few vectors waits for few warps.  us a step, one warp a
+//           vector and now (one barrier a projection in brackets): 4 steps of
+//           64^3 59 55 (62), 128^3 248 165 (199), 158^3 424 277 (343); 100
+//           steps of 64^3 100 90 (237), 128^3 468 401 (483), 158^3 934 881
+//           (861).  Taken back: four times the slots (64^3 92, 158^3 908), the
+//           update by groups of vectors instead of by chunks (158^3 980),
+//           eight vectors of the update in flight (128^3 385, but 158^3 931)
 //   solve   h = a - L h repeated until no bit changes: L is strictly lower
 //           triangular, so this is exact after at most j + 1 rounds, and two
 //           or three do when the basis is orthogonal to rounding
 //   update  thread t owns chunks t + q kResBlock of the slice
 constexpr int kResBlock = 1024;
 constexpr int kResUnroll = 2;
+// Tasks of the dots at most (their sums share the small arrays' memory), and
+// the 16-byte chunks a task has at least: two loads a lane.
+__host__ __device__ constexpr int gm_res_tasks(int m) { return 2 * (m + 1) > 128 ? 2 * (m + 1) : 128; }
+constexpr int kResTaskChunks = 64;
 
 // The end of one projection in the resident kernel: the block's partial
 // (the threads' v summed) goes to set[blockIdx.x]; after the grid barrier
@@ -471,7 +484,7 @@ __global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> 
   const int m = __ldg(&sc->m), ldh = m + 1;
   // shared memory: V_i.w, V_j.V_i and two rounds of h, then the slices
   double *ash = reinterpret_cast<double *>(gm_dyn), *gsh = ash + ldh, *hsh[2] = {gsh + ldh, gsh + 2 * ldh};
-  T *ws = reinterpret_cast<T *>(gsh + 3 * ldh);
+  T *ws = reinterpret_cast<T *>(ash + 2 * gm_res_tasks(m));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = kResBlock / 32;
   const int64_t lo = (int64_t)blockIdx.x * S;
@@ -504,23 +517,29 @@ __global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> 
   }
   __syncthreads();
   // dots: part4 holds [2 (m + 1)][gridDim.x], column i = V_i.w, column
-  // m + 1 + i = V_i.V_j
+  // m + 1 + i = V_i.V_j; the tasks' sums lie where the small arrays follow
   const T *vjr = two ? vs : vj;
-  for (int i = warp; i <= j; i += NW) {
+  const int tasks_max = gm_res_tasks(m);
+  double *tw = ash, *tg = ash + tasks_max;
+  int parts = 1;
+  while (parts < NW && (j + 1) * parts * 2 <= tasks_max && nv >= (int64_t)parts * 2 * kResTaskChunks) parts *= 2;
+  for (int t = warp; t < (j + 1) * parts; t += NW) {
+    const int i = t / parts, part = t - i * parts;
+    const int64_t step = 32 * parts;
     const T *vi = v.V + (int64_t)i * v.ldv + lo;
     Acc<T> aw, ag;
     constexpr int UD = 4;
-    for (int64_t k0 = lane; k0 < nv; k0 += UD * 32) {
+    for (int64_t k0 = part * 32 + lane; k0 < nv; k0 += UD * step) {
       T a[UD][W];
 #pragma unroll
       for (int u = 0; u < UD; ++u)
-        if (k0 + u * 32 < nv) ld<W>(vi + (k0 + u * 32) * W, a[u]);
+        if (k0 + u * step < nv) ld<W>(vi + (k0 + u * step) * W, a[u]);
 #pragma unroll
       for (int u = 0; u < UD; ++u)
-        if (k0 + u * 32 < nv) {
+        if (k0 + u * step < nv) {
           T wv[W], gv[W];
-          ld<W>(ws + (k0 + u * 32) * W, wv);
-          ld<W>(vjr + (k0 + u * 32) * W, gv);
+          ld<W>(ws + (k0 + u * step) * W, wv);
+          ld<W>(vjr + (k0 + u * step) * W, gv);
 #pragma unroll
           for (int q = 0; q < W; ++q) {
             aw.add(wv[q] * a[u][q]);
@@ -528,15 +547,26 @@ __global__ void __launch_bounds__(kResBlock, 1) gm_arnoldi_res_kernel(GmBufs<T> 
           }
         }
     }
-    for (int64_t e = nv * W + lane; e < len; e += 32) {
-      aw.add(ws[e] * vi[e]);
-      ag.add(vjr[e] * vi[e]);
-    }
+    if (part == 0)
+      for (int64_t e = nv * W + lane; e < len; e += 32) {
+        aw.add(ws[e] * vi[e]);
+        ag.add(vjr[e] * vi[e]);
+      }
     const double sw = warp_sum(aw.value()), sg = warp_sum(ag.value());
     if (lane == 0) {
-      part4[(int64_t)i * gridDim.x + blockIdx.x] = sw;
-      part4[(int64_t)(ldh + i) * gridDim.x + blockIdx.x] = sg;
+      tw[t] = sw;
+      tg[t] = sg;
     }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i <= j; i += (int)bd) {
+    double sw = 0.0, sg = 0.0;
+    for (int q = 0; q < parts; ++q) {
+      sw += tw[i * parts + q];
+      sg += tg[i * parts + q];
+    }
+    part4[(int64_t)i * gridDim.x + blockIdx.x] = sw;
+    part4[(int64_t)(ldh + i) * gridDim.x + blockIdx.x] = sg;
   }
   if (stall) return;  // test hook: this block never reaches the barrier
   if (!grid_barrier_count(&sc->bar_count, (bar0 + 1ull) * gridDim.x, &sc->err)) {
@@ -696,7 +726,7 @@ template <typename T> static GmBufs<T> gm_bufs(const GmresState *s) {
 }
 
 // Shared memory of the resident step's small arrays (before the slices).
-static size_t gm_res_small(const GmresState *s) { return sizeof(double) * 4 * (size_t)(s->m + 1); }
+static size_t gm_res_small(const GmresState *s) { return sizeof(double) * 2 * (size_t)gm_res_tasks(s->m); }
 
 // The Arnoldi kernel as a cooperative launch (all blocks resident, which its
 // grid barrier needs), captured into the graph like any kernel node.
