@@ -168,9 +168,35 @@ __global__ void __launch_bounds__(kBlock) coo_scatter_kernel(int64_t nnz, const 
 }
 
 // The reference's per-row selection sort (lmatrix_formats.h:405-431) on
-// col[b, e) / val[b, e) in place, then the first diagonal entry.
+// col[b, e) / val[b, e) in place, then the first diagonal entry; one lane.
 template <typename T>
 __device__ void row_selection_sort(int k, int b, int e, int *col, T *val, int *diag) {
+  for (int i = b; i != e; ++i) {
+    int mi = i, mc = col[i];
+    for (int j = i + 1; j < e; ++j)
+      if (col[j] < mc) {
+        mi = j;
+        mc = col[j];
+      }
+    const int tc = col[i];
+    col[i] = col[mi];
+    col[mi] = tc;
+    const T tv = val[i];
+    val[i] = val[mi];
+    val[mi] = tv;
+  }
+  int d = -1;
+  for (int i = b; i != e; ++i)
+    if (col[i] == k) {
+      d = i;
+      break;
+    }
+  diag[k] = d;
+}
+
+// The same by a warp, which looks for each minimum together (long rows).
+template <typename T>
+__device__ void warp_selection_sort(int k, int b, int e, int *col, T *val, int *diag) {
   const int lane = threadIdx.x & 31;
   for (int i = b; i != e; ++i) {
     // the first of the smallest columns (columns are < ncol <= INT_MAX)
@@ -250,7 +276,8 @@ __global__ void __launch_bounds__(kBlock) coo_rowsort_kernel(int nrow, const int
         val[b + r] = v;
       }
       __syncwarp();
-      row_selection_sort(k, b, e, col, val, diag);
+      if (lane == 0) row_selection_sort(k, b, e, col, val, diag);
+      __syncwarp();
       continue;
     }
     int r = 0;
@@ -324,7 +351,7 @@ __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__rest
     const int b = rowptr[k], e = rowptr[k + 1], L = e - b;
     if (L > kMaxQ * 32) {
       row_in_input_order<T, S>(b, e, packed, vals, col, val);
-      row_selection_sort(k, b, e, col, val, diag);
+      warp_selection_sort(k, b, e, col, val, diag);
       continue;
     }
     const int nq = (L + 31) >> 5;
@@ -356,7 +383,7 @@ __global__ void __launch_bounds__(kBlock) coo_long_rows_kernel(const int *__rest
     }
     if (__any_sync(0xffffffffu, dup)) {
       row_in_input_order<T, S>(b, e, packed, vals, col, val);
-      row_selection_sort(k, b, e, col, val, diag);
+      warp_selection_sort(k, b, e, col, val, diag);
       continue;
     }
     int d = INT_MAX;
