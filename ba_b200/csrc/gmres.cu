@@ -7,8 +7,8 @@
 //   G1  at a cycle end: x += P (sum_i y_i V_i) (y from the back substitution
 //       G4 left), one pass over the basis
 //   G2  at a (re)start: V0 = (b - A x) / res, z = P V0, reset H and g
-//   G3  w = A z (z = P V_j, or V_j itself without preconditioner), fused
-//       with the partial sums of w.V_0
+//   G3  w = A z (z = P V_j, or V_j itself without preconditioner), in the
+//       streaming form fused with the partial sums of w.V_0
 //   G4  the rest of the Arnoldi step in one cooperative kernel.  When w
 //       fits in the SMs' shared memory (up to ~4.3 M FP64 rows on 148
 //       SMs): all dots in one pass over the basis, the Gram-Schmidt
@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(kBlock) gm_restart_kernel(Op op, GmBufs<T> v, 
   }
 }
 
-// ---- G3: w = A z, partial sums of w.V0 ---------------------------------------------
+// ---- G3: w = A z, partial sums of w.V0 (the streaming step's first dot; the
+// resident step takes all its dots itself: DOT false) ------------------------
 template <typename T> struct ArnoldiSpmvEmit {
   T *__restrict__ w;
   const T *__restrict__ v0;
@@ -190,12 +191,18 @@ template <typename T> struct ArnoldiSpmvEmit {
   }
 };
 
-template <typename Op, typename T, bool PRE>
+template <typename Op, typename T, bool PRE, bool DOT>
 __global__ void __launch_bounds__(kBlock) gm_spmv_kernel(Op op, GmBufs<T> v, double *part3, GmScalars *sc) {
   if (__ldg(&sc->phase) != kGmStep) return;
   const int j = __ldg(&sc->j);
+  const T *x = PRE ? v.z : v.V + j * v.ldv;
+  if (!DOT) {
+    StoreEmit<T> e{v.w};
+    op.run(x, e);
+    return;
+  }
   ArnoldiSpmvEmit<T> e{v.w, v.V};
-  op.run(PRE ? v.z : v.V + j * v.ldv, e);
+  op.run(x, e);
   double s[1] = {e.acc.value()};
   __shared__ double red[32];
   block_sum<1>(s, red);
@@ -801,6 +808,12 @@ static int gm_size_resident(GmresState *s) {
   return B200LA_OK;
 }
 
+template <typename Op, typename T, bool PRE>
+static void gm_launch_spmv(GmresState *s, const Op &op, const GmBufs<T> &v, cudaStream_t st) {
+  if (s->grid_res > 0) gm_spmv_kernel<Op, T, PRE, false><<<s->grid_spmv, kBlock, 0, st>>>(op, v, s->part3, s->sc);
+  else gm_spmv_kernel<Op, T, PRE, true><<<s->grid_spmv, kBlock, 0, st>>>(op, v, s->part3, s->sc);
+}
+
 template <typename T, bool PRE, bool IN_GRAPH>
 static int gm_body_t(GmresState *s, cudaStream_t st, cudaGraphConditionalHandle h) {
   const GmBufs<T> v = gm_bufs<T>(s);
@@ -808,7 +821,7 @@ static int gm_body_t(GmresState *s, cudaStream_t st, cudaGraphConditionalHandle 
   B_TRY(with_schedule<T>(s->A, [&](auto op) -> int {
     using Op = decltype(op);
     gm_restart_kernel<Op, T, PRE><<<s->grid_restart, kBlock, 0, st>>>(op, v, s->part, s->sc);
-    gm_spmv_kernel<Op, T, PRE><<<s->grid_spmv, kBlock, 0, st>>>(op, v, s->part3, s->sc);
+    gm_launch_spmv<Op, T, PRE>(s, op, v, st);
     return B200LA_OK;
   }));
   return gm_launch_arnoldi<T, PRE, IN_GRAPH>(s, st, h);
@@ -817,6 +830,7 @@ static int gm_body_t(GmresState *s, cudaStream_t st, cudaGraphConditionalHandle 
 template <typename T, bool PRE>
 static int gm_grids_t(GmresState *s) {
   b200la_ctx c = s->A->ctx;
+  B_TRY((gm_size_resident<T, PRE>(s)));  // the form decides which product kernel runs
   B_TRY(grid_for(c, (const void *)gm_update_kernel<T, PRE>, (s->n + Vec16<T>::n - 1) / Vec16<T>::n, kBlock,
                  &s->grid_ew));
   B_TRY(with_schedule<T>(s->A, [&](auto op) -> int {
@@ -824,8 +838,8 @@ static int gm_grids_t(GmresState *s) {
     B_TRY(grid_for(c, (const void *)gm_start_kernel<Op, T>, op.work_items(), Op::kRowsPerBlock, &s->grid_start));
     B_TRY(grid_for(c, (const void *)gm_restart_kernel<Op, T, PRE>, op.work_items(), Op::kRowsPerBlock,
                    &s->grid_restart));
-    B_TRY(grid_for(c, (const void *)gm_spmv_kernel<Op, T, PRE>, op.work_items(), Op::kRowsPerBlock,
-                   &s->grid_spmv));
+    const auto spmv = s->grid_res > 0 ? gm_spmv_kernel<Op, T, PRE, false> : gm_spmv_kernel<Op, T, PRE, true>;
+    B_TRY(grid_for(c, (const void *)spmv, op.work_items(), Op::kRowsPerBlock, &s->grid_spmv));
     return B200LA_OK;
   }));
   // every block of the cooperative kernel must be resident at once
@@ -839,7 +853,7 @@ static int gm_grids_t(GmresState *s) {
   int64_t cap = (int64_t)c->num_sms * per_sm;
   if (cap > kMaxReduceBlocks) cap = kMaxReduceBlocks;
   s->grid_coop = (int)(need < 1 ? 1 : (need < cap ? need : cap));
-  return gm_size_resident<T, PRE>(s);
+  return B200LA_OK;
 }
 
 template <typename T, bool PRE>
@@ -962,7 +976,7 @@ static int gm_profile_t(GmresState *s, const void *b_dev, const void *x_dev, int
       using Op = decltype(op);
       gm_restart_kernel<Op, T, PRE><<<s->grid_restart, kBlock, 0, st>>>(op, v, s->part, s->sc);
       cudaEventRecord(e[2], st);
-      gm_spmv_kernel<Op, T, PRE><<<s->grid_spmv, kBlock, 0, st>>>(op, v, s->part3, s->sc);
+      gm_launch_spmv<Op, T, PRE>(s, op, v, st);
       cudaEventRecord(e[3], st);
       return B200LA_OK;
     });
