@@ -2899,7 +2899,9 @@ int b200la_batch_tune(b200la_batch B, int *rows, double *usec) {
   // tile_rows, each candidate set is timed on real passes over the running
   // systems (each kernel's time depends only on its own item size, so every
   // kernel picks its own best), and every system's carried state (x, c, r,
-  // p and its scalars) is restored after each trial.  Each kernel keeps the
+  // p and its scalars) is restored after each trial.  Systems on clusters
+  // never run in these kernels and take no part; with none left the sizes
+  // stay as they are.  Each kernel keeps the
   // smallest item within 3% of its best time: mid-solve passes, where
   // finished systems and residual passes mix in, favour short items.
   // K1 is held to 128..256 rows and keeps 128 unless 256 is more than 8%
@@ -2909,7 +2911,7 @@ int b200la_batch_tune(b200la_batch B, int *rows, double *usec) {
   // at 256 (1,024-system batch).
   static const int cand[4][3] = {{128, 256, 256}, {256, 512, 512}, {256, 1024, 1024}, {256, 2048, 2048}};
   int active = 0;
-  B_TRY(upload_tiles(B, true, &active, nullptr));
+  B_TRY(upload_tiles(B, true, &active, nullptr, true));
   double best_ms = 0.0;
   if (active) {
     const bool pre = B->kp.precond != 0;
@@ -2924,7 +2926,7 @@ int b200la_batch_tune(b200la_batch B, int *rows, double *usec) {
       double t[4][3];
       for (int c = 0; c < 4 && rc == B200LA_OK; ++c) {
         for (int k = 0; k < 3; ++k) B->lst[k].rows = cand[c][k];
-        rc = upload_tiles(B, true, &active, nullptr);
+        rc = upload_tiles(B, true, &active, nullptr, true);
         if (rc == B200LA_OK) rc = trial(t[c]);
         if (rc == B200LA_OK) rc = snapshot_restore(B, snap);
       }
@@ -2942,7 +2944,7 @@ int b200la_batch_tune(b200la_batch B, int *rows, double *usec) {
           B->lst[k].rows = cand[best][k];
           best_ms += t[best][k];
         }
-        rc = upload_tiles(B, true, &active, nullptr);
+        rc = upload_tiles(B, true, &active, nullptr, true);
       }
     } else {
       double k[3] = {0, 0, 0};

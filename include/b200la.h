@@ -561,8 +561,9 @@ int b200la_batch_get_items(b200la_batch b, int *rows /* [3] */);
 /* Autotuner: unless the batch was created with a fixed tile_rows, times
  * candidate item sizes (K1 128..256, K2/K3 256..2048 rows) on real passes
  * over the running systems, whose carried state is restored after every
- * trial, and keeps each kernel's fastest.  Writes the three item sizes and
- * the pass time (microseconds, K1 + K2 + K3). */
+ * trial, and keeps each kernel's fastest.  Systems on clusters take no part.
+ * Writes the three item sizes and the pass time (microseconds, K1 + K2 + K3;
+ * 0 when no running system uses these kernels). */
 int b200la_batch_tune(b200la_batch b, int *rows /* [3] */, double *usec);
 /* Instrumentation: mean milliseconds of the inner solve's batched SpMV over
  * every slot (reps launches, CUDA events) and its algorithmic bytes:

@@ -687,3 +687,26 @@ def test_systems_whose_cluster_cannot_be_placed_use_the_pass_kernels(plat, monke
             assert r.solver_state == lmp.kSolverSuccess, (cap, s.name, r)
             assert _true_rel_res(s, r.x) < (1.001e-9 if mixed else 2e-9), (cap, s.name)
         B.close()
+
+
+def test_tune_times_what_the_pass_kernels_run(plat):
+    """tune() leaves out the systems on clusters: with nothing else it times
+    nothing and keeps the item sizes, with a system of the pass kernels it
+    picks among its candidates."""
+    s = P.q1_system(2, 40, 2, 1.0, "tune")
+    B = Batch(2, mixed=True, precond=True, rtol=1e-8, platform=plat)
+    a = B.add(s.rowptr, s.col, s.val, s.b)
+    before = B.items()
+    assert B.form(a) == FORM_CLUSTER and B.tune() == (before, 0.0)
+    val = s.val.copy()
+    val[s.rowptr[s.n // 2]] *= 1.0 + 1e-3
+    b = B.add(s.rowptr, s.col, val, s.b)
+    assert B.form(b) == FORM_KERNELS
+    rows, us = B.tune()
+    assert us > 0.0 and rows[0] in (128, 256) and rows[1] in (256, 512, 1024, 2048)
+    B.solve()
+    for v, sl in ((s.val, a), (val, b)):
+        r = B.result(sl)
+        assert r.solver_state == lmp.kSolverSuccess
+        assert np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, v, r.x)) < 1.001e-8 * np.linalg.norm(s.b)
+    B.close()
