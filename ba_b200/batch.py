@@ -231,6 +231,12 @@ class Batch:
         call("b200la_batch_last_run", self.handle, C.byref(n), None)
         return n.value
 
+    def launches(self) -> int:
+        """Kernels that runs and restarts have launched since the batch was created."""
+        d = C.c_double()
+        call("b200la_batch_last_run", self.handle, None, C.byref(d))
+        return int(d.value)
+
     def restart(self):
         """Restart every system from x = 0 (matrices and right-hand sides stay resident)."""
         call("b200la_batch_restart", self.handle)

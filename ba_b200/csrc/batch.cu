@@ -1446,6 +1446,7 @@ struct b200la_batch_s {
   int *cl_list;                // device [capacity]
   std::vector<int> cl_slots;   // slots of the last launch, as listed
   int list_passes;             // passes of the pass kernels in the last run
+  int64_t launched;            // kernels launched by runs and restarts
   cudaStream_t cl_stream[4];
   cudaEvent_t cl_event[5];
   // kernel instances prepared (cl_prepare): 1 can be placed, -1 not
@@ -1848,8 +1849,10 @@ int host_loop_t(BatchHandle B) {
   int grids[3] = {1, 1, 1};
   B_TRY((pass_grids<T, PRE, false>(B, grids)));
   batch_start_kernel<<<1, 1, 0, st>>>(B->glob);
+  B->launched += 1;
   for (;;) {
     for (int k = 0; k < 8; ++k) launch_pass<T, PRE, false>(B, grids, st, 0);
+    B->launched += 3 * 8;
     B_CUDA(cudaGetLastError());
     B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
     B_CUDA(cudaStreamSynchronize(st));
@@ -2001,6 +2004,7 @@ template <typename T> int launch_clusters_t(BatchHandle B, int budget) {
   B_CUDA(cudaStreamSynchronize(st));  // the list is rebuilt on the host for the next launch
   cluster_begin_kernel<<<((int)sl.size() + kBlock - 1) / kBlock, kBlock, 0, st>>>(B->cl_list, (int)sl.size(), B->st);
   B_CUDA(cudaGetLastError());
+  B->launched += 1;
   B_CUDA(cudaEventRecord(B->cl_event[4], st));
   SideStreams side{B};
   int turn = 0;
@@ -2023,6 +2027,7 @@ template <typename T> int launch_clusters_t(BatchHandle B, int budget) {
       const cudaLaunchConfig_t cfg = cl_config(h.cl_blocks, smem, B->cl_stream[q], attr, (int)(e - a));
       B_CUDA(cudaLaunchKernelEx(&cfg, k, (const int *)(B->cl_list + a), (const SysDesc<T> *)B->desc, B->st, B->kp,
                                 budget));
+      B->launched += 1;
       return B200LA_OK;
     })));
     a = e;
@@ -2040,6 +2045,7 @@ int launch_clusters(BatchHandle B, int budget) {
 void count_clusters(BatchHandle B) {
   BatchGlobals &g = *B->glob_host;
   B->list_passes = g.passes;
+  if (B->ctx->use_graphs && g.passes > 0) B->launched += 1 + 3 * (int64_t)g.passes;  // the graph's
   for (int s : B->cl_slots) {
     g.passes = std::max(g.passes, B->st_host[s].cl_passes);
     if (B->st_host[s].phase != PH_DONE) g.active += 1;
@@ -2747,10 +2753,10 @@ int b200la_batch_solve(b200la_batch B, int chunk_passes, int *total_passes) {
   return B200LA_OK;
 }
 
-int b200la_batch_last_run(b200la_batch B, int *passes, double *reserved) {
+int b200la_batch_last_run(b200la_batch B, int *passes, double *launches) {
   B_CHECK(B, B200LA_ERR_INVALID, "batch_last_run: null batch");
   if (passes) *passes = B->glob_host->passes;
-  if (reserved) *reserved = 0.0;
+  if (launches) *launches = (double)B->launched;
   return B200LA_OK;
 }
 
@@ -2858,6 +2864,7 @@ int b200la_batch_restart(b200la_batch B) {
     batch_restart_kernel<double><<<(int)slots.size(), kBlock, 0, st>>>(d_slots, (const SysDesc<double> *)B->desc,
                                                                         B->st);
   B_CUDA(cudaGetLastError());
+  B->launched += 1;
   B_CUDA(cudaFreeAsync(d_slots, st));
   B_CUDA(cudaStreamSynchronize(st));
   for (int s : slots) {

@@ -330,6 +330,7 @@ def _pinned(a, torch):
 
 def run_batch(args, rank, local_rank, world, torch, dist, barrier):
     from ba_b200 import lmp
+    from ba_b200._lib import FORM_CLUSTER
     from ba_b200.batch import Batch
 
     plat = lmp.Platform(local_rank)
@@ -365,12 +366,14 @@ def run_batch(args, rank, local_rank, world, torch, dist, barrier):
     barrier()
     clocks.start()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    launched = B.launches()
     e0.record(stream)
     passes_tot = 0
     for _ in range(args.steps):
         passes_tot += step()
     e1.record(stream)
     e1.synchronize()
+    launched = B.launches() - launched
     barrier()
     clk = clocks.stop()
     ms_max = D.max_over_ranks(e0.elapsed_time(e1))
@@ -467,14 +470,19 @@ def run_batch(args, rank, local_rank, world, torch, dist, barrier):
     e2e_value = k_e2e * solved_per_step / (D.max_over_ranks(h0.elapsed_time(h1)) / 1e3)
     E.close()
 
-    # roofline of the dominant kernel: K1 of the inner solve (batched FP32
-    # sliced-ELL SpMV fused with p.Ap), timed launch by launch with CUDA
-    # events on the solve stream over a full inner pass of every system
+    # roofline of the timed step: batch_cluster_kernel iterates on chip, so what
+    # it moves is shared memory: a row and inner iteration reads the values
+    # and the direction at its offsets (one word each) and reads and writes
+    # its own direction (nine-point rows: 20 words)
+    on_chip = [B.form(k) == FORM_CLUSTER for k in range(len(systems))]
+    smem_bytes = sum(4.0 * (2 * 9 + 2) * s.n * r.iters for s, r, c in zip(systems, res, on_chip) if c)
+    smem_gbs = smem_bytes / (ms_max / args.steps / 1e3) / 1e9
+    smem_peak = plat.num_sms * 128.0 * (clk["sm_mhz"] or 1965.0) / 1e3
+    # and, for systems that no cluster holds, the pass kernels launch by launch
+    # over an inner pass of every system (the timed step does not run them
+    # where all systems are on clusters)
     B.profile_pass(5)  # warms the GPU up after the host-bound e2e loop
     pass_ms, pass_bytes = B.profile_pass(5)
-    spmv_ms, spmv_bytes_alg = pass_ms[0], pass_bytes[0]
-    peak, peak_kind = measured_peak_gbs()
-    achieved = spmv_bytes_alg / (spmv_ms / 1e3) / 1e9
     kernels = {name: {"ms": t, "algorithmic_bytes": b, "gbs": b / (t / 1e3) / 1e9}
                for name, t, b in zip(("K1_spmv_pAp", "K2_update", "K3_direction"), pass_ms, pass_bytes)}
 
@@ -498,13 +506,18 @@ def run_batch(args, rank, local_rank, world, torch, dist, barrier):
                 "parallelism": (f"split x{world}: one batch partitioned over the ranks by nnz (greedy, largest "
                                 f"first); rank 0 solved {len(systems)} systems") if args.split
                                else f"replicas x{world}: every rank solves its own seeded batch",
-                "precision": f"FP32 Jacobi-PCG inner solves (FP32 matrix values and vectors, compensated FP32 "
-                             f"dots) inside FP64 refinement: the FP64 residual replaces the inner one every "
+                "precision": f"FP32 Jacobi-PCG inner solves (FP32 matrix values and vectors; dots of the FP32 products "
+                             f"summed in FP64 on clusters, compensated FP32 in the pass kernels) inside FP64 refinement: the FP64 residual replaces the inner one every "
                              f"{inner_rtol:g}x reduction, the search direction is kept",
-                "spmv_schedule": ("one thread-block cluster a system, symmetric half of the values and the p window in "
-                                  "shared memory; the profiled pass kernels: sliced ELL, values only"),
+                "spmv_schedule": (f"{sum(on_chip)} of {len(systems)} systems on one thread-block cluster each, symmetric "
+                                  "half of the values and the p window in shared memory; the others by the pass "
+                                  "kernels: sliced ELL, values only"),
+                "pass_kernels": {"note": "each kernel over an inner pass of every system, launch by launch; a system on "
+                                         "a cluster does not run them in the timed step", **kernels,
+                                 "item_rows": {"spmv": item_rows[0], "update": item_rows[1],
+                                               "direction": item_rows[2]}},
                 "p50_latency_ms": float(np.percentile(lat, 50)), "p99_latency_ms": float(np.percentile(lat, 99)),
-                "latency": "per-system device time from its first residual to its finish inside the step",
+                "latency": "per-system device time from the start of the solve to its finish inside the step",
                 "converged": f"{ok}/{len(systems)}", "worst_true_rel_residual_sampled": worst,
                 "error_vs_cpu_oracle": err_oracle,
                 "inner_iters_mean": float(iters.mean()), "inner_iters_max": int(iters.max()),
@@ -519,16 +532,14 @@ def run_batch(args, rank, local_rank, world, torch, dist, barrier):
                                     "speedup_of_mixed_pcg": value / world / pcg_value}},
             "clocks": clk,
             "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-            # a restart and at least one launch of clusters a step (one per group of equal cluster
-            # size); the pass kernels launch only for systems that no cluster holds
-            "gpu_launches": 2 * args.steps,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": profile_traffic("batch1024/f32/spmv"), "peak_source": peak_kind,
-                         "kernel": "batch_spmv_kernel<float> (K1: sliced-ELL SpMV + p.Ap) over an inner pass of "
-                                   "all 1024 systems",
-                         "algorithmic_bytes": spmv_bytes_alg, "kernel_ms": spmv_ms, "pass_kernels": kernels,
-                         "item_rows": {"spmv": item_rows[0], "update": item_rows[1], "direction": item_rows[2]},
-                         **dram_rate(profile_traffic("batch1024/f32/spmv"), spmv_ms, peak)},
+            # a step: the restart, the start stamp, one launch a group of equal clusters, and the
+            # pass kernels for systems that no cluster holds
+            "gpu_launches": launched,
+            "roofline": {"bound": "smem", "achieved": smem_gbs, "peak": smem_peak, "unit": "GB/s",
+                         "frac": smem_gbs / smem_peak, "traffic": None,
+                         "peak_source": "nominal: SMs x 128 B a cycle x the sampled SM clock",
+                         "kernel": "batch_cluster_kernel<float> (whole solves, one cluster a system) over the timed step",
+                         "algorithmic_bytes": smem_bytes, "kernel_ms": ms_max / args.steps},
             "cpu_baseline": cpu,
         }
         print(json.dumps(out))
@@ -1637,9 +1648,9 @@ def run_coo(args, rank, local_rank, world, torch, dist, barrier):
             "gpu_launches": args.steps * 7,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": peak_kind,
-                         "kernel": "whole conversion (check, radix sort by row, row offsets, gather, row sort)",
+                         "kernel": "whole conversion (check and count, prefix sum, scatter, row sort)",
                          "algorithmic_bytes": alg,
-                         "note": "the radix sort moves the keys and positions several times; the algorithmic "
+                         "note": "each entry is scattered and read back as a random 32-byte sector; the algorithmic "
                                  "bytes count one read of the triplets and one write of the CSR"},
             "cpu_baseline": cpu}))
 

@@ -538,8 +538,10 @@ int b200la_batch_set_outputs(b200la_batch b, int count, const int *slots, double
  * passes; between launches the tile list is rebuilt from the systems still
  * running.  Writes the passes taken. */
 int b200la_batch_solve(b200la_batch b, int chunk_passes, int *total_passes);
-/* Body passes (iterations of the device loop) taken by the last run. */
-int b200la_batch_last_run(b200la_batch b, int *passes, double *reserved);
+/* Body passes (iterations of the device loop) taken by the last run, and the
+ * kernels that runs and restarts have launched since the batch was created
+ * (either may be NULL). */
+int b200la_batch_last_run(b200la_batch b, int *passes, double *launches);
 /* Result of a slot (solution copied to x if non-NULL). */
 int b200la_batch_result(b200la_batch b, int slot, double *x, b200la_sys_result *result);
 /* Results of `count` slots at once; x[k] (or x itself) may be NULL.  The
