@@ -1487,10 +1487,10 @@ size_t slot_bytes(int64_t n, int64_t nnz, int64_t ell, bool mixed, bool col16 = 
 // r, Ap, invD and c of each live in registers, 128 a thread, so 17 FP32 or 9
 // FP64 rows at most; 27-point systems run out of shared memory first.
 template <typename T, int H> struct ClRows {
-  static constexpr int n = H > 4 ? 3 : (sizeof(T) == 4 ? 6 : 4);
+  static constexpr int n = H > 4 ? (sizeof(T) == 4 ? 3 : 2) : (sizeof(T) == 4 ? 6 : 4);
   static constexpr int at(int k) {
     constexpr int few[6] = {2, 4, 6, 9, 13, 17};
-    constexpr int wide[3] = {2, 4, sizeof(T) == 4 ? 7 : 5};
+    constexpr int wide[3] = {2, 4, 7};
     return H > 4 ? wide[k] : few[k];
   }
 };
@@ -1552,10 +1552,24 @@ template <typename T> int cl_prepare(BatchHandle B, const HostSys &h, bool *fits
   return B200LA_OK;
 }
 
+constexpr int kClWideMax = 128;
+constexpr size_t kClWideSmem = 196 * 1024 - 1024;  // the carve-out step below the largest, less the block's own 1 KB
+
 // Picks the cluster that holds a system: the smallest one it fits on, since
 // an iteration's two barriers cost the same whatever a block's rows are and
 // other systems fill the rest of the GPU.  A system that fits on none, or only
 // on clusters the device cannot place, stays with the pass kernels.
+// Systems of more than nine entries a row (27-point: 14 values a row on chip)
+// take a cluster only while it is worth its SMs when the GPU is full:
+// blocks x rows a thread x bytes a value up to 128, and no instance of seven
+// rows where the block's memory leaves the L1 28 KB (its spills then go to
+// L2: 18^3 nodes 1.6 ms on two blocks, 0.7 for 19^3 on four).  Measured, ms
+// for 64 and 256 equal 3D systems on clusters / by the pass kernels: FP32,
+// 17^3 nodes 1.1 / 3.0, 4.2 / 6.0 (2 blocks x 7 rows), 21^3 2.4 / 3.4,
+// 9.3 / 9.7 (4 x 7), 25^3 4.9 / 5.9, 17.2 / 16.7 (8 x 4), beyond the line
+// 26^3 6.2 / 6.1, 22.1 / 19.0 and 27^3 10.1 / 7.6, 37.0 / 21.6 (8 x 7); FP64,
+// 19^3 2.0 / 2.4, 6.8 / 6.2 (8 x 2), beyond it 21^3 3.6 / 2.8, 12.6 / 9.0
+// (8 x 4) and 25^3 6.3 / 5.2, 23.4 / 17.5 (16 x 2).
 template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
   h.cl_H = d.cl_H;
   h.cl_blocks = 0;
@@ -1569,6 +1583,8 @@ template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d
     const int held = d.cl_H <= 4 ? cl_rows_for<T, 4>(need) : cl_rows_for<T, kClMaxOff>(need);
     const size_t smem = cl_smem_bytes(rpc, halo, d.cl_H, held, sizeof(T));
     if (held == 0 || smem + 1024 > (size_t)optin) continue;
+    const bool wide = d.cl_H > 4;
+    if (wide && (blocks * held * (int)sizeof(T) > kClWideMax || (held == 7 && smem > kClWideSmem))) continue;
     h.cl_blocks = blocks;
     h.cl_rows = held;
     h.cl_smem = smem;
