@@ -111,7 +111,7 @@ struct SysState {
   double rz, pAp, alpha, beta;
   double res_in, res_in0;      // inner recurrence residual and its start value
   double res, res0;            // FP64 true residual and the initial one
-  unsigned long long t_begin;  // %globaltimer at the system's first residual (on a cluster: at its run's start)
+  unsigned long long t_begin;  // %globaltimer at the system's first residual (where a run has clusters: at its start)
   unsigned long long t_done;   // %globaltimer when the system finished
   int state;                   // B200LA_* iterate state at the end
   unsigned bad_row;            // first row without a usable diagonal (Jacobi), else ~0u
@@ -512,7 +512,7 @@ __device__ __forceinline__ void resid_item(const Tile &tl, int t, const ItemGeo 
     S.res = res;
     if (S.outer == 0) {
       S.res0 = res;
-      S.t_begin = globaltimer();
+      if (S.t_begin == 0) S.t_begin = globaltimer();
     }
     int s = outer_check(res, S.res0, prm);
     if (s == B200LA_ITERATE && S.outer >= prm.max_outer) s = B200LA_FAIL_MAXITS;
@@ -1164,10 +1164,10 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
   }
 }
 
-// The start of the listed systems that have not run yet, as the first pass of
-// the pass kernels records it: a system that waits for the SMs of others has
-// begun.
-__global__ void cluster_begin_kernel(const int *__restrict__ list, int count, SysState *st) {
+// The start of the listed systems that have not run yet (where a run has
+// clusters; else the first pass records it): a system that waits for the SMs
+// of others has begun.
+__global__ void batch_begin_kernel(const int *__restrict__ list, int count, SysState *st) {
   const unsigned long long now = globaltimer();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     SysState &S = st[list[k]];
@@ -1379,6 +1379,7 @@ struct HostSys {
   int cl_H = 0;            // cluster form possible if the values are symmetric (sym_host)
   int cl_blocks = 0, cl_rows = 0;  // blocks of its cluster, rows a thread (0: does not fit)
   size_t cl_smem = 0;
+  bool flying = false;     // its cluster runs on a side stream: state and x are the kernel's
 };
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -1445,7 +1446,8 @@ struct b200la_batch_s {
   int *sym, *sym_host;         // device, pinned host [capacity]
   int *cl_list;                // device [capacity]
   std::vector<int> cl_slots;   // slots of the last launch, as listed
-  int list_passes;             // passes of the pass kernels in the last run
+  std::vector<int> list_slots; // slots of the item lists
+  std::vector<int> all_slots;  // both, as copied to cl_list
   int64_t launched;            // kernels launched by runs and restarts
   cudaStream_t cl_stream[4];
   cudaEvent_t cl_event[5];
@@ -1922,10 +1924,11 @@ int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_byte
   int act = 0;
   int64_t bytes = 0;
   const int64_t vb = B->kp.mixed ? 4 : 8;
-  std::vector<int> run;
+  std::vector<int> &run = B->list_slots;
+  run.clear();
   for (int s = 0; s < B->capacity; ++s) {
     const HostSys &h = B->sys[s];
-    if (!h.used) continue;
+    if (!h.used || h.flying) continue;
     const int ph = B->st_host[s].phase;
     if (running_only && (ph == PH_DONE || ph == PH_EMPTY)) continue;
     if (on_clusters && h.cl_blocks > 0 && B->sym_host[s]) {
@@ -1979,13 +1982,25 @@ int upload_tiles(BatchHandle B, bool running_only, int *count, int64_t *alg_byte
   return B200LA_OK;
 }
 
-// Puts the side streams a launch has used in front of the context stream's
-// later work, on every way out: after an error too, the caller may read the
-// states, run again or destroy the batch.
+// The side streams that carry a launch's clusters beside the pass kernels.
+// join() puts them in front of the context stream's later work; so does every
+// way out: after an error too, the caller may read the states, run again or
+// destroy the batch.
 struct SideStreams {
   BatchHandle B;
-  int used = 0;  // streams 0 .. used - 1 carry clusters
+  int used = 0;            // streams 0 .. used - 1 carry clusters
+  std::vector<int> slots;  // of these systems
+  bool done() const {
+    for (int q = 0; q < used; ++q)
+      if (cudaStreamQuery(B->cl_stream[q]) != cudaSuccess) {
+        cudaGetLastError();  // "not ready" is no error
+        return false;
+      }
+    return true;
+  }
   int join() {
+    for (int s : slots) B->sys[s].flying = false;
+    slots.clear();
     cudaError_t bad = cudaSuccess;
     for (int q = 0; q < used; ++q) {
       cudaError_t e = cudaEventRecord(B->cl_event[q], B->cl_stream[q]);
@@ -1998,31 +2013,45 @@ struct SideStreams {
     return B200LA_OK;
   }
   ~SideStreams() {
-    if (used == 0) return;
+    if (used == 0 && slots.empty()) return;
     const std::string first = b200la_last_error();
     if (join() != B200LA_OK) fail(B200LA_ERR_CUDA, "%s", first.c_str());  // the first error stays
   }
 };
 
-// Launches the listed systems' clusters: one launch per group of equal
-// cluster size, offset count and rows a thread, the largest clusters first,
-// on side streams between two events of the context stream, so that the
-// groups share the GPU.
-template <typename T> int launch_clusters_t(BatchHandle B, int budget) {
+// Orders the listed clusters (the largest first, groups of equal instances
+// together), copies the list and stamps the start; the clusters may run from
+// the event recorded here on.
+int stage_clusters(BatchHandle B) {
   std::vector<int> &sl = B->cl_slots;
+  if (sl.empty()) return B200LA_OK;
   cudaStream_t st = B->ctx->stream;
   auto key = [&](int s) { return cl_instance(B->sys[s]); };
   std::stable_sort(sl.begin(), sl.end(), [&](int a, int b) {
     const int ka = key(a), kb = key(b);
     return ka != kb ? ka > kb : B->sys[a].n > B->sys[b].n;
   });
-  B_CUDA(cudaMemcpyAsync(B->cl_list, sl.data(), sizeof(int) * sl.size(), cudaMemcpyHostToDevice, st));
-  B_CUDA(cudaStreamSynchronize(st));  // the list is rebuilt on the host for the next launch
-  cluster_begin_kernel<<<((int)sl.size() + kBlock - 1) / kBlock, kBlock, 0, st>>>(B->cl_list, (int)sl.size(), B->st);
+  // the clusters' systems, then those of the item lists (for the start only)
+  std::vector<int> &all = B->all_slots;  // outlives the copy
+  all = sl;
+  all.insert(all.end(), B->list_slots.begin(), B->list_slots.end());
+  B_CUDA(cudaMemcpyAsync(B->cl_list, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, st));
+  batch_begin_kernel<<<((int)all.size() + kBlock - 1) / kBlock, kBlock, 0, st>>>(B->cl_list, (int)all.size(), B->st);
   B_CUDA(cudaGetLastError());
   B->launched += 1;
   B_CUDA(cudaEventRecord(B->cl_event[4], st));
-  SideStreams side{B};
+  return B200LA_OK;
+}
+
+// Launches the listed systems' clusters: one launch per group of equal
+// cluster size, offset count and rows a thread, on side streams behind
+// stage_clusters' event, so that the groups share the GPU with one another and
+// with the pass kernels.
+template <typename T> int launch_clusters_t(BatchHandle B, int budget, SideStreams &side) {
+  std::vector<int> &sl = B->cl_slots;
+  auto key = [&](int s) { return cl_instance(B->sys[s]); };
+  side.slots = sl;
+  for (int s : sl) B->sys[s].flying = true;
   int turn = 0;
   for (size_t a = 0; a < sl.size();) {
     size_t e = a;
@@ -2048,20 +2077,24 @@ template <typename T> int launch_clusters_t(BatchHandle B, int budget) {
     })));
     a = e;
   }
-  return side.join();
+  return B200LA_OK;
 }
 
-int launch_clusters(BatchHandle B, int budget) {
+int launch_clusters(BatchHandle B, int budget, SideStreams &side) {
   if (B->cl_slots.empty()) return B200LA_OK;
-  return B->kp.mixed ? launch_clusters_t<float>(B, budget) : launch_clusters_t<double>(B, budget);
+  return B->kp.mixed ? launch_clusters_t<float>(B, budget, side) : launch_clusters_t<double>(B, budget, side);
+}
+
+// After the globals came back: the kernels of the graph's passes.
+void count_lists(BatchHandle B) {
+  const BatchGlobals &g = *B->glob_host;
+  if (B->ctx->use_graphs && g.passes > 0) B->launched += 1 + 3 * (int64_t)g.passes;
 }
 
 // After the states came back: adds the cluster systems of the launch to the
 // passes it took and to the systems still running.
 void count_clusters(BatchHandle B) {
   BatchGlobals &g = *B->glob_host;
-  B->list_passes = g.passes;
-  if (B->ctx->use_graphs && g.passes > 0) B->launched += 1 + 3 * (int64_t)g.passes;  // the graph's
   for (int s : B->cl_slots) {
     g.passes = std::max(g.passes, B->st_host[s].cl_passes);
     if (B->st_host[s].phase != PH_DONE) g.active += 1;
@@ -2661,7 +2694,7 @@ int issue_early_copies(b200la_batch B) {
   const bool mixed = B->kp.mixed != 0;
   for (int s = 0; s < B->capacity; ++s) {
     HostSys &h = B->sys[s];
-    if (!h.used || !h.out || h.out_copied || B->st_host[s].phase != PH_DONE) continue;
+    if (!h.used || h.flying || !h.out || h.out_copied || B->st_host[s].phase != PH_DONE) continue;
     const double *xd = mixed ? h.d32.x : h.d64.x;
     B_CUDA(cudaMemcpyAsync(h.out, xd, 8 * (size_t)h.n, cudaMemcpyDeviceToHost, B->xfer));
     h.out_copied = true;
@@ -2679,49 +2712,42 @@ int wait_early_copies(b200la_batch B) {
   return B200LA_OK;
 }
 
+// States and globals back to the host, behind what the context stream holds.
+int read_back(b200la_batch B) {
+  cudaStream_t st = B->ctx->stream;
+  B_CUDA(cudaMemcpyAsync(B->st_host, B->st, sizeof(SysState) * B->capacity, cudaMemcpyDeviceToHost, st));
+  B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
+  B_CUDA(cudaStreamSynchronize(st));
+  B->pass_total = B->glob_host->pass_total;
+  return B200LA_OK;
+}
+
 // Completes a b200la_batch_launch: the states and globals come back after the
 // launch (and after any add queued since, which the context stream waits for).
 int complete_inflight(b200la_batch B) {
   if (!B->in_flight) return B200LA_OK;
-  cudaStream_t st = B->ctx->stream;
   B->in_flight = false;
-  B_CUDA(cudaMemcpyAsync(B->st_host, B->st, sizeof(SysState) * B->capacity, cudaMemcpyDeviceToHost, st));
-  B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
-  B_CUDA(cudaStreamSynchronize(st));
-  B->pass_total = B->glob_host->pass_total;
+  B_TRY(read_back(B));
+  count_lists(B);
   count_clusters(B);
   return issue_early_copies(B);
 }
 
-// One run: the cluster systems for at most cluster_passes passes, then the
-// pass kernels over the others for at most max_passes.
-int run_passes(b200la_batch B, int max_passes, int cluster_passes, int *active_out) {
-  B_TRY(complete_inflight(B));
-  cudaStream_t st = B->ctx->stream;
-  int active = 0;
-  B_TRY(upload_tiles(B, true, &active, nullptr, true));
-  BatchGlobals &g = *B->glob_host;
-  if (active == 0 && B->cl_slots.empty()) {
-    g.passes = 0;
-    B->list_passes = 0;
-    if (active_out) *active_out = 0;
-    return B200LA_OK;
-  }
+// The pass kernels over the uploaded lists, on the context stream (the host
+// loop waits for them).
+int run_lists(b200la_batch B, int active) {
+  if (active == 0) return B200LA_OK;
+  if (!B->ctx->use_graphs) return host_loop(B);
+  B_CUDA(cudaGraphLaunch(B->exec, B->ctx->stream));
+  return B200LA_OK;
+}
+
+// Globals of the next launch over the uploaded lists, and its graph.
+int prepare_lists(b200la_batch B, int active, int max_passes) {
   if (active > 0 && B->ctx->use_graphs && !B->exec) B_TRY(build_graph(B));
   set_globals(B, active, max_passes);
-  B_CUDA(cudaMemcpyAsync(B->glob, &g, sizeof(BatchGlobals), cudaMemcpyHostToDevice, st));
-  B_TRY(launch_clusters(B, cluster_passes));
-  if (active > 0) {
-    if (B->ctx->use_graphs) B_CUDA(cudaGraphLaunch(B->exec, st));
-    else B_TRY(host_loop(B));
-  }
-  B_CUDA(cudaMemcpyAsync(B->st_host, B->st, sizeof(SysState) * B->capacity, cudaMemcpyDeviceToHost, st));
-  B_CUDA(cudaMemcpyAsync(B->glob_host, B->glob, sizeof(BatchGlobals), cudaMemcpyDeviceToHost, st));
-  B_CUDA(cudaStreamSynchronize(st));
-  B->pass_total = B->glob_host->pass_total;
-  count_clusters(B);
-  if (active_out) *active_out = B->glob_host->active;
-  return issue_early_copies(B);
+  B_CUDA(cudaMemcpyAsync(B->glob, B->glob_host, sizeof(BatchGlobals), cudaMemcpyHostToDevice, B->ctx->stream));
+  return B200LA_OK;
 }
 }  // namespace
 
@@ -2730,42 +2756,86 @@ extern "C" {
 int b200la_batch_launch(b200la_batch B, int max_passes) {
   B_CHECK(B && max_passes >= 1, B200LA_ERR_INVALID, "batch_launch: bad argument");
   B_TRY(complete_inflight(B));
-  cudaStream_t st = B->ctx->stream;
-  int active = 0;
-  B_TRY(upload_tiles(B, true, &active, nullptr, true));
-  BatchGlobals &g = *B->glob_host;
-  if (active == 0 && B->cl_slots.empty()) return B200LA_OK;
   if (!B->ctx->use_graphs) {  // the host loop waits on the device anyway
     int a = 0;
     return b200la_batch_run(B, max_passes, &a);
   }
-  if (active > 0 && !B->exec) B_TRY(build_graph(B));
-  set_globals(B, active, max_passes);
-  B_CUDA(cudaMemcpyAsync(B->glob, &g, sizeof(BatchGlobals), cudaMemcpyHostToDevice, st));
-  B_TRY(launch_clusters(B, max_passes));
-  if (active > 0) B_CUDA(cudaGraphLaunch(B->exec, st));
+  int active = 0;
+  B_TRY(upload_tiles(B, true, &active, nullptr, true));
+  if (active == 0 && B->cl_slots.empty()) return B200LA_OK;
+  B_TRY(prepare_lists(B, active, max_passes));
+  SideStreams side{B};
+  B_TRY(stage_clusters(B));
+  if (B->ctx->use_graphs) B_TRY(run_lists(B, active));
+  B_TRY(launch_clusters(B, max_passes, side));
+  if (!B->ctx->use_graphs) B_TRY(run_lists(B, active));
+  B_TRY(side.join());
   B->in_flight = true;
   return B200LA_OK;
 }
 
+// One run: clusters and pass kernels side by side, at most max_passes passes.
 int b200la_batch_run(b200la_batch B, int max_passes, int *active_out) {
   B_CHECK(B && max_passes >= 1, B200LA_ERR_INVALID, "batch_run: bad argument");
-  return run_passes(B, max_passes, max_passes, active_out);
+  B_TRY(complete_inflight(B));
+  int active = 0;
+  B_TRY(upload_tiles(B, true, &active, nullptr, true));
+  if (active == 0 && B->cl_slots.empty()) {
+    B->glob_host->passes = 0;
+    if (active_out) *active_out = 0;
+    return B200LA_OK;
+  }
+  B_TRY(prepare_lists(B, active, max_passes));
+  SideStreams side{B};
+  B_TRY(stage_clusters(B));
+  if (B->ctx->use_graphs) B_TRY(run_lists(B, active));
+  B_TRY(launch_clusters(B, max_passes, side));
+  if (!B->ctx->use_graphs) B_TRY(run_lists(B, active));
+  B_TRY(side.join());
+  B_TRY(read_back(B));
+  count_lists(B);
+  count_clusters(B);
+  if (active_out) *active_out = B->glob_host->active;
+  return issue_early_copies(B);
 }
 
 int b200la_batch_solve(b200la_batch B, int chunk_passes, int *total_passes) {
   B_CHECK(B && chunk_passes >= 1, B200LA_ERR_INVALID, "batch_solve: bad argument");
-  int active = 1, lists = 0, total = 0;
-  // each run ends after chunk_passes passes; the next run's tile list holds
-  // only the systems still running, so finished systems stop costing passes
+  B_TRY(complete_inflight(B));
+  int active = 0;
+  B_TRY(upload_tiles(B, true, &active, nullptr, true));
+  // systems on clusters have nothing to compact: they run to their end beside
+  // the pass kernels, whose launches end after chunk_passes passes; the next
+  // one's list holds only the systems still running, so finished systems stop
+  // costing passes
+  const std::vector<int> on_clusters = B->cl_slots;
+  SideStreams side{B};
+  B_TRY(stage_clusters(B));
+  int lists = 0;
+  bool flown = false;
   while (active > 0) {
-    // systems on clusters have nothing to compact: they run to their end
-    B_TRY(run_passes(B, chunk_passes, INT32_MAX, &active));
-    lists += B->list_passes;
-    total = std::max(total, std::max(lists, B->glob_host->passes));
+    B_TRY(prepare_lists(B, active, chunk_passes));
+    if (B->ctx->use_graphs) B_TRY(run_lists(B, active));
+    if (!flown) B_TRY(launch_clusters(B, INT32_MAX, side));
+    flown = true;
+    if (!B->ctx->use_graphs) B_TRY(run_lists(B, active));
+    if (side.used > 0 && side.done()) B_TRY(side.join());  // their solutions can go out
+    B_TRY(read_back(B));
+    count_lists(B);
+    lists += B->glob_host->passes;
+    B_TRY(issue_early_copies(B));
+    B_TRY(upload_tiles(B, true, &active, nullptr, true));
   }
-  B->glob_host->passes = total;
-  if (total_passes) *total_passes = total;
+  if (!flown) B_TRY(launch_clusters(B, INT32_MAX, side));
+  B_TRY(side.join());
+  if (!on_clusters.empty()) {
+    B_TRY(read_back(B));
+    B_TRY(issue_early_copies(B));
+  }
+  B->cl_slots = on_clusters;
+  B->glob_host->passes = lists;
+  count_clusters(B);
+  if (total_passes) *total_passes = B->glob_host->passes;
   return B200LA_OK;
 }
 

@@ -711,3 +711,46 @@ def test_tune_times_what_the_pass_kernels_run(plat):
         assert r.solver_state == lmp.kSolverSuccess
         assert np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, v, r.x)) < 1.001e-8 * np.linalg.norm(s.b)
     B.close()
+
+
+def test_clusters_and_pass_kernels_side_by_side(plat):
+    """solve() runs the clusters beside the launches of the pass kernels: with
+    launches of 4 passes the lists are rebuilt many times while clusters are
+    in flight.  Every system ends with the bits it gets alone, the registered
+    outputs hold them, and no system's time is longer than the solve."""
+    import time
+
+    import torch
+    systems = []
+    for k, c in enumerate((20, 150, 40, 180, 90, 250)):
+        s = P.q1_system(2, c, 700 + k, 1.0, f"side{k}")
+        val = s.val.copy()
+        if k % 2:
+            val[s.rowptr[s.n // 2]] *= 1.0 + 1e-3
+        systems.append((s.rowptr, s.col, val, s.b))
+    kw = dict(mixed=True, precond=True, rtol=1e-8, platform=plat)
+    ref = []
+    for t in systems:
+        A = Batch(1, **kw)
+        A.set_items(128, 512, 512, adaptive=False)
+        sl = A.add(*t)
+        A.solve()
+        ref.append(A.result(sl))
+        A.close()
+    B = Batch(len(systems), **kw)
+    B.set_items(128, 512, 512, adaptive=False)
+    slots = B.add_many(systems)
+    assert [B.form(sl) for sl in slots] == [FORM_CLUSTER, FORM_KERNELS] * 3
+    for chunk in (4, 64):
+        outs = [torch.empty(t[3].size, dtype=torch.float64).pin_memory().numpy() for t in systems]
+        B.restart()
+        B.set_outputs(slots, outs)
+        plat.synchronize()
+        t0 = time.perf_counter()
+        B.solve(chunk)
+        wall = 1e6 * (time.perf_counter() - t0)
+        for r, g, o in zip(ref, B.results(slots, out=outs), outs):
+            assert g.solver_state == lmp.kSolverSuccess and (g.iters, g.outer) == (r.iters, r.outer)
+            assert g.x is o and np.array_equal(o, r.x)
+            assert 0.0 < g.device_us <= wall
+    B.close()
