@@ -615,7 +615,7 @@ def test_a_failed_cluster_launch_leaves_nothing_running(plat, monkeypatch):
     group's clusters, already launched on a side stream, are in front of the
     context stream's later work: a wait for that stream finds their solution
     written, and the next solve ends every system with the usual bits."""
-    big, small = P.q1_system(2, 250, 3, 1.0, "big"), P.q1_system(2, 20, 4, 1.0, "small")
+    big, small = P.q1_system(2, 250, 3, 1.0, "big"), P.q1_system(2, 120, 4, 1.0, "small")
     items = [(s.rowptr, s.col, s.val, s.b) for s in (big, small)]
     kw = dict(mixed=True, precond=True, rtol=1e-8, platform=plat)
     A = Batch(2, **kw)
@@ -754,3 +754,16 @@ def test_clusters_and_pass_kernels_side_by_side(plat):
             assert g.x is o and np.array_equal(o, r.x)
             assert 0.0 < g.device_us <= wall
     B.close()
+
+
+def test_small_systems_do_not_wait_for_large_ones(plat):
+    """Small systems of a batch finish before the large ones: with 40 of 250
+    cells, which fill the GPU several times over, 40 of 30 cells take a small
+    part of the time."""
+    sizes = [250, 30] * 40
+    B = Batch(len(sizes), mixed=True, precond=True, rtol=1e-8, platform=plat)
+    slots = [B.add_q1(2, n, 900 + k, 1.0) for k, n in enumerate(sizes)]
+    B.solve()
+    us = [r.device_us for r in B.results(slots, with_x=False)]
+    B.close()
+    assert max(us[1::2]) < 0.25 * max(us[0::2]), (max(us[1::2]), max(us[0::2]))
