@@ -54,8 +54,9 @@
 //               -> RESID (mixed) or DONE (FP64 mode)
 //   DONE    skipped by every kernel
 // Systems that fit on the SMs of one thread-block cluster (cluster_cg.cuh:
-// symmetric, structured offsets, up to ~70,000 rows) do not take part in the
-// passes below: batch_cluster_kernel walks the same phases with the matrix
+// symmetric, structured offsets, nine entries a row up to 136,161 FP32 or
+// 66,049 FP64 rows, 27 up to 15,625 or 8,000) do not take part in the passes
+// below: batch_cluster_kernel walks the same phases with the matrix
 // and the Krylov vectors on chip, one cluster a system, as many passes as the
 // run allows, and leaves the state as the pass kernels would.  Which form a
 // system takes depends on the system alone, never on the batch around it.

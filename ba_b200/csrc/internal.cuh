@@ -132,8 +132,6 @@ struct b200la_mat_s {
 
 namespace b200la {
 
-// Host validation of a CSR structure: rowptr[0] == 0, non-decreasing,
-// rowptr[nrow] == nnz, 0 <= col < ncol.  Writes the longest row length.
 // Threads per row of the CSR schedule a matrix starts with: enough for the
 // rows' length, but on rows of nearly equal length that fill the GPU more
 // than about twice (2,048 threads a SM) only 2 (up to 14 entries) or 4 (up to
@@ -150,6 +148,8 @@ inline int csr_start_lanes(int64_t nrow, double avg, int max_row, int sms) {
   return avg <= 14 ? 2 : 4;
 }
 
+// Host validation of a CSR structure: rowptr[0] == 0, non-decreasing,
+// rowptr[nrow] == nnz, 0 <= col < ncol.  Writes the longest row length.
 int validate_csr(int nrow, int ncol, int64_t nnz, const int *rowptr, const int *col, int *max_row);
 
 // Q1 system assembly on the device (assemble.cu).

@@ -441,9 +441,10 @@ int b200la_mp_solve(b200la_mp s, b200la_vec b, b200la_vec x, b200la_mp_result *r
  * solves inside FP64 refinement (mixed = 1, MPIR structure, mpir.cc:52-230).
  * Systems can be added and removed between runs (continuous batching).
  * Systems with a symmetric, structured matrix that fits on the SMs of one
- * thread-block cluster (up to ~70,000 rows of nine entries in mixed mode) are
- * iterated there, one cluster a system, instead of by the swept kernels; a run
- * takes them the same number of passes. */
+ * thread-block cluster (nine entries a row: up to 136,161 rows in mixed mode,
+ * 66,049 in FP64) are iterated there, one cluster a system, beside the swept
+ * kernels instead of by them.  A run or launch takes them its number of
+ * passes, a solve to their end. */
 typedef struct {
   int capacity;       /* system slots */
   int mixed;          /* 1: FP32 inner PCG + FP64 refinement; 0: FP64 PCG */

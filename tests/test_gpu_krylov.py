@@ -452,3 +452,40 @@ def test_gmres_solvers_of_several_sizes_live_together(plat):
         g.Solve(b, x)
         assert g.iter() == 20
         assert np.linalg.norm(s.b - oracle.spmv(s.rowptr, s.col, s.val, x.numpy())) < np.linalg.norm(s.b)
+
+
+def test_gmres_when_the_basis_loses_orthogonality(plat, monkeypatch):
+    """One long cycle on an unscaled system (coefficient contrast e^9), whose
+    Gram-Schmidt basis is orthogonal to 5e-11 after 100 steps, to 1.5e-5 after
+    200 and not at all after 300 (shown here in numpy).  The resident step
+    takes its coefficients from a triangular system instead of the chain of
+    projections; both forms must follow the oracle's chain as far as the basis
+    carries it and end with a backward error of a stable method, n eps."""
+    import scipy.sparse as sp
+    s = P.q1_system(2, 20, 7, 3.0, "lost")
+    A = sp.csr_matrix((s.val, s.col, s.rowptr), shape=(s.n, s.n))
+    V = np.zeros((s.n, 301))
+    V[:, 0] = s.b / np.linalg.norm(s.b)
+    for j in range(300):
+        w = A @ V[:, j]
+        for i in range(j + 1):
+            w -= (V[:, i] @ w) * V[:, i]
+        V[:, j + 1] = w / np.linalg.norm(w)
+    lost = {k: np.linalg.norm(np.eye(k + 1) - V[:, :k + 1].T @ V[:, :k + 1]) for k in (100, 200, 300)}
+    assert lost[100] < 1e-9 < 1e-6 < lost[200] < 1e-3 and lost[300] > 1.0
+    anorm = sp.linalg.norm(A)
+    for form in ("1", "0"):
+        monkeypatch.setenv("B200LA_GMRES_RESIDENT", form)
+        for k in (100, 200, 300):
+            ref = oracle.gmres(s.rowptr, s.col, s.val, s.b, size_basis=k, maxits=k, atol=0.0, rtol=1e-13,
+                               precond=False)
+            solver, _, x = _solve_gmres(plat, s, False, k, maxits=k, rtol=1e-13)
+            assert solver.iter() == ref.iters == k
+            if k < 300:
+                # rounding moves a step's residual by about what the basis has lost
+                assert abs(solver.res() - ref.res) <= 100 * lost[k] * ref.res, (form, k, solver.res(), ref.res)
+            true_res = np.linalg.norm(s.b - A @ x)
+            if k == 300:
+                bound = s.n * np.finfo(np.float64).eps
+                assert true_res <= bound * (anorm * np.linalg.norm(x) + np.linalg.norm(s.b)), (form, true_res)
+                assert true_res <= 100 * np.linalg.norm(s.b - A @ ref.x), (form, true_res)
