@@ -10,7 +10,8 @@
 //      fails the upload) and counts the rows with atomics, each entry keeping
 //      the count it met as its place in the row,
 //   2. the row pointer as the counts' prefix sum,
-//   3. a scatter of (column, input position) pairs to their places; within a
+//   3. a scatter of (column, input position) pairs to their places, in windows
+//      that fit in the L2 where the triplets come in no order; within a
 //      row these come in the order the atomics ran in, which is never used:
 //   4. the row sort, one warp per row: when the row's columns are distinct
 //      the sorted row is unique, ranks come from shuffles and each value from
@@ -24,6 +25,7 @@
 // 12-byte records) and a separate gather took 1.4 + 1.2 of 3.8 ms on 57 M
 // triplets.
 // The result is the reference's CSR bit for bit, duplicates included.
+#include <algorithm>
 #include <climits>
 #include <cstring>
 
@@ -33,13 +35,20 @@ namespace b200la {
 
 // First bad triplet (smallest index), or all ones when every index is in
 // range; place[i] = how many entries of its row were counted before entry i.
-// Four entries in flight per thread.
+// Four entries in flight per thread.  With FAR one block in kFarBlocks
+// counts, of one entry in four, the neighbours in the input whose rows lie
+// span or more apart (far).
+constexpr int kFarBlocks = 8;
+template <bool FAR>
 __global__ void __launch_bounds__(kBlock) coo_count_kernel(int64_t nnz, int nrow, int ncol,
                                                            const int *__restrict__ rows,
                                                            const int *__restrict__ cols, int *__restrict__ count,
-                                                           int *__restrict__ place, unsigned long long *bad) {
+                                                           int *__restrict__ place, unsigned long long *bad, int span,
+                                                           int *far) {
   constexpr int U = 4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const bool sample = FAR && blockIdx.x % kFarBlocks == 0;
+  int jumps = 0;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nnz; i0 += U * stride) {
     int r[U], c[U];
 #pragma unroll
@@ -48,6 +57,7 @@ __global__ void __launch_bounds__(kBlock) coo_count_kernel(int64_t nnz, int nrow
       r[u] = in ? rows[i0 + u * stride] : 0;
       c[u] = in ? cols[i0 + u * stride] : 0;
     }
+    if (sample && i0 + 1 < nnz) jumps += abs(rows[i0 + 1] - r[0]) >= span ? 1 : 0;
     int p[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -63,6 +73,10 @@ __global__ void __launch_bounds__(kBlock) coo_count_kernel(int64_t nnz, int nrow
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (i0 + u * stride < nnz) place[i0 + u * stride] = p[u];
+  }
+  if (sample) {
+    jumps = (int)warp_sum((double)jumps);
+    if ((threadIdx.x & 31) == 0 && jumps) atomicAdd(far, jumps);
   }
 }
 
@@ -144,8 +158,20 @@ __global__ void __launch_bounds__(kBlock) coo_rowptr_kernel(int nrow, int nnz, c
 }
 
 // Each triplet's column (high word) and input position (low word) to its
-// place in its row.
-__global__ void __launch_bounds__(kBlock) coo_scatter_kernel(int64_t nnz, const int *__restrict__ rows,
+// place in its row; with PART only those of rows row0 .. row1 - 1.
+// Triplets in random order write random 8 bytes of the pairs' array.  Beyond
+// the L2 each write costs a sector of its own, so the array is then filled in
+// windows that stay in the L2, one launch each, which re-reads the rows (4
+// bytes an entry and launch) and lets a sector's entries meet.  us a
+// conversion, one launch and windows (radix sort by row in brackets): 96^3,
+// 24 M triplets, 193 MB of pairs 1,448 1,267 (1,591), 128^3, 57 M 4,173 3,510
+// (3,796), 140^3, 75 M 5,704 4,960 (5,007); windows of half the size 3,580 on
+// 128^3, of twice 3,535.
+constexpr int kMaxWindows = 8;
+
+template <bool PART>
+__global__ void __launch_bounds__(kBlock) coo_scatter_kernel(int64_t nnz, int row0, int row1,
+                                                             const int *__restrict__ rows,
                                                              const int *__restrict__ cols,
                                                              const int *__restrict__ place,
                                                              const int *__restrict__ rowptr,
@@ -153,16 +179,23 @@ __global__ void __launch_bounds__(kBlock) coo_scatter_kernel(int64_t nnz, const 
   constexpr int U = 4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nnz; i0 += U * stride) {
-    int at[U], c[U];
+    int at[U], c[U], r[U];
+    bool mine[U];  // PART: the row decides; else the other loads need not wait for it
+    if (PART) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) r[u] = i0 + u * stride < nnz ? rows[i0 + u * stride] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) mine[u] = PART ? r[u] >= row0 && r[u] < row1 : i0 + u * stride < nnz;
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (i0 + u * stride < nnz) {
-        at[u] = __ldg(rowptr + rows[i0 + u * stride]) + place[i0 + u * stride];
+      if (mine[u]) {
+        at[u] = __ldg(rowptr + (PART ? r[u] : rows[i0 + u * stride])) + place[i0 + u * stride];
         c[u] = cols[i0 + u * stride];
       }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (i0 + u * stride < nnz)
+      if (mine[u])
         out[at[u]] = ((unsigned long long)(unsigned)c[u] << 32) | (unsigned long long)(unsigned)(i0 + u * stride);
   }
 }
@@ -449,13 +482,14 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
         !cu(cudaMallocAsync(&m->col, sizeof(int) * nz, s), "allocation") ||
         !cu(cudaMallocAsync(&m->val, dtype_size(dtype) * nz, s), "allocation") ||
         !cu(cudaMallocAsync(&m->diag, sizeof(int) * (size_t)(nrow > 0 ? nrow : 1), s), "allocation") ||
-        !cu(cudaMallocAsync(&bad, sizeof(unsigned long long) + 2 * sizeof(int), s), "allocation"))
+        !cu(cudaMallocAsync(&bad, sizeof(unsigned long long) + 4 * sizeof(int), s), "allocation"))
       break;
     max_row_d = reinterpret_cast<int *>(bad + 1);
     n_long_d = max_row_d + 1;
+    int *far_d = max_row_d + 2;
     const unsigned long long none = ~0ull;
     if (!cu(cudaMemcpyAsync(bad, &none, sizeof(none), cudaMemcpyHostToDevice, s), "copy") ||
-        !cu(cudaMemsetAsync(max_row_d, 0, 2 * sizeof(int), s), "memset"))
+        !cu(cudaMemsetAsync(max_row_d, 0, 4 * sizeof(int), s), "memset"))
       break;
     if (nnz == 0) {
       if (!cu(cudaMemsetAsync(m->rowptr, 0, sizeof(int) * ((size_t)nrow + 1), s), "memset")) break;
@@ -481,14 +515,25 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
     int *count = m->diag, *place = m->col;
     const int g = grid_1d(c, (nnz + 3) / 4);
     if (nrow > 0 && !cu(cudaMemsetAsync(count, 0, sizeof(int) * (size_t)nrow, s), "memset")) break;
-    coo_count_kernel<<<g, kBlock, 0, s>>>(nnz, nrow, ncol, r_in, c_in, count, place, bad);
-    unsigned long long hbad = 0;
+    // windows of the scatter (three quarters of the L2 each), where the order
+    // of the triplets needs them: more than one neighbour in eight apart
+    int l2 = 0;
+    if (!cu(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c->device), "L2 size")) break;
+    const int64_t window = std::max<int64_t>(1, (int64_t)l2 / 4 * 3);
+    int windows = (int)std::min<int64_t>(kMaxWindows, ((int64_t)sizeof(unsigned long long) * nnz + window - 1) / window);
+    const int span = windows > 1 ? std::max(1, nrow / windows) : 0;
+    const auto count_rows = span > 0 ? coo_count_kernel<true> : coo_count_kernel<false>;
+    count_rows<<<g, kBlock, 0, s>>>(nnz, nrow, ncol, r_in, c_in, count, place, bad, span, far_d);
+    struct {
+      unsigned long long bad;
+      int max_row, n_long, far, pad;
+    } seen = {};
     if (!cu(cudaGetLastError(), "check") ||
-        !cu(cudaMemcpyAsync(&hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, s), "copy") ||
+        !cu(cudaMemcpyAsync(&seen, bad, sizeof(seen), cudaMemcpyDeviceToHost, s), "copy") ||
         !cu(cudaStreamSynchronize(s), "check"))
       break;
-    if (hbad != ~0ull) {
-      rc = fail(B200LA_ERR_MATRIX, "coo_upload: triplet %llu has an index out of range", hbad);
+    if (seen.bad != ~0ull) {
+      rc = fail(B200LA_ERR_MATRIX, "coo_upload: triplet %llu has an index out of range", seen.bad);
       break;
     }
     const int blocks = (int)(((int64_t)nrow + kScanRows - 1) / kScanRows);  // nrow > 0: every index is in range
@@ -499,7 +544,14 @@ extern "C" int b200la_coo_upload(b200la_ctx c, int nrow, int ncol, int64_t nnz, 
     coo_block_sum_kernel<<<blocks, kBlock, 0, s>>>(nrow, count, sums);
     coo_scan_sums_kernel<<<1, 1024, 0, s>>>(blocks, sums);
     coo_rowptr_kernel<<<blocks, kBlock, 0, s>>>(nrow, (int)nnz, count, sums, m->rowptr);
-    coo_scatter_kernel<<<g, kBlock, 0, s>>>(nnz, r_in, c_in, place, m->rowptr, packed);
+    if (seen.far <= nnz / (8 * 4 * kFarBlocks)) windows = 1;
+    for (int k = 0; k < windows; ++k) {
+      const int row0 = (int)((int64_t)nrow * k / windows), row1 = (int)((int64_t)nrow * (k + 1) / windows);
+      if (windows == 1)
+        coo_scatter_kernel<false><<<g, kBlock, 0, s>>>(nnz, row0, row1, r_in, c_in, place, m->rowptr, packed);
+      else
+        coo_scatter_kernel<true><<<g, kBlock, 0, s>>>(nnz, row0, row1, r_in, c_in, place, m->rowptr, packed);
+    }
     const int gr = grid_1d(c, (int64_t)nrow * 32);
     auto sort_rows = [&](auto t, auto u) {
       using T = decltype(t);

@@ -185,3 +185,44 @@ def test_row_and_block_edges_match_oracle(plat, nrow, dup):
     A = lmp.B200_CSR_lMatrix.TransformFromCOO(rows, cols, vals, nrow, 400, platform=plat)
     for got, want in zip(A.csr(), ref):
         np.testing.assert_array_equal(got, want)
+
+
+def test_large_shuffled_and_ordered_triplets(plat):
+    """24 M triplets (193 MB of pairs, more than the L2): in random order the
+    scatter goes in windows, in row order in one launch, and with the rows'
+    halves interleaved (every neighbour far apart) in windows again.  Distinct
+    columns: the CSR is unique and equals the generator's."""
+    import torch
+    cells = 96
+    n1 = cells + 1
+    n = n1 ** 3
+    dev = "cuda"
+    node = torch.arange(n, device=dev)
+    z, y, x = node // (n1 * n1), node // n1 % n1, node % n1
+    rows, cols = [], []
+    for dz in (-1, 0, 1):
+        for dy in (-1, 0, 1):
+            for dx in (-1, 0, 1):
+                ok = ((z + dz >= 0) & (z + dz < n1) & (y + dy >= 0) & (y + dy < n1) & (x + dx >= 0) & (x + dx < n1))
+                rows.append(node[ok])
+                cols.append(node[ok] + dz * n1 * n1 + dy * n1 + dx)
+    rows, cols = torch.cat(rows), torch.cat(cols)
+    order = torch.argsort(rows * n + cols)
+    rows, cols = rows[order].to(torch.int32), cols[order].to(torch.int32)
+    vals = torch.rand(rows.numel(), device=dev, dtype=torch.float64)
+    assert rows.numel() * 8 > torch.cuda.get_device_properties(0).L2_cache_size
+    ptr = np.zeros(n + 1, np.int64)
+    np.cumsum(torch.bincount(rows, minlength=n).cpu().numpy(), out=ptr[1:])
+    half = rows.numel() // 2
+    weave = torch.stack([torch.arange(half, device=dev), torch.arange(half, 2 * half, device=dev)], 1).reshape(-1)
+    if 2 * half < rows.numel():
+        weave = torch.cat([weave, torch.tensor([2 * half], device=dev)])
+    for p in (None, torch.randperm(rows.numel(), device=dev), weave):
+        trip = (rows, cols, vals) if p is None else (rows[p].contiguous(), cols[p].contiguous(), vals[p].contiguous())
+        torch.cuda.synchronize()
+        A = lmp.B200_CSR_lMatrix.TransformFromCOO(*trip, n, n, platform=plat)
+        rp, cc, vv = A.csr()
+        np.testing.assert_array_equal(rp, ptr)
+        np.testing.assert_array_equal(cc, cols.cpu().numpy())
+        np.testing.assert_array_equal(vv, vals.cpu().numpy())
+        A.Clear()
