@@ -97,10 +97,17 @@ template <typename T> struct SysDesc {
   double *x;
   T *c, *r, *p, *Ap;
   const T *invd;
-  int cl_H;           // upper offsets of the symmetric set (cluster form), 0: none
-  int cl_off[kClMaxOff];
   int stencil;        // 1: values-only layout, entry k of a row at column row + soff[k] (scol unused)
   int soff[kMaxStencil];  // ascending column offsets of the stencil layout (ell of them)
+};
+
+// Upper offsets of a slot's symmetric set (cluster form; H = 0: none).  Apart
+// from SysDesc, which the pass kernels index for every item: with 56 more
+// bytes there, batch_spmv_kernel<double> spilled and took 59.7 us over 37 3D
+// systems instead of 44.6.
+struct ClDesc {
+  int H;
+  int off[kClMaxOff];
 };
 
 // Per-system scalars and counters (device).
@@ -957,6 +964,7 @@ __global__ void slot_setup_kernel(SysDesc<T> d, unsigned *bad) {
 // whether x starts at zero.
 template <typename T> struct SetupJob {
   SysDesc<T> d;
+  ClDesc cl;
   int slot;
   int zero_x;
 };
@@ -964,7 +972,7 @@ template <typename T> struct SetupJob {
 // Descriptor and fresh RESID state of every job's slot (thread per job).
 template <typename T>
 __global__ void slot_init_many_kernel(const SetupJob<T> *__restrict__ jobs, int count, SysDesc<T> *desc,
-                                      SysState *st, int *sym) {
+                                      SysState *st, ClDesc *cl, int *sym) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     const int s = jobs[k].slot;
     desc[s] = jobs[k].d;
@@ -972,7 +980,8 @@ __global__ void slot_init_many_kernel(const SetupJob<T> *__restrict__ jobs, int 
     z.phase = PH_RESID;
     z.bad_row = 0xffffffffu;
     st[s] = z;
-    sym[s] = jobs[k].d.cl_H > 0 ? 1 : 0;
+    cl[s] = jobs[k].cl;
+    sym[s] = jobs[k].cl.H > 0 ? 1 : 0;
   }
 }
 
@@ -995,7 +1004,8 @@ __global__ void slot_setup_many_kernel(const SetupJob<T> *__restrict__ jobs, int
 template <typename T, int H, int R, bool PRE>
 __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int *__restrict__ list,
                                                                       const SysDesc<T> *__restrict__ desc,
-                                                                      SysState *st, BatchParams prm, int budget) {
+                                                                      const ClDesc *__restrict__ cld, SysState *st,
+                                                                      BatchParams prm, int budget) {
   extern __shared__ __align__(16) unsigned char cl_dyn[];
   const int sys = list[cl_cluster_id()];
   const SysDesc<T> &d = desc[sys];
@@ -1005,9 +1015,10 @@ __global__ void __launch_bounds__(kClThreads, 1) batch_cluster_kernel(const int 
   if (phase != PH_RESID && phase != PH_INNER) return;
   ClMatrix<double> m;
   m.n = d.n;
-  m.H = d.cl_H;
-  m.halo = d.cl_off[d.cl_H - 1];
-  for (int k = 0; k < kClMaxOff; ++k) m.off[k] = d.cl_off[k];
+  const ClDesc &cd = cld[sys];
+  m.H = cd.H;
+  m.halo = cd.off[cd.H - 1];
+  for (int k = 0; k < kClMaxOff; ++k) m.off[k] = cd.off[k];
   m.rowptr = d.rowptr;
   m.col = d.col;
   m.val = d.val64;
@@ -1182,7 +1193,7 @@ template <typename T>
 __global__ void sym_check_many_kernel(const SetupJob<T> *__restrict__ jobs, int count, int *sym) {
   for (int k = blockIdx.y; k < count; k += gridDim.y) {
     const SysDesc<T> &d = jobs[k].d;
-    if (d.cl_H == 0) continue;
+    if (jobs[k].cl.H == 0) continue;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n; i += gridDim.x * blockDim.x)
       if (!sym_row_ok(d.rowptr, d.col, d.val64, i)) sym[jobs[k].slot] = 0;
   }
@@ -1377,7 +1388,7 @@ struct HostSys {
   SysDesc<float> d32{};
   double *out = nullptr;   // registered host destination of the solution
   bool out_copied = false; // its copy is queued on the transfer stream
-  int cl_H = 0;            // cluster form possible if the values are symmetric (sym_host)
+  ClDesc cl{};             // cluster form possible if the values are symmetric (sym_host)
   int cl_blocks = 0, cl_rows = 0;  // blocks of its cluster, rows a thread (0: does not fit)
   size_t cl_smem = 0;
   bool flying = false;     // its cluster runs on a side stream: state and x are the kernel's
@@ -1452,6 +1463,7 @@ struct b200la_batch_s {
   // the last launch by group, and the streams that let groups overlap
   int *sym, *sym_host;         // device, pinned host [capacity]
   int *cl_list;                // device [capacity]
+  ClDesc *cl_desc;             // device [capacity]
   std::vector<int> cl_slots;   // slots of the last launch, as listed
   std::vector<int> list_slots; // slots of the item lists
   std::vector<int> all_slots;  // both, as copied to cl_list
@@ -1528,7 +1540,7 @@ template <typename T, typename F> int cl_with_kernel(BatchHandle B, int up, int 
   return up <= 4 ? with_h(std::integral_constant<int, 4>()) : with_h(std::integral_constant<int, kClMaxOff>());
 }
 
-int cl_instance(const HostSys &h) { return h.cl_blocks * 1000 + (h.cl_H > 4 ? 500 : 0) + h.cl_rows; }
+int cl_instance(const HostSys &h) { return h.cl_blocks * 1000 + (h.cl.H > 4 ? 500 : 0) + h.cl_rows; }
 
 // Prepares a system's instance when the batch first meets it: the attributes
 // belong to the kernel on the device and not to a batch, so every batch, in
@@ -1541,7 +1553,7 @@ template <typename T> int cl_prepare(BatchHandle B, const HostSys &h, bool *fits
   if (ready != 0) return B200LA_OK;
   int optin = 0, clusters = 0;
   B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device));
-  B_TRY((cl_with_kernel<T>(B, h.cl_H, h.cl_rows, [&](auto k) -> int {
+  B_TRY((cl_with_kernel<T>(B, h.cl.H, h.cl_rows, [&](auto k) -> int {
     cudaFuncAttributes fa;
     B_CUDA(cudaFuncGetAttributes(&fa, k));
     B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
@@ -1579,20 +1591,20 @@ constexpr size_t kClWideSmem = 196 * 1024 - 1024;  // the carve-out step below t
 // 26^3 6.2 / 6.1, 22.1 / 19.0 and 27^3 10.1 / 7.6, 37.0 / 21.6 (8 x 7); FP64,
 // 19^3 2.0 / 2.4, 6.8 / 6.2 (8 x 2), beyond it 21^3 3.6 / 2.8, 12.6 / 9.0
 // (8 x 4) and 25^3 6.3 / 5.2, 23.4 / 17.5 (16 x 2).
-template <typename T> int cl_plan(BatchHandle B, HostSys &h, const SysDesc<T> &d) {
-  h.cl_H = d.cl_H;
+template <typename T> int cl_plan(BatchHandle B, HostSys &h, const ClDesc &cl) {
+  h.cl = cl;
   h.cl_blocks = 0;
-  if (d.cl_H == 0 || !B->ctx->use_onchip) return B200LA_OK;
+  if (cl.H == 0 || !B->ctx->use_onchip) return B200LA_OK;
   int optin = 0;
   B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->ctx->device));
-  const int halo = d.cl_off[d.cl_H - 1];
+  const int halo = cl.off[cl.H - 1];
   for (int blocks = 1; blocks <= kClMaxBlocks; blocks *= 2) {
-    const int rpc = cl_rows_per_block(d.n, blocks);
+    const int rpc = cl_rows_per_block(h.n, blocks);
     const int need = (rpc + kClThreads - 1) / kClThreads;
-    const int held = d.cl_H <= 4 ? cl_rows_for<T, 4>(need) : cl_rows_for<T, kClMaxOff>(need);
-    const size_t smem = cl_smem_bytes(rpc, halo, d.cl_H, held, sizeof(T));
+    const int held = cl.H <= 4 ? cl_rows_for<T, 4>(need) : cl_rows_for<T, kClMaxOff>(need);
+    const size_t smem = cl_smem_bytes(rpc, halo, cl.H, held, sizeof(T));
     if (held == 0 || smem + 1024 > (size_t)optin) continue;
-    const bool wide = d.cl_H > 4;
+    const bool wide = cl.H > 4;
     if (wide && (blocks * held * (int)sizeof(T) > kClWideMax || (held == 7 && smem > kClWideSmem))) continue;
     h.cl_blocks = blocks;
     h.cl_rows = held;
@@ -1710,7 +1722,7 @@ int upload_stage(BatchHandle B, int slot, int n, int64_t nnz, const int *rowptr,
 }
 
 template <typename T>
-int finish_stage(BatchHandle B, int slot, const CsrCheck &c, SysDesc<T> &d) {
+int finish_stage(BatchHandle B, int slot, const CsrCheck &c, SysDesc<T> &d, ClDesc &cl) {
   if (c.err != ~0ull) {
     const int row = (int)(c.err >> 8), code = (int)(c.err & 0xff);
     if (code == kChkStart)
@@ -1725,7 +1737,8 @@ int finish_stage(BatchHandle B, int slot, const CsrCheck &c, SysDesc<T> &d) {
   B_TRY(alloc_sell_part<T>(B, slot, stencil ? c.slen : std::max(c.max_row, 1), col16, d, B->xfer,
                            stencil ? c.soff : nullptr));
   d.max_off = c.max_off;
-  d.cl_H = c.stencil && c.slen >= c.max_row ? cl_offsets(c.soff, c.slen, d.cl_off) : 0;
+  cl = ClDesc();
+  if (c.stencil && c.slen >= c.max_row) cl.H = cl_offsets(c.soff, c.slen, cl.off);
   return B200LA_OK;
 }
 
@@ -2087,11 +2100,11 @@ template <typename T> int launch_clusters_t(BatchHandle B, int budget, SideStrea
       B_CUDA(cudaStreamWaitEvent(B->cl_stream[q], B->cl_event[kClStreams], 0));
       side.used = q + 1;
     }
-    B_TRY((cl_with_kernel<T>(B, h.cl_H, h.cl_rows, [&](auto k) -> int {
+    B_TRY((cl_with_kernel<T>(B, h.cl.H, h.cl_rows, [&](auto k) -> int {
       cudaLaunchAttribute attr[1];
       const cudaLaunchConfig_t cfg = cl_config(h.cl_blocks, smem, B->cl_stream[q], attr, (int)(e - a));
-      B_CUDA(cudaLaunchKernelEx(&cfg, k, (const int *)(B->cl_list + a), (const SysDesc<T> *)B->desc, B->st, B->kp,
-                                budget));
+      B_CUDA(cudaLaunchKernelEx(&cfg, k, (const int *)(B->cl_list + a), (const SysDesc<T> *)B->desc,
+                                (const ClDesc *)B->cl_desc, B->st, B->kp, budget));
       B->launched += 1;
       return B200LA_OK;
     })));
@@ -2383,8 +2396,9 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
   for (int k = 0; k < count; ++k) {
     if (sl[k] < 0) continue;
     HostSys &h = B->sys[sl[k]];
-    int rc = finish_stage<T>(B, sl[k], B->chk_host[k], d[k]);
-    if (rc == B200LA_OK) rc = cl_plan<T>(B, h, d[k]);
+    ClDesc cl;
+    int rc = finish_stage<T>(B, sl[k], B->chk_host[k], d[k], cl);
+    if (rc == B200LA_OK) rc = cl_plan<T>(B, h, cl);
     if (rc != B200LA_OK) {
       free_slot_memory(B, h);
       h = HostSys();
@@ -2396,7 +2410,7 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
     memset(&s0, 0, sizeof(SysState));
     s0.phase = PH_RESID;
     s0.bad_row = 0xffffffffu;
-    sj[nsetup++] = SetupJob<T>{d[k], sl[k], (x0 && x0[k]) ? 0 : 1};
+    sj[nsetup++] = SetupJob<T>{d[k], cl, sl[k], (x0 && x0[k]) ? 0 : 1};
     max_n = std::max(max_n, d[k].n);
     B->device_bytes += (int64_t)h.bytes;
     slots[k] = sl[k];
@@ -2407,7 +2421,7 @@ int add_many_t(BatchHandle B, int count, const int *n, const int64_t *nnz, const
     void *sj_dev = (char *)B->jobs_dev + align256(sizeof(CheckJob) * B->chk_cap);
     B_CUDA(cudaMemcpyAsync(sj_dev, sj, sizeof(SetupJob<T>) * nsetup, cudaMemcpyHostToDevice, st));
     slot_init_many_kernel<T><<<(nsetup + kBlock - 1) / kBlock, kBlock, 0, st>>>(
-        (const SetupJob<T> *)sj_dev, nsetup, (SysDesc<T> *)B->desc, B->st, B->sym);
+        (const SetupJob<T> *)sj_dev, nsetup, (SysDesc<T> *)B->desc, B->st, B->cl_desc, B->sym);
     const dim3 grid((unsigned)std::min((max_n + 32 + kBlock - 1) / kBlock, 256), (unsigned)std::min(nsetup, 65535));
     slot_setup_many_kernel<T><<<grid, kBlock, 0, st>>>((const SetupJob<T> *)sj_dev, nsetup, B->st);
     sym_check_many_kernel<T><<<grid, kBlock, 0, st>>>((const SetupJob<T> *)sj_dev, nsetup, B->sym);
@@ -2442,7 +2456,7 @@ int b200la_batch_destroy(b200la_batch B) {
   if (B->exec) cudaGraphExecDestroy(B->exec);
   if (B->graph) cudaGraphDestroy(B->graph);
   for (HostSys &h : B->sys) free_slot_memory(B, h);
-  void *bufs[] = {B->desc, B->st, B->glob, B->chk, B->sysfirst, B->sym, B->cl_list};
+  void *bufs[] = {B->desc, B->st, B->glob, B->chk, B->sysfirst, B->sym, B->cl_list, B->cl_desc};
   for (void *p : bufs)
     if (p) cudaFreeAsync(p, st);
   for (ItemList &L : B->lst) {
@@ -2512,6 +2526,7 @@ int b200la_batch_create(b200la_ctx ctx, const b200la_batch_params *p, b200la_bat
             cudaMallocHost(&B->glob_host, sizeof(BatchGlobals)) == cudaSuccess &&
             cudaMallocAsync(&B->sym, sizeof(int) * p->capacity, st) == cudaSuccess &&
             cudaMallocAsync(&B->cl_list, sizeof(int) * p->capacity, st) == cudaSuccess &&
+            cudaMallocAsync(&B->cl_desc, sizeof(ClDesc) * p->capacity, st) == cudaSuccess &&
             cudaMallocHost(&B->sym_host, sizeof(int) * p->capacity) == cudaSuccess &&
             cudaMemsetAsync(B->sym, 0, sizeof(int) * p->capacity, st) == cudaSuccess;
   // the side streams and their events are made when a launch first uses them
@@ -2592,17 +2607,19 @@ int b200la_batch_add_q1(b200la_batch B, int dim, int cells, uint64_t seed, doubl
     d.max_off = (int)std::min<int64_t>(q1_max_off(dim, cells), INT32_MAX);
     // assembled symmetric: both rows of a pair sum the same cells in the same
     // order, and Dirichlet rows hold only their diagonal
+    ClDesc cl{};
     if (cells >= 2) {
       const int64_t mm = (int64_t)cells + 1;
       int full[kMaxStencil], k = 0;
       for (int dz = (dim == 3 ? -1 : 0); dz <= (dim == 3 ? 1 : 0); ++dz)
         for (int dy = -1; dy <= 1; ++dy)
           for (int dx = -1; dx <= 1; ++dx) full[k++] = (int)(dz * mm * mm + dy * mm + dx);
-      d.cl_H = cl_offsets(full, k, d.cl_off);
+      cl.H = cl_offsets(full, k, cl.off);
     }
-    B_TRY((cl_plan<T>(B, h, d)));
+    B_TRY((cl_plan<T>(B, h, cl)));
+    B_CUDA(cudaMemcpyAsync(B->cl_desc + slot, &cl, sizeof(ClDesc), cudaMemcpyHostToDevice, st));
     B_CUDA(cudaMemsetAsync(B->sym + slot, 0, sizeof(int), st));
-    if (d.cl_H > 0) B_CUDA(cudaMemsetAsync(B->sym + slot, 1, 1, st));  // the low byte: 1
+    if (cl.H > 0) B_CUDA(cudaMemsetAsync(B->sym + slot, 1, 1, st));  // the low byte: 1
     B_CUDA(cudaMemcpyAsync(B->sym_host, B->sym, sizeof(int) * B->capacity, cudaMemcpyDeviceToHost, st));
     B_TRY(q1_assemble(st, B->ctx->num_sms, dim, cells, seed, sigma, (int *)d.rowptr, (int *)d.col,
                       (double *)d.val64, (double *)d.b));
