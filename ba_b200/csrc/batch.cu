@@ -55,7 +55,7 @@
 //   DONE    skipped by every kernel
 // Systems that fit on the SMs of one thread-block cluster (cluster_cg.cuh:
 // symmetric, structured offsets, nine entries a row up to 136,161 FP32 or
-// 66,049 FP64 rows, 27 up to 15,625 or 8,000) do not take part in the passes
+// 66,049 FP64 rows, 27 up to 8,000 or 4,096) do not take part in the passes
 // below: batch_cluster_kernel walks the same phases with the matrix
 // and the Krylov vectors on chip, one cluster a system, as many passes as the
 // run allows, and leaves the state as the pass kernels would.  Which form a
@@ -1573,7 +1573,7 @@ template <typename T> int cl_prepare(BatchHandle B, const HostSys &h, bool *fits
   return B200LA_OK;
 }
 
-constexpr int kClWideMax = 128;
+constexpr int kClWideMax = 64;
 constexpr size_t kClWideSmem = 196 * 1024 - 1024;  // the carve-out step below the largest, less the block's own 1 KB
 
 // Picks the cluster that holds a system: the smallest one it fits on, since
@@ -1581,16 +1581,18 @@ constexpr size_t kClWideSmem = 196 * 1024 - 1024;  // the carve-out step below t
 // other systems fill the rest of the GPU.  A system that fits on none, or only
 // on clusters the device cannot place, stays with the pass kernels.
 // Systems of more than nine entries a row (27-point: 14 values a row on chip)
-// take a cluster only while it is worth its SMs when the GPU is full:
-// blocks x rows a thread x bytes a value up to 128, and no instance of seven
+// take a cluster only while it does their work with clearly less of the GPU:
+// blocks x rows a thread x bytes a value up to 64, and no instance of seven
 // rows where the block's memory leaves the L1 28 KB (its spills then go to
 // L2: 18^3 nodes 1.6 ms on two blocks, 0.7 for 19^3 on four).  Measured, ms
-// for 64 and 256 equal 3D systems on clusters / by the pass kernels: FP32,
-// 17^3 nodes 1.1 / 3.0, 4.2 / 6.0 (2 blocks x 7 rows), 21^3 2.4 / 3.4,
-// 9.3 / 9.7 (4 x 7), 25^3 4.9 / 5.9, 17.2 / 16.7 (8 x 4), beyond the line
-// 26^3 6.2 / 6.1, 22.1 / 19.0 and 27^3 10.1 / 7.6, 37.0 / 21.6 (8 x 7); FP64,
-// 19^3 2.0 / 2.4, 6.8 / 6.2 (8 x 2), beyond it 21^3 3.6 / 2.8, 12.6 / 9.0
-// (8 x 4) and 25^3 6.3 / 5.2, 23.4 / 17.5 (16 x 2).
+// for 256 equal 3D systems on clusters / by the pass kernels: FP32, 17^3 nodes
+// 4.2 / 5.9 (2 blocks x 7 rows), 20^3 6.1 / 8.7 (4 x 4), beyond the line 21^3
+// 9.3 / 9.7 (4 x 7), 25^3 17.2 / 16.5 (8 x 4), 27^3 37.0 / 21.6 (8 x 7); FP64,
+// 16^3 2.6 / 3.5 (4 x 2), beyond it 17^3 4.8 / 4.8 (4 x 4), 21^3 12.6 / 9.0
+// (8 x 4).  Beyond the line a system alone is still faster on a cluster (25^3
+// FP32 0.9 / 1.9), but beside larger ones it holds up their pass kernels: 14
+// batches of 8 to 59 systems of 8 to 19..45 cells, geometric mean 4.67 ms with
+// the line at 128, 4.51 at 64, 4.66 at 32, none on clusters 4.67.
 template <typename T> int cl_plan(BatchHandle B, HostSys &h, const ClDesc &cl) {
   h.cl = cl;
   h.cl_blocks = 0;
