@@ -2863,7 +2863,8 @@ int b200la_batch_solve(b200la_batch B, int chunk_passes, int *total_passes) {
     count_lists(B);
     lists += B->glob_host->passes;
     B_TRY(issue_early_copies(B));
-    B_TRY(upload_tiles(B, true, &active, nullptr, true));
+    active = B->glob_host->active;
+    if (active > 0) B_TRY(upload_tiles(B, true, &active, nullptr, true));
   }
   if (!flown) B_TRY(launch_clusters(B, INT32_MAX, side));
   B_TRY(side.join());
