@@ -2042,22 +2042,28 @@ struct SideStreams {
 };
 
 // Orders the listed clusters by group (one kernel instance and cluster size):
-// small systems first (one block, up to kClSmallRows rows a thread), then the
-// others, each part the largest first.  The small ones are done before a
-// larger cluster would be, and falling order keeps the long solves off the end.
+// where some take more than one block, small systems first (one block, up to
+// kClSmallRows rows a thread), then the others, each part the largest first.
+// The small ones are done before a larger cluster would be, and falling order
+// keeps the long solves off the end; in a batch of one-block systems only that
+// would put their longest last (512 of 16 to 64 cells 2.3 ms against 1.7).
 // ms to the median system and to the end of 1,024 systems of 16 to 256 cells:
-// 1.7 of 74.6, with all groups in falling order 73 of 75.0 (by the pass kernels
-// 63 of 170); FP64 1.7 of 128.4 and 129 of 130.2; the other side, 16 to 128
-// cells 2.1 of 13.0 and 11.1 of 12.2.  Copies the list and stamps the start; the clusters may run
-// from the event recorded here on.
-constexpr int kClSmallRows = 9;
+// 30 of 74.1, with all groups in falling order 73 of 75.0 (by the pass kernels
+// 63 of 170); FP64 54 of 126.7 and 129 of 130.2; 16 to 128 cells 1.5 of 12.4
+// and 11.1 of 12.2.  14 batches of 10 to 355 systems of 16 to 66..233 cells,
+// geometric mean of the end: 3.69 ms in falling order, 3.57 with 4 rows, 3.56
+// with 6, 3.75 with 9.  Copies the list and stamps the start; the clusters may
+// run from the event recorded here on.
+constexpr int kClSmallRows = 6;
 
 int stage_clusters(BatchHandle B) {
   std::vector<int> &sl = B->cl_slots;
   if (sl.empty()) return B200LA_OK;
   cudaStream_t st = B->ctx->stream;
   auto key = [&](int s) { return cl_instance(B->sys[s]); };
-  auto small = [&](int s) { return B->sys[s].cl_blocks == 1 && B->sys[s].cl_rows <= kClSmallRows; };
+  bool large = false;
+  for (int x : sl) large = large || B->sys[x].cl_blocks > 1;
+  auto small = [&](int x) { return large && B->sys[x].cl_blocks == 1 && B->sys[x].cl_rows <= kClSmallRows; };
   std::stable_sort(sl.begin(), sl.end(), [&](int a, int b) {
     const int ka = key(a), kb = key(b), na = B->sys[a].n, nb = B->sys[b].n;
     const bool sa = small(a), sb = small(b);
